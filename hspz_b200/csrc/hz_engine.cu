@@ -240,12 +240,15 @@ unsigned grid_for(uint64_t n, unsigned threads, unsigned cap = 148u * 64u) {
 
 // A sequence packed 2 bits per base for the lockstep gate (pack2_kernel):
 // the forward half and the reversed half, each `half` bases, codes and
-// special masks.
+// special masks, after kPackPad zero records (a gate window may start before
+// the sequence).  Component w of the first record holds the non-ACGT codes
+// that occur in the sequence.
+constexpr uint64_t kPackPad = 2;
 struct Packed {
   DBuf<uint4> blk;  // one 16-byte record per 32 bases
   uint64_t half = 0;
   bool valid = false;
-  const uint4 *half_ptr(int rev) const { return blk.p + (rev ? half / 32 : 0); }
+  const uint4 *half_ptr(int rev) const { return blk.p + kPackPad + (rev ? half / 32 : 0); }
   void release() {
     blk.release();
     valid = false;
@@ -475,68 +478,81 @@ int pack_seq(hz_engine *e, const uint8_t *codes, uint64_t n, Packed *p) {
   p->valid = false;
   p->half = (n + 64 + 31) & ~31ull;
   const uint64_t blocks = 2 * p->half / 32;
-  TRY(p->blk.ensure(blocks + 4, s));
-  CK(cudaMemsetAsync(p->blk.p + blocks, 0, 4 * sizeof(uint4), s));  // read by windows past the end
-  uint4 *bk = p->blk.p;
+  TRY(p->blk.ensure(kPackPad + blocks + 4, s));
+  uint4 *bk = p->blk.p + kPackPad;
+  CK(cudaMemsetAsync(p->blk.p, 0, kPackPad * sizeof(uint4), s));
+  CK(cudaMemsetAsync(bk + blocks, 0, 4 * sizeof(uint4), s));  // read by windows past the end
   const uint64_t half = p->half;
-  TRY(e->launch("pack", [&] { pack2_kernel<<<grid_for(blocks, 256), 256, 0, s>>>(codes, n, half, bk); }));
+  uint32_t *seen = &p->blk.p[0].w;
+  TRY(e->launch("pack", [&] { pack2_kernel<<<grid_for(blocks, 256), 256, 0, s>>>(codes, n, half, bk, seen); }));
   p->valid = true;
   return HZ_OK;
 }
 
-// The lockstep gate reads each cell's score as a signed byte and keeps
-// positions in 32 bits; otherwise the lane-refill gate runs.
+// The lockstep gate reads each cell's cost (the negated score) as a signed
+// byte and keeps positions in 32 bits; otherwise the lane-refill gate runs.
 bool gate2_usable(const hz_engine *e) {
   if (e->gate_version != 2 || !e->ref_p.valid || !e->qry_p.valid) return false;
   if ((uint64_t)e->rlen + 128 >= (1ull << 32) || (uint64_t)e->qstore.len + 128 >= (1ull << 32)) return false;
   for (int r = 0; r < 4; r++)
     for (int q = 0; q < 4; q++) {
       const int32_t v = e->cfg.sub_mat[r * kNuc + q];
-      if (v < -128 || v > 127) return false;
+      if (v < -127 || v > 127) return false;
     }
-  // the group states a round keeps modulo 2^16 (gate2_kernel, near16)
-  return (int64_t)e->cfg.xdrop + kRound * 255 < 32768;
+  // drawdowns are kept in 16 bits (gate2_kernel), and long_kernel's group
+  // states modulo 2^16 (near16)
+  return e->cfg.xdrop >= 0 && e->cfg.xdrop <= kGate2MaxXdrop && (int64_t)e->cfg.xdrop + kRound * 255 < 32768;
 }
 
-template <int TW> size_t gate2_smem() { return sizeof(Gate2Smem<TW>); }
-
-template <int TW, bool SPARSE> int launch_gate2_as(hz_engine *e, const GateArgs &ga) {
-  static bool configured[64] = {false};
+template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, const Gate2Args &a2) {
+  static size_t configured[64] = {0};
   static std::mutex mu;  // serving workers launch from several host threads
-  size_t smem = gate2_smem<TW>();
+  const size_t smem = gate2_smem(e->gate_tile);
   {
     std::lock_guard<std::mutex> lock(mu);
-    if (!configured[e->device & 63]) {
-      CK(cudaFuncSetAttribute(gate2_kernel<TW, SPARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured[e->device & 63] = true;
+    if (configured[e->device & 63] < smem) {
+      CK(cudaFuncSetAttribute(gate2_kernel<SPARSE, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      configured[e->device & 63] = smem;
     }
   }
   int per_sm = e->gate_blocks_per_sm;
   if (per_sm <= 0) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gate2_kernel<TW, SPARSE>, kGateThreads, smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gate2_kernel<SPARSE, GENERAL>, kGateThreads, smem));
     if (per_sm < 1) per_sm = 1;
   }
-  Gate2Args a2;
-  a2.g = ga;
-  a2.ref = e->ref_p.half_ptr(0);
-  a2.refr = e->ref_p.half_ptr(1);
-  a2.qry = e->qry_p.half_ptr(0);
-  a2.qryr = e->qry_p.half_ptr(1);
-  a2.qtotal = (uint32_t)e->qstore.len;
-  unsigned grid = (unsigned)(e->sm_count * per_sm);
-  return e->launch("gate", [&] { gate2_kernel<TW, SPARSE><<<grid, kGateThreads, smem, e->st>>>(a2); });
+  const unsigned grid = (unsigned)(e->sm_count * per_sm);
+  return e->launch("gate", [&] { gate2_kernel<SPARSE, GENERAL><<<grid, kGateThreads, smem, e->st>>>(a2); });
 }
 
 // The sparse tile setup when a tile is expected to span more than three
 // passes of (position, seed) pairs (32 / per_pos positions each), from the
-// hits per query position: seeds per position times the average bucket.
-template <int TW> int launch_gate2(hz_engine *e, const GateArgs &ga) {
+// hits per query position: seeds per position times the average bucket.  The
+// one-table score lookup when complementary pairs score alike (CostTable).
+int launch_gate2(hz_engine *e, const GateArgs &ga) {
+  Gate2Args a2;
+  a2.g = ga;
+  a2.ref = e->ref_p.half_ptr(0) - kPackPad;
+  a2.qry = e->qry_p.half_ptr(0) - kPackPad;
+  a2.tile = (uint32_t)e->gate_tile;
+  a2.soft_codes = 0;
+  bool alike = true;
+  for (int i = 0; i < kNuc; i++)
+    for (int j = 0; j < kNuc; j++) {
+      const int32_t v = ga.sub[i * kNuc + j];
+      if (i < 4 && j < 4) alike = alike && v == ga.sub[(i ^ 3) * kNuc + (j ^ 3)];
+      // a code ends every extension that meets it when all its scores drop
+      // below -xdrop
+      if ((int64_t)v + ga.xdrop < 0) continue;
+      if (i >= 4) a2.soft_codes |= 1u << i;
+      if (j >= 4) a2.soft_codes |= 1u << j;
+    }
   const double per_bucket = (double)e->n_pos / (double)(1ull << (2 * e->shape.kmer_size));
   const double hits_per_pos = std::max(ga.w.per_pos * per_bucket, 1e-9);
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
-      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)TW / hits_per_pos > 3.0 * positions_per_pass;
-  return sparse ? launch_gate2_as<TW, true>(e, ga) : launch_gate2_as<TW, false>(e, ga);
+      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)e->gate_tile / hits_per_pos > 3.0 * positions_per_pass;
+  if (alike) return sparse ? launch_gate2_as<true, false>(e, a2) : launch_gate2_as<false, false>(e, a2);
+  return sparse ? launch_gate2_as<true, true>(e, a2) : launch_gate2_as<false, true>(e, a2);
 }
 
 // The long candidates of a wave, extended to their ends in lockstep over the
@@ -883,11 +899,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       ga.tile_first = e->tile_first.p;
       ga.tile_call = e->tile_call.p;
       if (gate2_usable(e)) {
-        switch (e->gate_tile) {
-          case 64: TRY(launch_gate2<64>(e, ga)); break;
-          case 256: TRY(launch_gate2<256>(e, ga)); break;
-          default: TRY(launch_gate2<128>(e, ga)); break;
-        }
+        TRY(launch_gate2(e, ga));
         TRY(launch_long(e, ga));
       } else {
         switch (e->gate_tile) {

@@ -49,9 +49,11 @@ __global__ void encode_kernel(const uint8_t *__restrict__ ascii, uint64_t n, uin
 // special mask (bit i set when base i is not uppercase ACGT -- soft-masked,
 // N, other or separator -- whose code packs as 0), w = 0.  Positions past the
 // block in each half are 0 and not special; extensions never score them.  One
-// record per thread.
+// record per thread.  The non-ACGT codes that occur (bit c for code c) are
+// gathered in *seen.
 __global__ void pack2_kernel(const uint8_t *__restrict__ codes, uint64_t n, uint64_t half,
-                             uint4 *__restrict__ blk) {
+                             uint4 *__restrict__ blk, uint32_t *__restrict__ seen) {
+  uint32_t special = 0;
   const uint64_t blocks = (2 * half) / 32;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < blocks; b += stride) {
@@ -67,9 +69,13 @@ __global__ void pack2_kernel(const uint8_t *__restrict__ codes, uint64_t n, uint
       if (i < 16) lo |= bits << (2 * i);
       else hi |= bits << (2 * (i - 16));
       sp |= (uint32_t)(c >= 4) << i;
+      special |= 1u << c;
     }
     blk[b] = make_uint4(lo, hi, sp, 0u);
   }
+  special = __reduce_or_sync(0xffffffffu, special) & 0xF0u;
+  // most warps find their codes there already and spare the atomic
+  if ((threadIdx.x & 31) == 0 && (special & ~*(volatile uint32_t *)seen)) atomicOr(seen, special);
 }
 
 // The 32 bases of a packed half that start at base p: their codes (lo: the

@@ -29,6 +29,67 @@
 
 namespace hz {
 
+constexpr int kRound = 48;             // cells long_kernel scores per round
+constexpr int kChunks = kRound / 16;   // 16-cell code words per sequence in a round
+constexpr int kGroups = kRound / 8;    // eight-cell groups per round
+
+// The kRound bases of a packed half that start at base p: their codes, 16
+// per word, and their special bits (cells 0..31 in *sp_lo, the rest in
+// *sp_hi), from the 16-byte records that hold them.
+__device__ __forceinline__ void window_round(const uint4 *__restrict__ blk, uint32_t p, uint32_t code[kChunks],
+                                             uint32_t *sp_lo, uint32_t *sp_hi) {
+  constexpr int kRec = (kRound + 31) / 32 + 1;
+  uint4 r[kRec];
+#pragma unroll
+  for (int i = 0; i < kRec; i++) r[i] = __ldg(blk + (p >> 5) + i);
+  uint32_t c[2 * kRec];
+#pragma unroll
+  for (int i = 0; i < kRec; i++) {
+    c[2 * i] = r[i].x;
+    c[2 * i + 1] = r[i].y;
+  }
+  const uint32_t o = p & 31u, sh = (o & 15u) << 1;
+  const bool upper = o >= 16;  // the window starts in a record's second code word
+  uint32_t cs[kChunks + 1];
+#pragma unroll
+  for (int k = 0; k <= kChunks; k++) cs[k] = upper ? c[k + 1] : c[k];
+#pragma unroll
+  for (int k = 0; k < kChunks; k++) code[k] = __funnelshift_r(cs[k], cs[k + 1], sh);
+  *sp_lo = __funnelshift_r(r[0].z, r[1].z, o);
+  *sp_hi = kRound > 32 ? __funnelshift_r(r[1].z, r[kRec - 1].z, o) : 0u;
+}
+
+// The four index words of 16 cells: word j holds cells j, j+4, j+8, j+12 in
+// its bytes 0..3, each byte being that cell's table index (reference code |
+// query code << 2) with its upper four bits clear.  Every lane's score lookup
+// then falls in the same 16 bytes of shared memory, four banks, so a warp's
+// lookup is one wavefront whatever the codes.
+__device__ __forceinline__ void pair_words(uint32_t r, uint32_t q, uint32_t t[4]) {
+  const uint32_t x = (r & 0x33333333u) | ((q << 2) & 0xCCCCCCCCu);  // nibble n: index of cell 2n
+  const uint32_t y = ((r >> 2) & 0x33333333u) | (q & 0xCCCCCCCCu);  // nibble n: index of cell 2n + 1
+  t[0] = x & 0x0F0F0F0Fu;
+  t[1] = y & 0x0F0F0F0Fu;
+  t[2] = (x >> 4) & 0x0F0F0F0Fu;
+  t[3] = (y >> 4) & 0x0F0F0F0Fu;
+}
+
+// Score of cell k (0..15) of the 16 cells whose index words are t.
+__device__ __forceinline__ int32_t cell_score(const int8_t *tbl, const uint32_t t[4], int k) {
+  return tbl[__byte_perm(t[k & 3], 0u, 0x4440u + (uint32_t)(k >> 2))];
+}
+
+__device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
+
+// The value v with v = h (mod 2^16) and base - 32768 <= v < base + 32768.
+// A round's group states are read back against the running sum after all
+// its kRound cells, which lies within kRound * 128 of every stored sum; a
+// stored maximum read back exceeds its sum by at most xdrop plus one group's
+// fall, so every value read lies within kRound * 255 + xdrop of the base
+// (gate2_usable checks that this is below 32768).
+__device__ __forceinline__ int32_t near16(int32_t base, uint32_t h) {
+  return wadd(base, (int32_t)(int16_t)(uint16_t)(h - (uint32_t)base));
+}
+
 constexpr uint32_t kDoneFlag = 1u << 30;  // Cand::call: maxima and positions filled in by long_kernel
 
 struct LongArgs {

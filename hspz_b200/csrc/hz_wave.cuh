@@ -67,7 +67,9 @@ struct WaveTotals {
 };
 
 // Gate candidate: a hit whose score bound passes the threshold, or whose
-// extension ran past the per-direction cap ("long").
+// extension ran past the per-direction cap.  Those that long_kernel extends
+// carry kLongFlag: every candidate of the lockstep gate, the ones past the
+// cap of the lane-refill gate.
 struct Cand {
   uint32_t scope;  // dedup scope of the hit
   uint32_t r0;     // reference anchor

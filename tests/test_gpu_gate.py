@@ -1,0 +1,87 @@
+"""The lockstep gate's own edges against the oracle: extensions that end at
+the window's last cells, in later rounds, at soft-masked, N and IUPAC bases,
+at sequence ends and at the cap; score matrices with and without strand
+symmetry; drops that need more than one flagged group."""
+import numpy as np
+import pytest
+
+from hspz_b200 import EngineConfig, synth
+from hspz_b200.build import build
+from tests.test_gpu_parity import engine_for, oracle_run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    build()
+
+
+def sequences(seed: int):
+    """A pair rich in ends: many short records' worth of N, IUPAC codes,
+    lowercase and planted segments of 19..400 bases, some at the ends."""
+    rng = np.random.default_rng(seed)
+    t, q = synth.random_bases(rng, 40_000), synth.random_bases(rng, 30_000)
+    synth.plant(rng, t, q, 120, 19, 400, 0.0, 0.25)
+    q[:300] = t[-300:]
+    q[-250:] = t[:250]
+    for s in (t, q):
+        s[rng.integers(0, s.size, 60)] = ord("N")
+        s[rng.integers(0, s.size, 60)] = ord("R")
+        for a in rng.integers(0, s.size - 60, 40).tolist():
+            s[a:a + int(rng.integers(1, 60))] |= 0x20
+        s[rng.integers(0, s.size, 6)] = ord("&")
+    return t, q
+
+
+def matrix(kind: str, xdrop: int):
+    m = EngineConfig().sub_mat if kind != "ambiguous" else None
+    if m is None:
+        from hspz_b200 import build_sub_mat
+        return build_sub_mat("n", xdrop)
+    m = list(m)
+    if kind == "general":  # no two of the sixteen ACGT scores are tied by strand
+        rng = np.random.default_rng(5)
+        for r in range(4):
+            for c in range(4):
+                m[r * 8 + c] = int(rng.integers(60, 127)) if r == c else -int(rng.integers(20, 127))
+    return m
+
+
+@pytest.mark.parametrize("kind,xdrop,cap,sparse", [
+    ("default", 910, 128, 0), ("default", 910, 128, 1), ("default", 910, 40, 0), ("default", 910, 56, 1),
+    ("default", 910, 96, 0), ("default", 910, 8, 0), ("default", 910, 65528, 0), ("default", 120, 128, 0),
+    ("default", 0, 128, 0), ("default", 9000, 1024, 1), ("default", 20000, 256, 0),
+    ("general", 910, 128, 0), ("general", 910, 104, 1), ("general", 150, 128, 0), ("ambiguous", 910, 128, 0),
+    ("ambiguous", 910, 4096, 1)])
+def test_gate_edges_match_the_oracle(kind, xdrop, cap, sparse):
+    t, q = sequences(xdrop + cap)
+    sm = matrix(kind, xdrop)
+    hspthresh = 3000 if xdrop >= 500 else 1500
+    want, st_o = oracle_run(t, q, sm, xdrop=xdrop, hspthresh=hspthresh)
+    with engine_for(sm, xdrop=xdrop, hspthresh=hspthresh) as e:
+        e.set_tuning(gate_cap=cap, gate_sparse=sparse)
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+    assert want.size > 20
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
+
+
+@pytest.mark.parametrize("n", [19, 20, 40, 57, 95, 96, 97, 130])
+def test_short_sequences_match_the_oracle(n):
+    """Targets and queries around a window long: windows reach past both ends."""
+    rng = np.random.default_rng(n)
+    t = synth.random_bases(rng, n)
+    q = np.concatenate([t, synth.random_bases(rng, 40), t])
+    sm = EngineConfig().sub_mat
+    want, st_o = oracle_run(t, q, sm, hspthresh=1000)
+    with engine_for(sm, hspthresh=1000) as e:
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
