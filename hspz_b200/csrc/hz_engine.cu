@@ -354,6 +354,8 @@ struct hz_engine {
   DBuf<HitNz> np_partial, np_grand;
   DBuf<WaveTotals> tot;
   DBuf<Cand> cand;
+  DBuf<uint32_t> gate_ring;       // the lockstep gate's waiting hits, for gate_ring_blocks blocks
+  unsigned gate_ring_blocks = 0;
   DBuf<SegmentPair> raw;
   HBuf<CallDev> h_calls;
   HBuf<WaveTotals> h_tot;
@@ -372,7 +374,7 @@ struct hz_engine {
   // reuse the host memory instead of growing (and faulting in) a new vector
   std::vector<WaveRecord> batch_recs;
   int gate_sparse = -1;  // lockstep gate tile setup: -1 chosen from the target's buckets, 0 pairs, 1 lane per position
-  int gate_tile = 128;  // hits per gate warp tile
+  int gate_tile = 0;  // hits per gate warp tile; 0: the gate's own choice (wave_tile)
   uint32_t gate_cap = 128;  // the autotuner's usual choice
   int gate_blocks_per_sm = 0;
   uint64_t wave_positions = 1ull << 27;  // seed positions per batched wave
@@ -504,10 +506,16 @@ bool gate2_usable(const hz_engine *e) {
   return e->cfg.xdrop >= 0 && e->cfg.xdrop <= kGate2MaxXdrop && (int64_t)e->cfg.xdrop + kRound * 255 < 32768;
 }
 
-template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, const Gate2Args &a2) {
+// Hits per warp tile: the knob's, or what suits the gate that runs.  The
+// lane-refill gate stages every hit in shared memory, and beyond 128 hits that
+// costs it the L1 it lives on.
+int wave_tile(const hz_engine *e) { return e->gate_tile ? e->gate_tile : gate2_usable(e) ? 256 : 128; }
+
+// Prepares one instance of the lockstep gate for 'smem' bytes of shared
+// memory and returns its blocks per SM.
+template <bool SPARSE, bool GENERAL> int gate2_blocks(hz_engine *e, size_t smem, int *per_sm) {
   static size_t configured[64] = {0};
   static std::mutex mu;  // serving workers launch from several host threads
-  const size_t smem = gate2_smem(e->gate_tile);
   {
     std::lock_guard<std::mutex> lock(mu);
     if (configured[e->device & 63] < smem) {
@@ -515,25 +523,36 @@ template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, const Gat
       configured[e->device & 63] = smem;
     }
   }
-  int per_sm = e->gate_blocks_per_sm;
-  if (per_sm <= 0) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gate2_kernel<SPARSE, GENERAL>, kGateThreads, smem));
-    if (per_sm < 1) per_sm = 1;
+  *per_sm = e->gate_blocks_per_sm;
+  if (*per_sm <= 0) {
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, gate2_kernel<SPARSE, GENERAL>, kGate2Threads, smem));
+    if (*per_sm < 1) *per_sm = 1;
   }
-  const unsigned grid = (unsigned)(e->sm_count * per_sm);
-  return e->launch("gate", [&] { gate2_kernel<SPARSE, GENERAL><<<grid, kGateThreads, smem, e->st>>>(a2); });
+  return HZ_OK;
 }
 
-// The sparse tile setup when a tile is expected to span more than three
-// passes of (position, seed) pairs (32 / per_pos positions each), from the
-// hits per query position: seeds per position times the average bucket.  The
-// one-table score lookup when complementary pairs score alike (CostTable).
+template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, Gate2Args &a2) {
+  const size_t smem = gate2_smem((int)a2.tile);
+  int per_sm = 0;
+  TRY((gate2_blocks<SPARSE, GENERAL>(e, smem, &per_sm)));
+  const unsigned grid = std::min<unsigned>((unsigned)(e->sm_count * per_sm), e->gate_ring_blocks);
+  return e->launch("gate", [&] { gate2_kernel<SPARSE, GENERAL><<<grid, kGate2Threads, smem, e->st>>>(a2); });
+}
+
+// The sparse tile setup (a lane per position) when a tile is expected to span
+// more than 7.5 passes of (position, seed) pairs (32 / per_pos positions
+// each), from the hits per query position: seeds per position times the
+// average bucket.  256-hit tiles, 13 seeds, ps per hit by hits per position,
+// pairs against lanes: 4.7: 48.1 / 41.8, 9.5: 37.7 / 35.0, 18.9: 32.2 / 32.6,
+// 42: 29.3 / 32.2, 113: 28.4 / 32.4.  The one-table score lookup when
+// complementary pairs score alike (CostTable).
 int launch_gate2(hz_engine *e, const GateArgs &ga) {
   Gate2Args a2;
   a2.g = ga;
   a2.ref = e->ref_p.half_ptr(0) - kPackPad;
   a2.qry = e->qry_p.half_ptr(0) - kPackPad;
-  a2.tile = (uint32_t)e->gate_tile;
+  a2.ring = e->gate_ring.p;
+  a2.tile = (uint32_t)wave_tile(e);
   a2.soft_codes = 0;
   bool alike = true;
   for (int i = 0; i < kNuc; i++)
@@ -546,11 +565,22 @@ int launch_gate2(hz_engine *e, const GateArgs &ga) {
       if (i >= 4) a2.soft_codes |= 1u << i;
       if (j >= 4) a2.soft_codes |= 1u << j;
     }
+  {  // (i32)(f32)total >= hspthresh holds from some total on: the gate compares integers
+    int64_t lo = INT32_MIN, hi = INT32_MAX;  // the answer lies in [lo, hi]
+    while (lo < hi) {
+      const int64_t mid = lo + (hi - lo) / 2;
+      const double f = (double)(float)(int32_t)mid;
+      const int32_t t = f >= 2147483647.0 ? INT32_MAX : (int32_t)f;
+      if (t >= ga.hspthresh) hi = mid;
+      else lo = mid + 1;
+    }
+    a2.min_total = (int32_t)lo;
+  }
   const double per_bucket = (double)e->n_pos / (double)(1ull << (2 * e->shape.kmer_size));
   const double hits_per_pos = std::max(ga.w.per_pos * per_bucket, 1e-9);
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
-      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)e->gate_tile / hits_per_pos > 3.0 * positions_per_pass;
+      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 7.5 * positions_per_pass;
   if (alike) return sparse ? launch_gate2_as<true, false>(e, a2) : launch_gate2_as<false, false>(e, a2);
   return sparse ? launch_gate2_as<true, true>(e, a2) : launch_gate2_as<false, true>(e, a2);
 }
@@ -834,12 +864,19 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
   const bool packed_q = e->qry_p.valid && e->shape.size <= 32 && e->qry_p.half >= e->qstore.len;
   w.qp2 = packed_q ? e->qry_p.half_ptr(0) : nullptr;
   w.pos_kmer = e->pos_kmer.p;
+  const int tile = wave_tile(e);
 
   for (int attempt = 0; attempt < 8; attempt++) {  // each rerun fixes every capacity it found short
     uint32_t scope_cap = std::max<uint32_t>(e->scope_cap, (uint32_t)n * 2 + 16);
     TRY(e->scope_lo.ensure(scope_cap + 1, s));
     TRY(e->scope_call.ensure(scope_cap + 1, s));
     TRY(e->cand.ensure(e->cand_cap, s));
+    if (gate2_usable(e)) {
+      // room for every block that can run
+      e->gate_ring_blocks =
+          (unsigned)(e->sm_count * (e->gate_blocks_per_sm > 0 ? e->gate_blocks_per_sm : kGate2BlocksPerSm));
+      TRY(e->gate_ring.ensure(gate2_ring_words(e->gate_ring_blocks), s));
+    }
     TRY(e->raw.ensure(e->raw_cap, s));
     TRY(e->raw_scope.ensure(e->raw_cap, s));
     TRY(e->tile_first.ensure(e->tile_cap, s));
@@ -868,7 +905,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
           4));
       TRY(e->launch("tile_table", [&] {
         tile_table_kernel<<<grid_for(npos, 256, e->sm_count * 8), 256, 0, s>>>(
-            e->np_excl.p, e->pos_hits.p, e->np_pos.p, e->calls.p, (uint32_t)n, e->tot.p, (uint32_t)e->gate_tile,
+            e->np_excl.p, e->pos_hits.p, e->np_pos.p, e->calls.p, (uint32_t)n, e->tot.p, (uint32_t)tile,
             e->tile_first.p, e->tile_call.p, e->tile_cap);
       }));
       TRY(e->launch("scopes", [&] {
@@ -902,7 +939,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
         TRY(launch_gate2(e, ga));
         TRY(launch_long(e, ga));
       } else {
-        switch (e->gate_tile) {
+        switch (tile) {
           case 64: TRY(launch_gate<64>(e, ga)); break;
           case 256: TRY(launch_gate<256>(e, ga)); break;
           default: TRY(launch_gate<128>(e, ga)); break;
@@ -958,7 +995,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     // buffers stay bounded on repeat-dense input
     if (n > 1 && t.hits > e->wave_hits_cap) return kSplitWave;
     if (t.status & 4u) {  // the gate skipped the wave: its tile table was too small
-      e->tile_cap = (uint32_t)std::min<uint64_t>(t.hits / (uint64_t)e->gate_tile + 1024, 0xFFFFFFF0ull);
+      e->tile_cap = (uint32_t)std::min<uint64_t>(t.hits / (uint64_t)tile + 1024, 0xFFFFFFF0ull);
       again = true;
     }
     if (t.n_scopes > scope_cap) {
@@ -1292,6 +1329,7 @@ void hz_engine_destroy(hz_engine *e) {
   e->np_grand.release();
   e->tot.release();
   e->cand.release();
+  e->gate_ring.release();
   e->raw.release();
   e->h_calls.release();
   e->h_tot.release();
@@ -2264,7 +2302,7 @@ int hz_engine_autotune(hz_engine *e, uint64_t sample_positions, hz_tuning *out) 
     e->use_graph = start.graph;
     return rc;
   }
-  out->gate_tile = pick.tile;
+  out->gate_tile = wave_tile(e);
   out->gate_cap = (int32_t)pick.cap;
   out->gate_blocks_per_sm = e->gate_blocks_per_sm;
   out->graph = pick.graph ? 1 : 0;
@@ -2355,7 +2393,7 @@ uint64_t wave_footprint(const hz_engine *w) {
        dbytes(w->pos_kmer) + dbytes(w->np_kmer) +
        dbytes(w->scope_call) + dbytes(w->raw_scope) + dbytes(w->tile_first) + dbytes(w->tile_call) +
        dbytes(w->np_excl) + dbytes(w->call_hit_lo) + dbytes(w->scope_lo) + dbytes(w->np_partial) +
-       dbytes(w->np_grand) + dbytes(w->tot) + dbytes(w->cand) + dbytes(w->raw) + dbytes(w->d_out);
+       dbytes(w->np_grand) + dbytes(w->tot) + dbytes(w->cand) + dbytes(w->gate_ring) + dbytes(w->raw) + dbytes(w->d_out);
   for (const DBuf<uint32_t> *x : {&w->d_perm_a, &w->d_perm_b, &w->d_keys_a, &w->d_keys_b, &w->d_keep,
                                   &w->d_keep_excl, &w->d_hist, &w->d_hpart, &w->d_total})
     b += dbytes(*x);
@@ -2381,6 +2419,7 @@ void release_wave_buffers(hz_engine *w) {
   w->np_partial.release();
   w->np_grand.release();
   w->cand.release();
+  w->gate_ring.release();
   w->raw.release();
   w->d_out.release();
   w->calls.release();
@@ -2673,7 +2712,7 @@ int hz_serve_start(hz_engine *e, const hz_serve_config *cfg) {
   // starting rate: a query k-mer drawn uniformly meets per_pos buckets of the
   // average size
   s->hits_per_pos = e->index_len ? (double)e->per_pos(e->cfg.transitions) * (double)e->n_pos / (double)e->index_len : 0;
-  s->gate_tile = e->gate_tile;
+  s->gate_tile = e->gate_tile ? e->gate_tile : 128;  // the smallest tile a wave takes by itself
   e->server = s;
   for (uint32_t i = 0; i < (uint32_t)s->workers.size(); i++) s->threads.emplace_back(serve_worker, s, i, s->workers[i]);
   return HZ_OK;

@@ -3,12 +3,12 @@
 // The same work as gate_kernel -- fused hit expansion and the X-drop score
 // bound of every hit, src/gpu/kernels.rs:521-1057 -- organised so that a
 // warp's 32 lanes run one instruction stream:
-//   * a lane owns one hit and scores both of its extensions in one round over
-//     one window of each sequence, kLeft bases before the anchor and kRight
-//     after it.  Random hits end after ~40 cells to the left (19 of them the
-//     seed) and ~21 to the right, so one round ends 92 % of the hits; a lane
-//     whose extension goes on keeps its hit for another round, with the
-//     anchor moved to where the extension stands;
+//   * a warp takes 32 hits of its tile at a time, a lane each, and scores both
+//     extensions of each in one round over one window of each sequence, kLeft
+//     bases before the anchor and kRight after it.  Random hits end after ~40
+//     cells to the left (19 of them the seed) and ~21 to the right, so one
+//     round ends 92 % of the hits; those that go on wait in a ring until 32
+//     have gathered for another round from where they stand;
 //   * both extensions read the same forward copy of each sequence: the left
 //     one takes its cells in descending order, which costs nothing because
 //     every cell's place in the window is a constant of the code;
@@ -32,10 +32,12 @@
 // run beside that pipe, and one window of four 16-byte records per sequence
 // instead of six for two separate ones.
 //
-// Measured against the kernel before it (one direction per round over two
-// packed copies, a shared-memory table lookup and three adds per cell): a 200
-// Mbp target took 60.1 ps per hit and takes 36.5 (326.6 -> 198.3 ms for 5.4e9
-// hits), a 10 Mbp bin 68 -> 47 ps.
+// Measured, ps per hit against a 200 Mbp target (5.4e9 hits) / a 10 Mbp bin: a
+// kernel of one direction per round over two packed copies, a shared-memory
+// lookup and three adds per cell took 60.1 / 68; this one, with the 8 % that
+// go on keeping their lanes, 36.5 / 47; with the ring, which leaves the first
+// round without per-lane state, 33.7 / 42; with a tile's bucket bounds loaded
+// together and 256-hit tiles, 28.0 / 35.  ncu: issue 81 %, ALU 71 %, L1 72 %.
 //
 // The extension semantics are those of the scalar oracle and the reference
 // warp kernel: S += sub[r][q]; M' = max(M, S) includes the cell; the
@@ -61,6 +63,14 @@ constexpr int kSolo = (kLeft - kRight) / 8;   // the left extension's first grou
 constexpr int kGroupsL = kLeft / 8;           // eight-cell groups of each direction
 constexpr int kGroupsR = kRight / 8;
 constexpr uint32_t kMaxTile = 256;
+// Blocks of four warps, seven per SM: 72 registers a thread.  At 64 registers
+// (32 warps) the compiler rebuilds constants and addresses, 806 instructions
+// per round instead of 730, and 24 warps at 80 registers leave the issue slots
+// empty: 27.97 ps per hit against 29.9 and 29.0 (200 Mbp target, 256-hit
+// tiles).
+constexpr int kGate2Threads = 128;
+constexpr int kGate2Warps = kGate2Threads / 32;
+constexpr int kGate2BlocksPerSm = 7;
 // Running costs are kept as kCostBase + A in 16 unsigned bits.  A falls by at
 // most kLeft * 127 in a round and rises by at most kLeft * 128 above
 // kCostBase + xdrop.
@@ -72,19 +82,39 @@ static_assert(kLeft % 8 == 0 && kRight % 8 == 0 && kLeft > kRight, "groups of ei
 // up to 128 per cell.
 constexpr int32_t kGate2MaxXdrop = 32767 - 128;
 
-// Shared memory of one warp; slot[] follows with one entry per hit of a tile.
+// Shared memory of one warp; the slot arrays follow, 12 bytes per hit of a
+// tile: 5.6 KB with 256-hit tiles, 164 KB per SM, which leaves 88 KB of L1.
+// 128-hit tiles take 29.7 ps per hit (a setup every four rounds, mostly
+// latency), 64-hit ones 34.1.
 struct GateWarp {
   uint2 sel[kWinChunks][32];    // each lane's table indices: of the even and the odd cells of 16 bases
   uint32_t grp[kGroupsL][32];   // drawdowns before each group, biased (right low half, left high half)
   uint32_t bits[kMaxTile / 32];   // tile hits at which a slot starts
   uint32_t carry[kMaxTile / 32];  // the last slot that starts before the 32 hits
-  uint32_t hdr[4];              // the claimed next tile's first position, the position after it, its call
+  uint32_t hdr[3];              // the claimed next tile's first position, the position after it, its call
+  uint32_t nz;                  // positions with hits, and hits, of the wave
+  unsigned long long total;
 };
-// A slot is a run of tile hits of one (position, seed), indexed by its first
-// hit: x = pos_table index of tile hit 0 of the run (so hit t is x + t),
-// y = query anchor (absolute), z = call, w = cells to the query's right edge |
-// cells to its left edge << 16 (each saturated).
-inline size_t gate2_smem(int tile) { return kGateWarps * (sizeof(GateWarp) + (size_t)tile * sizeof(uint4)); }
+inline size_t gate2_smem(int tile) { return kGate2Warps * (sizeof(GateWarp) + (size_t)tile * 12); }
+
+// Hits that go on for another round (8 % of them) wait in a ring of their
+// warp in device memory, a word per field, fields kRingCap apart.  A round
+// adds at most 32, and 32 are taken as soon as the ring holds them, so at most
+// 31 + 32 wait.
+constexpr uint32_t kRingCap = 64;
+enum RingField : uint32_t {
+  kRingR, kRingQ,  // anchors
+  kRingCall,
+  kRingHit,        // wave index / 32; the rest of it is in kRingState
+  kRingOff,        // how far from the anchor the next window stands
+  kRingDraw,       // drawdowns (right low half, left high half)
+  kRingBound,      // summed bounds of the maxima so far
+  kRingState,      // kGo*, kWaitLeft | wave index % 32 << 3 | cells scored so far << 8
+  kRingFields
+};
+constexpr uint32_t kGoRight = 1, kGoLeft = 2;  // directions the next window scores
+constexpr uint32_t kWaitLeft = 4;              // the left extension goes on after the right one
+inline size_t gate2_ring_words(size_t blocks) { return blocks * kGate2Warps * kRingFields * kRingCap; }
 
 struct Gate2Args {
   GateArgs g;
@@ -92,8 +122,10 @@ struct Gate2Args {
   // their first base: a window may start kLeft bases before the sequence.
   // Component w of the first record holds the non-ACGT codes of the sequence.
   const uint4 *ref, *qry;
+  uint32_t *ring;       // gate2_ring_words words
   uint32_t tile;        // hits per warp tile, a multiple of 32, at most kMaxTile
   uint32_t soft_codes;  // bit c: code c (4..7) does not end every extension that meets it
+  int32_t min_total;    // the smallest total with (i32)(f32)total >= hspthresh
 };
 
 // 4-byte global -> shared copy that completes asynchronously (no register
@@ -111,6 +143,12 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ uint32_t permute(uint32_t a, uint32_t b, uint32_t s) {
   uint32_t d;
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
+  return d;
+}
+
+__device__ __forceinline__ uint32_t min_halves(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
 
@@ -192,59 +230,58 @@ __device__ __forceinline__ uint32_t add_byte(uint32_t word, int b, uint32_t acc)
 // position instead of per (position, seed) pair.  The engine picks it from
 // the target's average bucket size.  GENERAL: see CostTable.
 template <bool SPARSE, bool GENERAL>
-__global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_constant__ Gate2Args a2) {
+__global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel(const __grid_constant__ Gate2Args a2) {
   const GateArgs &a = a2.g;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (a.tot->status & 4u) return;  // no tile table: the host reruns the wave with a larger one
   const uint32_t tile = a2.tile;
-  unsigned char *mine = smem_raw + (threadIdx.x >> 5) * (sizeof(GateWarp) + tile * sizeof(uint4));
+  unsigned char *mine = smem_raw + (threadIdx.x >> 5) * (sizeof(GateWarp) + tile * 12);
   GateWarp &wt = *reinterpret_cast<GateWarp *>(mine);
-  uint4 *const slot = reinterpret_cast<uint4 *>(mine + sizeof(GateWarp));
+  // A slot is a run of tile hits of one (position, seed), stored at its first
+  // hit: its pos_table index less that hit (so hit t is slot_x + t), the query
+  // anchor (absolute) and the call.
+  uint32_t *const slot_x = reinterpret_cast<uint32_t *>(mine + sizeof(GateWarp));
+  uint32_t *const slot_q = slot_x + tile, *const slot_call = slot_q + tile;
   const uint32_t lane = threadIdx.x & 31;
   const CostTable<GENERAL> tab(a.sub);
   const uint32_t thr = 0x7FFFu - (uint32_t)a.xdrop;  // drawdown + thr has bit 15 set when it exceeds xdrop
   const uint32_t thr2 = thr * 0x10001u;
   const bool soft = ((a2.ref[0].w | a2.qry[0].w) & a2.soft_codes) != 0;
-  unsigned long long cells_acc = 0;
-  const unsigned long long total = a.tot->hits;
-  const uint32_t nz = a.tot->nz;
   const WaveIn &w = a.w;
+  uint32_t cells_acc = 0;  // cells of the lane's hits, added to the wave's count before it can wrap
 
-  // the tile the cursor hands hits out of (warp-uniform)
-  unsigned long long h0 = 0;
-  uint32_t nt = 0, cursor = 0;
-  bool tiles_done = false;
+  // the tile the cursor hands hits out of (warp-uniform); a wave's hits are
+  // below 2^37, so hit indices / 32 fit 32 bits
+  uint32_t tile_at = 0, nt = 0, cursor = 0;
   // the next tile's index, claimed from the work queue once half of the
   // current tile is handed out so that its latency is hidden (lane 0 holds it)
   bool claimed = false;
-  unsigned long long claim = 0;
+  uint32_t claim = 0;
   // The tile setup spreads a tile's (position, seed) pairs over the lanes:
   // 32 / per_pos positions per pass, lane l on seed l % per_pos of position
   // l / per_pos, so all bucket bounds of a pass are loaded at once.
   const uint32_t per = w.per_pos, ppi = 32u / per, lpi = lane / per, lvar = lane - lpi * per;
   bool hdr = false;  // the claimed tile's header is on its way into wt.hdr
-  auto put_slot = [&](uint32_t sl, uint32_t bst, uint32_t qa, uint32_t c, const CallDev &cd) {
-    slot[sl] = make_uint4(bst - sl, qa, c,
-                          min(cd.qoff + cd.qlen - qa, 0xFFFFu) | min(qa - cd.qoff, 0xFFFFu) << 16);
+  auto put_slot = [&](uint32_t sl, uint32_t bst, uint32_t qa, uint32_t c) {
+    slot_x[sl] = bst - sl;
+    slot_q[sl] = qa;
+    slot_call[sl] = c;
     atomicOr(&wt.bits[sl >> 5], 1u << (sl & 31u));
   };
-  // Takes the next tile from the work queue and finds its slots.  Every lane
-  // takes part; lanes busy with an earlier tile's hits hold what they need of
-  // them in registers.
+  // Takes the next tile from the work queue and finds its slots, from as few
+  // waits as it can (the positions, then their seeds' buckets); leaves nt 0
+  // when there is none.
   auto next_tile = [&]() {
-    unsigned long long j = claim;
-    if (!claimed && lane == 0) j = atomicAdd(&a.tot->tiles, 1ull);
-    j = __shfl_sync(0xffffffffu, j, 0);
+    if (!claimed && lane == 0) claim = (uint32_t)atomicAdd(&a.tot->tiles, 1ull);
+    const uint32_t j = __shfl_sync(0xffffffffu, claim, 0);
     const bool have_hdr = claimed && hdr;
     claimed = false;
     hdr = false;
-    h0 = j * (unsigned long long)tile;
+    const unsigned long long h0 = j * (unsigned long long)tile, total = wt.total;
+    tile_at = j;
     cursor = 0;
-    if (h0 >= total) {
-      tiles_done = true;
-      nt = 0;
-      return;
-    }
+    nt = 0;
+    if (h0 >= total) return;
     nt = (uint32_t)min((unsigned long long)tile, total - h0);
     uint32_t k0, k1, c0;
     if (have_hdr) {
@@ -261,89 +298,91 @@ __global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_con
     // positions k0 .. kend cover the tile (k1, the next tile's first
     // position, only if its hits start inside this one; the overlap test
     // below sorts that out)
-    const uint32_t kend = min(k1, nz - 1);
+    const uint32_t kend = min(k1, wt.nz - 1);
     const CallDev call0 = w.calls[c0];
     const uint32_t next_off = c0 + 1 < w.ncalls ? w.calls[c0 + 1].pos_off : 0xFFFFFFFFu;
     __syncwarp();  // every lane has read what it needs of the previous tile
     if (lane < kMaxTile / 32) wt.bits[lane] = 0;
     __syncwarp();
-    if constexpr (SPARSE) {
-      // a lane per position, its seeds' bucket bounds loaded five at a time
-      // (more would spill in this register budget)
-      for (uint32_t k = k0 + lane; k <= kend; k += 32) {
-        const uint32_t p = a.np_pos[k];
-        unsigned long long lo = a.np_excl[k];
-        uint32_t kmer, qpos, c = c0;
+    for (uint32_t kb = k0; kb <= kend; kb += 32) {
+      // a lane per position: its first hit, k-mer, query anchor and call, with
+      // one wait for all of them
+      const uint32_t nk = min(kend - kb + 1, 32u);
+      uint32_t kmer = 0, qa = 0, c = c0;
+      unsigned long long lo = 0;
+      if (lane < nk) {
+        const uint32_t p = a.np_pos[kb + lane];
+        lo = a.np_excl[kb + lane];
         CallDev cd = call0;
         if (p >= next_off) {  // the tile reaches into a later call
           while (c + 1 < w.ncalls && w.calls[c + 1].pos_off <= p) c++;
           cd = w.calls[c];
         }
+        uint32_t qpos;
         if (a.np_kmer && !w.seeds) {
-          kmer = a.np_kmer[k];
+          kmer = a.np_kmer[kb + lane];
           qpos = cd.start + (p - cd.pos_off);
         } else {
           position_seed(w, cd, p, &qpos, &kmer);
         }
-        const uint32_t qa = cd.qoff + qpos + w.shape.size;
+        qa = cd.qoff + qpos + w.shape.size;
+      }
+      if constexpr (SPARSE) {
+        // a lane looks up its own position's seeds, kBatch at a time
         constexpr uint32_t kBatch = 5;
-        for (uint32_t v0 = 0; v0 < per; v0 += kBatch) {
-          uint32_t beg[kBatch], cnt[kBatch];
+        if (lane < nk)
+          for (uint32_t v0 = 0; v0 < per; v0 += kBatch) {
+            uint32_t beg[kBatch], cnt[kBatch];
 #pragma unroll
-          for (uint32_t u = 0; u < kBatch; u++) {
+            for (uint32_t u = 0; u < kBatch; u++) {
+              cnt[u] = 0;
+              beg[u] = 0;
+              if (v0 + u < per) cnt[u] = bucket(w, seed_variant(kmer, v0 + u), &beg[u]);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kBatch; u++) {
+              const unsigned long long hi = lo + cnt[u];
+              if (cnt[u] && hi > h0 && lo < h0 + nt) {
+                const unsigned long long first = lo > h0 ? lo : h0;
+                put_slot((uint32_t)(first - h0), beg[u] + (uint32_t)(first - lo), qa, c);
+              }
+              lo = hi;
+            }
+          }
+      } else {
+        // the lanes spread over (position, seed) pairs, the bucket bounds of
+        // up to kPasses passes loaded before any is used
+        constexpr uint32_t kPasses = 3;
+        for (uint32_t b = 0; b < nk; b += kPasses * ppi) {
+          uint32_t beg[kPasses], cnt[kPasses];
+#pragma unroll
+          for (uint32_t u = 0; u < kPasses; u++) {
             cnt[u] = 0;
             beg[u] = 0;
-            if (v0 + u < per) cnt[u] = bucket(w, seed_variant(kmer, v0 + u), &beg[u]);
-          }
-#pragma unroll
-          for (uint32_t u = 0; u < kBatch; u++) {
-            const unsigned long long hi = lo + cnt[u];
-            if (cnt[u] && hi > h0 && lo < h0 + nt) {
-              const unsigned long long first = lo > h0 ? lo : h0;
-              put_slot((uint32_t)(first - h0), beg[u] + (uint32_t)(first - lo), qa, c, cd);
+            if (b + u * ppi < nk) {
+              const uint32_t src = b + u * ppi + lpi;
+              const uint32_t km = __shfl_sync(0xffffffffu, kmer, src & 31u);
+              if (lpi < ppi && src < nk) cnt[u] = bucket(w, seed_variant(km, lvar), &beg[u]);
             }
-            lo = hi;
           }
-        }
-      }
-    } else {
-      for (uint32_t kb = k0; kb <= kend; kb += ppi) {
-        const uint32_t k = kb + lpi;
-        const bool act = lpi < ppi && k <= kend;
-        uint32_t cnt = 0, beg = 0, qa = 0, c = c0;
-        unsigned long long lo = 0;
-        CallDev cd = call0;
-        if (act) {
-          const uint32_t p = a.np_pos[k];
-          lo = a.np_excl[k];
-          uint32_t kmer, qpos;
-          if (p >= next_off) {  // the tile reaches into a later call
-            while (c + 1 < w.ncalls && w.calls[c + 1].pos_off <= p) c++;
-            cd = w.calls[c];
-          }
-          if (a.np_kmer && !w.seeds) {
-            kmer = a.np_kmer[k];
-            qpos = cd.start + (p - cd.pos_off);
-          } else {
-            position_seed(w, cd, p, &qpos, &kmer);
-          }
-          qa = cd.qoff + qpos + w.shape.size;
-          cnt = bucket(w, seed_variant(kmer, lvar), &beg);
-        }
-        // the position's earlier seeds' hits come first: inclusive scan of the
-        // counts over the position's lanes
-        uint32_t incl = cnt;
 #pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-          const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
-          if (lvar >= d) incl += up;
-        }
-        if (cnt) {
-          lo += incl - cnt;
-          const unsigned long long hi = lo + cnt;
-          if (hi > h0 && lo < h0 + nt) {
-            const unsigned long long first = lo > h0 ? lo : h0;
-            put_slot((uint32_t)(first - h0), beg + (uint32_t)(first - lo), qa, c, cd);
+          for (uint32_t u = 0; u < kPasses; u++) {
+            if (b + u * ppi >= nk) break;
+            const uint32_t src = (b + u * ppi + lpi) & 31u;
+            // the position's earlier seeds' hits come first: inclusive scan of
+            // the counts over the position's lanes
+            uint32_t incl = cnt[u];
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+              const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+              if (lvar >= d) incl += up;
+            }
+            const unsigned long long at = __shfl_sync(0xffffffffu, lo, src) + (incl - cnt[u]);
+            const uint32_t sq = __shfl_sync(0xffffffffu, qa, src), sc = __shfl_sync(0xffffffffu, c, src);
+            if (cnt[u] && at + cnt[u] > h0 && at < h0 + nt) {
+              const unsigned long long first = at > h0 ? at : h0;
+              put_slot((uint32_t)(first - h0), beg[u] + (uint32_t)(first - at), sq, sc);
+            }
           }
         }
       }
@@ -364,82 +403,36 @@ __global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_con
   };
 
   // The tile's next 32 hits, one per lane (the reference position and the
-  // slot), loaded a round before lanes take them.
+  // slot), loaded while the hits before them are scored.
   uint32_t pos_next = 0, slot_next = 0;
   auto fetch_hits = [&]() {
     const uint32_t t = cursor + lane;
     if (t < nt) {
       const uint32_t b = wt.bits[t >> 5] & (0xFFFFFFFFu >> (31u - (t & 31u)));
       slot_next = b ? (t & ~31u) + 31u - (uint32_t)__clz((int)b) : wt.carry[t >> 5];
-      pos_next = __ldg(w.pos_table + (slot[slot_next].x + t));
+      pos_next = __ldg(w.pos_table + (slot_x[slot_next] + t));
     }
-  };
-
-  // Lane state: its hit (anchors, call, index in the wave); the directions
-  // scored this round (act) and the one that waits for its turn; how far from
-  // the anchor the round's window stands; cells left to the edge or the cap
-  // per direction (right low half, left high half) and whether that is the
-  // cap; drawdowns at the round's start (halves); the summed bounds of the
-  // maxima; cells scored.
-  bool have = false, wait_left = false, cap_r = false, cap_l = false;
-  uint32_t act = 0, hr0 = 0, hq0 = 0, hcall = 0, left = 0, draw = 0, cells = 0;
-  int32_t off = 0, bound = 0;
-  unsigned long long hidx = 0;
-  constexpr uint32_t kGoRight = 1, kGoLeft = 2;
-
-  while (true) {
-    if (!claimed && !tiles_done && 2 * cursor >= nt) {
-      if (lane == 0) claim = atomicAdd(&a.tot->tiles, 1ull);
+    if (!claimed && 2 * cursor >= nt) {
+      if (lane == 0) claim = (uint32_t)atomicAdd(&a.tot->tiles, 1ull);
       claimed = true;
     } else if (claimed && !hdr) {
-      // a round after the claim: the claimed tile's header, copied into
-      // shared memory while this round is scored
-      const unsigned long long jn = __shfl_sync(0xffffffffu, claim, 0);
-      if (jn * (unsigned long long)tile < total && lane < 3)
+      // 32 hits after the claim: the claimed tile's header, copied into
+      // shared memory while hits are scored
+      const uint32_t jn = __shfl_sync(0xffffffffu, claim, 0);
+      if (jn * (unsigned long long)tile < wt.total && lane < 3)
         cp_async4(&wt.hdr[lane], lane == 0 ? a.tile_first + jn : lane == 1 ? a.tile_first + jn + 1 : a.tile_call + jn);
       cp_async_commit();
       hdr = true;
     }
-    // lanes without a hit take the tile's next ones; when the tile runs out
-    // the next one is set up at once, so that no round runs half empty
-    unsigned need = __ballot_sync(0xffffffffu, !have);
-    while (need && !tiles_done) {
-      if (cursor >= nt) {
-        next_tile();
-        if (tiles_done) break;
-        fetch_hits();
-      }
-      const uint32_t rank = (uint32_t)__popc(need & lanemask_lt());
-      const uint32_t sl = __shfl_sync(0xffffffffu, slot_next, rank);
-      const uint32_t pos = __shfl_sync(0xffffffffu, pos_next, rank);
-      if (!have && cursor + rank < nt) {
-        const uint4 s = slot[sl];
-        have = true;
-        hr0 = pos + w.shape.size;
-        hq0 = s.y;
-        hcall = s.z;
-        hidx = h0 + cursor + rank;
-        const uint32_t er = min(w.rlen - hr0, s.w & 0xFFFFu), el = min(hr0, s.w >> 16);
-        cap_r = er > a.cap;
-        cap_l = el > a.cap;
-        left = min(er, a.cap) | min(el, a.cap) << 16;
-        act = kGoRight | kGoLeft;
-        wait_left = false;
-        off = 0;
-        draw = 0;
-        bound = 0;
-        cells = 0;
-      }
-      cursor = min(cursor + (uint32_t)__popc(need), nt);
-      __syncwarp();
-      fetch_hits();
-      need = __ballot_sync(0xffffffffu, !have);
-    }
-    if (!__any_sync(0xffffffffu, have)) break;  // no hits left in the queue
-    // an idle lane scores the first window of each sequence
-    const uint32_t vr = have ? hr0 + (uint32_t)off : (uint32_t)kLeft, vq = have ? hq0 + (uint32_t)off : (uint32_t)kLeft;
-    if (!have) act = 0;
-    uint32_t Rc[kWinChunks], Qc[kWinChunks], sp[3];
+  };
+
+  // Scores one window per lane from the drawdowns `draw`: the minima and last
+  // costs of both extensions, one past the first drop of each direction (one
+  // past the window: none), one past the first special base.  `between` runs
+  // while the group states wait in shared memory.
+  auto score = [&](uint32_t vr, uint32_t vq, uint32_t draw, uint32_t &m2, uint32_t &P, uint32_t &drop,
+                   uint32_t &special, auto between) {
+    uint32_t Rc[kWinChunks], Qc[kWinChunks];
     {
       const uint4 *rp = a2.ref + ((vr + (64 - kLeft)) >> 5), *qp = a2.qry + ((vq + (64 - kLeft)) >> 5);
       uint4 rr[4], qr[4];
@@ -451,7 +444,15 @@ __global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_con
       window_codes(rr, vr, Rc, rs);
       window_codes(qr, vq, Qc, qs);
 #pragma unroll
-      for (int i = 0; i < 3; i++) sp[i] = rs[i] | qs[i];
+      for (int i = 0; i < 3; i++) rs[i] |= qs[i];
+      static_assert(kLeft == 56, "the special words below split at base 56");
+      // the first set bit, among the next 32 when there is none (a bit past
+      // the window stands for none at all)
+      const uint32_t r0 = __funnelshift_r(rs[1], rs[2], 24), r1 = rs[2] >> 24 | 1u << (kRight - 32);
+      const uint32_t l0 = __funnelshift_l(rs[0], rs[1], 8), l1 = rs[0] << 8 | 1u << (63 - kLeft);
+      const uint32_t sp_r = (uint32_t)__clz((int)__brev(r0 ? r0 : r1)) + (r0 ? 1u : 33u);
+      const uint32_t sp_l = (uint32_t)__clz((int)(l0 ? l0 : l1)) + (l0 ? 1u : 33u);
+      special = sp_l << 16 | sp_r;
     }
     uint2 sel[kWinChunks];
 #pragma unroll
@@ -465,7 +466,6 @@ __global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_con
     // dropped).  Flags: left group g at bit 31 - g, right group g at bit
     // 15 - kSolo - g.
     uint32_t flags = 0;
-    uint32_t m2, P;
     {
       uint32_t Ar = kCostBase + (draw & 0xFFFFu), Al = kCostBase + (draw >> 16), ml = kCostBase;
 #pragma unroll
@@ -509,112 +509,189 @@ __global__ void __launch_bounds__(kGateThreads, 4) gate2_kernel(const __grid_con
         flags |= ((hi - m2 + thr2) & 0x80008000u) >> (g + kSolo);
       }
     }
-    // The first dropping cell of each direction (kRight, kLeft: none): the
-    // eight cells of its first flagged group, both directions at once.  A
-    // drawdown runs biased by thr, floored at it, and shows in bit 15.  When
-    // seven largest scores can exceed xdrop a flag may be loose (the minimum
-    // fell after the drawdown): the next flagged group is looked at then.
+    between();
     __syncwarp();
-    uint32_t drop_r = kRight, drop_l = kLeft;
-    uint32_t todo = flags & ((act & kGoRight ? 0xFFFFu : 0u) | (act & kGoLeft ? 0xFFFF0000u : 0u));
-    while (__any_sync(0xffffffffu, todo != 0)) {
-      const uint32_t tl = todo & 0xFFFF0000u, tr = todo << 16;
-      const uint32_t gl = tl ? (uint32_t)__clz((int)tl) : 0u, gr = tr ? (uint32_t)__clz((int)tr) - kSolo : 0u;
-      const uint32_t fl = kGroupsL - 1 - gl, fr = kGroupsL + gr;
+    // One past the first dropping cell of each direction: the eight cells of
+    // its first flagged group, or of its last group when none is flagged, both
+    // directions at once.  A drawdown runs biased by thr, floored at it, and
+    // shows in bit 15; the cells from the drop on are counted, so none leaves
+    // one past the window.  When seven largest scores can exceed xdrop a flag
+    // may be loose (the minimum fell after the drawdown) and the next flagged
+    // group is looked at.
+    flags |= 0x80000000u >> (kGroupsL - 1) | 0x8000u >> (kGroupsL - 1);
+    while (true) {
+      // left group gl, right group gr - kSolo; their bases in the window
+      const uint32_t gl = (uint32_t)__clz((int)flags), gr = (uint32_t)__clz((int)(flags << 16));
+      const uint32_t fl = kGroupsL - 1 - gl, fr = kGroupsL - kSolo + gr;
       const uint2 wl = wt.sel[fl >> 1][lane], wr = wt.sel[fr >> 1][lane];
       const uint32_t shl = (fl & 1u) << 4, shr = (fr & 1u) << 4;
       const uint32_t le = tab.costs(wl.x >> shl), lo = tab.costs(wl.y >> shl), re = tab.costs(wr.x >> shr),
                      ro = tab.costs(wr.y >> shr);
-      uint32_t E = permute(wt.grp[gr + kSolo][lane], wt.grp[gl][lane], 0x7610u);
-      uint32_t F = 0;  // bits 15 and 31: the direction has dropped
-      int32_t after = 0;  // -128 * (cells from the drop on, right + 16 * left)
+      uint32_t E = permute(wt.grp[gr][lane], wt.grp[gl][lane], 0x7610u);
+      uint32_t F = 0;      // bits 15 and 31: the direction has dropped
+      uint32_t after = 0;  // 128 * (cells from the drop on: right + 16 * left)
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         // both cells' costs, sign-extended to 16 bits
         const uint32_t rb = (uint32_t)right_byte(k), lb = 4u + (uint32_t)left_byte(k);
         const uint32_t c2 = permute(right_word(k, re, ro), left_word(k, le, lo),
-                                        rb | (8u | rb) << 4 | lb << 8 | (8u | lb) << 12);
+                                    rb | (8u | rb) << 4 | lb << 8 | (8u | lb) << 12);
         E = __viaddmax_u16x2(E, c2, thr2);
         F = (F | E) & 0x80008000u;
-        after = __dp4a((int)F, 0x10000100, after);
+        after = __dp4a(F, 0x10000100u, after);
       }
-      const uint32_t n = (uint32_t)(-after) >> 7, n_r = n & 15u, n_l = n >> 4;
-      if (tr) {
-        if (n_r) drop_r = 8 * gr + 8 - n_r;
-        todo = n_r ? todo & 0xFFFF0000u : todo & ~(0x8000u >> (gr + kSolo));
-      }
-      if (tl) {
-        if (n_l) drop_l = 8 * gl + 8 - n_l;
-        todo = n_l ? todo & 0xFFFFu : todo & ~(0x80000000u >> gl);
-      }
+      const uint32_t n = ((after >> 7) * 0x1001u) & 0x000F000Fu;  // the two counts in halves
+      drop = gl * 0x80000u + gr * 8u + (9u << 16 | 9u) - 8u * kSolo - n;
+      if (a.late_max_safe) break;
+      const uint32_t loose = (gl < kGroupsL - 1 && !(n >> 16) ? 0x80000000u >> gl : 0u) |
+                             (gr < kGroupsL - 1 && !(n & 0xFFFFu) ? 0x8000u >> gr : 0u);
+      flags &= ~loose;
+      if (!__any_sync(0xffffffffu, loose)) break;
     }
     __syncwarp();
-    // the first special base on each side (kRight, kLeft: none)
-    uint32_t sp_r, sp_l;
-    {
-      static_assert(kLeft == 56, "the special words below split at base 56");
-      const uint32_t r0 = __funnelshift_r(sp[1], sp[2], 24), r1 = sp[2] >> 24;
-      const uint32_t l0 = __funnelshift_l(sp[0], sp[1], 8), l1 = sp[0] << 8;
-      sp_r = r0 ? (uint32_t)__ffs((int)r0) - 1u : r1 ? 31u + (uint32_t)__ffs((int)r1) : (uint32_t)kRight;
-      sp_l = l0 ? (uint32_t)__clz((int)l0) : l1 ? 32u + (uint32_t)__clz((int)l1) : (uint32_t)kLeft;
+  };
+
+  // the warp's ring of waiting hits
+  uint32_t *const ring = a2.ring + (size_t)(blockIdx.x * kGate2Warps + (threadIdx.x >> 5)) * (kRingFields * kRingCap);
+  uint32_t ring_head = 0, ring_n = 0;
+  // Adds the lanes' hits with `on` set to the ring.
+  auto push = [&](bool on, uint32_t r0, uint32_t q0, uint32_t call, uint32_t hit, uint32_t off, uint32_t draw,
+                  int32_t bound, uint32_t state) {
+    const unsigned going = __ballot_sync(0xffffffffu, on);
+    if (on) {
+      uint32_t *to = ring + ((ring_head + ring_n + (uint32_t)__popc(going & lanemask_lt())) & (kRingCap - 1));
+      to[kRingR * kRingCap] = r0;
+      to[kRingQ * kRingCap] = q0;
+      to[kRingCall * kRingCap] = call;
+      to[kRingHit * kRingCap] = hit;
+      to[kRingOff * kRingCap] = off;
+      to[kRingDraw * kRingCap] = draw;
+      to[kRingBound * kRingCap] = (uint32_t)bound;
+      to[kRingState * kRingCap] = state;
     }
-    // How each direction ends: a drop, a special base, the edge or the cap --
-    // or not in this round.
-    const uint32_t left_r = left & 0xFFFFu, left_l = left >> 16;
-    const uint32_t lim_r = min(left_r, (uint32_t)kRight), lim_l = min(left_l, (uint32_t)kLeft);
-    const bool ar = (act & kGoRight) != 0, al = (act & kGoLeft) != 0;
-    const bool dr = drop_r < min(lim_r, sp_r), dl = drop_l < min(lim_l, sp_l);
-    const bool sr = !dr && sp_r < lim_r, sl = !dl && sp_l < lim_l;
-    const bool er = !dr && !sr && left_r <= (uint32_t)kRight, el = !dl && !sl && left_l <= (uint32_t)kLeft;
-    const bool more_r = ar && !dr && !sr && !er, more_l = al && !dl && !sl && !el;
-    bool exact = (ar && er && cap_r) || (al && el && cap_l);  // past the cap
-    if (soft && ((ar && sr) || (al && sl))) {  // a special base that may not end the extension
-      int32_t worst = (int32_t)0x80000000;
-      if (ar && sr) worst = a.sub[w.ref[vr + sp_r] * kNuc + w.qbuf[vq + sp_r]];
-      if (al && sl) worst = max(worst, a.sub[w.ref[vr - 1u - sp_l] * kNuc + w.qbuf[vq - 1u - sp_l]]);
-      exact |= (long long)worst + a.xdrop >= 0;
+    ring_n += (uint32_t)__popc(going);
+    __syncwarp();
+  };
+  // A hit that becomes a candidate.
+  auto emit = [&](unsigned long long hit, uint32_t r0, uint32_t q0, uint32_t call) {
+    const uint32_t at = atomicAdd(&a.tot->cand, 1u);
+    if (at < a.cand_cap)
+      a.cand[at] = Cand{scope_of(a.scope_lo, min(a.tot->n_scopes, a.scope_cap), hit), r0, q0, call | kLongFlag, 0, 0};
+  };
+  // Whether a special base that ends a direction (one past it: sp) may not do
+  // so by its score alone.
+  auto soft_end = [&](uint32_t r, uint32_t q) {
+    return (long long)a.sub[w.ref[r] * kNuc + w.qbuf[q]] + a.xdrop >= 0;
+  };
+  constexpr uint32_t kMoreBias = (0x7FFFu - kLeft) << 16 | (0x7FFFu - kRight);  // sets a half's top bit past the window
+
+  if (lane == 0) {
+    wt.total = a.tot->hits;
+    wt.nz = a.tot->nz;
+  }
+  __syncwarp();
+  next_tile();
+  if (nt) fetch_hits();
+  while (true) {
+    if (cells_acc >= 1u << 30) {
+      atomicAdd(&a.tot->cells, (unsigned long long)cells_acc);
+      cells_acc = 0;
     }
-    if (ar) {
-      cells += dr ? drop_r + 1 : sr ? sp_r + 1 : lim_r;
-      bound += (int32_t)(kCostBase - (m2 & 0xFFFFu));
-    }
-    if (al) {
-      cells += dl ? drop_l + 1 : sl ? sp_l + 1 : lim_l;
-      bound += (int32_t)(kCostBase - (m2 >> 16));
-    }
-    if (have) {
-      if (!exact && (more_r || more_l || wait_left)) {  // another round for this hit
-        const uint32_t m = (ar ? 0xFFFFu : 0u) | (al ? 0xFFFF0000u : 0u);
-        draw = ((P - m2) & m) | (draw & ~m);
-        if (more_l) left -= (uint32_t)kLeft << 16;
-        if (more_r) {  // the right extension first; the left one waits if it goes on as well
-          left -= kRight;
-          wait_left |= more_l;
-          act = kGoRight;
-          off += kRight;
-        } else {
-          // to the left: from where its first round ended, or on from there
-          off = wait_left ? -kLeft : off - kLeft;
-          wait_left = false;
-          act = kGoLeft;
-        }
-      } else {
-        const bool maybe = a.total_exact ? bound >= a.hspthresh
-                                         : sat_i32((double)__int2float_rn(bound)) >= a.hspthresh;
-        if (exact || maybe) {
-          const uint32_t at = atomicAdd(&a.tot->cand, 1u);
-          if (at < a.cand_cap)
-            a.cand[at] = Cand{scope_of(a.scope_lo, min(a.tot->n_scopes, a.scope_cap), hidx), hr0, hq0,
-                              hcall | kLongFlag, 0, 0};
-        } else {
-          cells_acc += cells;
-        }
-        have = false;
+    if (ring_n < 32 && cursor < nt) {
+      // 32 fresh hits of the tile; a lane without one scores the first window
+      // of each sequence
+      const bool have = cursor + lane < nt;
+      const uint32_t hit = tile_at * (tile >> 5) + (cursor >> 5);
+      const uint32_t vr = have ? pos_next + w.shape.size : (uint32_t)kLeft;
+      const uint32_t vq = have ? slot_q[slot_next] : (uint32_t)kLeft, call = have ? slot_call[slot_next] : 0u;
+      uint32_t m2, P, drop, special;
+      score(vr, vq, 0u, m2, P, drop, special, [&]() {
+        cursor += 32;
+        if (cursor >= nt) next_tile();
+        if (nt) fetch_hits();
+      });
+      // Cells scored: through the drop or the special base, to the edge or
+      // the cap -- or more than the window holds, and the direction goes on.
+      const CallDev cd = w.calls[call];
+      const uint32_t er = min(w.rlen - vr, cd.qoff + cd.qlen - vq), el = min(vr, vq - cd.qoff);
+      const uint32_t ends = min_halves(drop, special);
+      const uint32_t use = min_halves(ends, min(er, a.cap) | min(el, a.cap) << 16);
+      const uint32_t more = (use + kMoreBias) & 0x80008000u;
+      const bool more_r = (more & 0x8000u) != 0, more_l = (int32_t)more < 0;
+      bool exact = false;
+      if (a.cap <= (uint32_t)kLeft)  // past the cap
+        exact = (er > a.cap && a.cap <= (uint32_t)kRight && (use & 0xFFFFu) < (ends & 0xFFFFu)) ||
+                (el > a.cap && (use >> 16) < (ends >> 16));
+      if (soft && have) {
+        const uint32_t sp_r = special & 0xFFFFu, sp_l = special >> 16;
+        if (sp_r <= (uint32_t)kRight && sp_r == (use & 0xFFFFu)) exact |= soft_end(vr + sp_r - 1u, vq + sp_r - 1u);
+        if (sp_l <= (uint32_t)kLeft && sp_l == use >> 16) exact |= soft_end(vr - sp_l, vq - sp_l);
       }
+      const uint32_t cells = (use & 0xFFFFu) + (use >> 16) - (more_r ? 1u : 0u) - (more_l ? 1u : 0u);
+      const int32_t bound = (int32_t)(2u * kCostBase - (m2 & 0xFFFFu) - (m2 >> 16));
+      const bool on = have && more && !exact;
+      const bool cand = have && !on && (exact || bound >= a2.min_total);
+      cells_acc += have && !on && !cand ? cells : 0u;
+      if (cand) emit(hit * 32ull + lane, vr, vq, call);
+      // the right extension goes on first; the left one waits if it does too
+      push(on, vr, vq, call, hit, more_r ? (uint32_t)kRight : (uint32_t)-kLeft, P - m2, bound,
+           (more_r ? kGoRight | (more_l ? kWaitLeft : 0u) : kGoLeft) | lane << 3 | cells << 8);
+    } else if (ring_n) {
+      // up to 32 waiting hits, from where they stand
+      const uint32_t n = min(ring_n, 32u);
+      const bool have = lane < n;
+      uint32_t r0 = kLeft, q0 = kLeft, call = 0, hit = 0, off = 0, was = 0, state = 0;
+      int32_t bound = 0;
+      if (have) {
+        const uint32_t *at = ring + ((ring_head + lane) & (kRingCap - 1));
+        r0 = at[kRingR * kRingCap];
+        q0 = at[kRingQ * kRingCap];
+        call = at[kRingCall * kRingCap];
+        hit = at[kRingHit * kRingCap];
+        off = at[kRingOff * kRingCap];
+        was = at[kRingDraw * kRingCap];
+        bound = (int32_t)at[kRingBound * kRingCap];
+        state = at[kRingState * kRingCap];
+      }
+      ring_head += n;
+      ring_n -= n;
+      __syncwarp();  // every lane has its entry before new ones overwrite it
+      const uint32_t vr = r0 + off, vq = q0 + off;
+      const bool on_r = (state & kGoRight) != 0, on_l = (state & kGoLeft) != 0;
+      uint32_t m2, P, drop, special;
+      score(vr, vq, was, m2, P, drop, special, []() {});
+      // cells left to the edge or the cap; a left extension that waits has
+      // one window behind it
+      const CallDev cd = w.calls[call];
+      const uint32_t er = min(w.rlen - r0, cd.qoff + cd.qlen - q0), el = min(r0, q0 - cd.qoff);
+      const uint32_t left_r = min(er, a.cap) - off, left_l = min(el, a.cap) + off;
+      const uint32_t ends_r = min(drop & 0xFFFFu, special & 0xFFFFu), ends_l = min(drop >> 16, special >> 16);
+      const uint32_t use_r = on_r ? min(ends_r, left_r) : 0u, use_l = on_l ? min(ends_l, left_l) : 0u;
+      const bool more_r = use_r > (uint32_t)kRight, more_l = use_l > (uint32_t)kLeft;
+      bool exact = (on_r && er > a.cap && use_r < ends_r && !more_r) || (on_l && el > a.cap && use_l < ends_l && !more_l);
+      if (soft && have) {
+        if (on_r && ends_r == (special & 0xFFFFu) && use_r == ends_r && !more_r)
+          exact |= soft_end(vr + use_r - 1u, vq + use_r - 1u);
+        if (on_l && ends_l == special >> 16 && use_l == ends_l && !more_l) exact |= soft_end(vr - use_l, vq - use_l);
+      }
+      const uint32_t cells = (state >> 8) + use_r + use_l - (more_r ? 1u : 0u) - (more_l ? 1u : 0u);
+      bound += (int32_t)((on_r ? kCostBase - (m2 & 0xFFFFu) : 0u) + (on_l ? kCostBase - (m2 >> 16) : 0u));
+      const bool waits = (state & kWaitLeft) != 0;
+      const bool on = have && !exact && (more_r || more_l || waits);
+      const bool cand = have && !on && (exact || bound >= a2.min_total);
+      cells_acc += have && !on && !cand ? cells : 0u;
+      if (cand) emit(hit * 32ull + (state >> 3 & 31u), r0, q0, call);
+      const uint32_t m = (on_r ? 0xFFFFu : 0u) | (on_l ? 0xFFFF0000u : 0u);
+      push(on, r0, q0, call, hit, more_r ? off + kRight : waits ? (uint32_t)-kLeft : off - kLeft,
+           ((P - m2) & m) | (was & ~m), bound,
+           (more_r ? kGoRight | (state & kWaitLeft) : kGoLeft) | (state & 31u << 3) | cells << 8);
+    } else {
+      break;
     }
   }
-  for (int d = 16; d > 0; d >>= 1) cells_acc += __shfl_down_sync(0xffffffffu, cells_acc, d);
-  if (lane == 0 && cells_acc) atomicAdd(&a.tot->cells, cells_acc);
+  unsigned long long sum = cells_acc;
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, d);
+  if (lane == 0 && sum) atomicAdd(&a.tot->cells, sum);
 }
 
 }  // namespace hz

@@ -228,12 +228,13 @@ int hz_engine_profile_reset(hz_engine *e);
 
 /* Launch-shape knobs (no reference counterpart; results never depend on
  * them): "gate_version" (2, the default: the lockstep gate over 2-bit packed
- * sequences, used whenever every ACGT score fits a signed byte; 1: the
+ * sequences, used whenever every ACGT score lies in -127..127; 1: the
  * lane-refill gate over 8-bit codes, which also serves wider scores),
  * "gate_sparse" (the lockstep gate's tile setup: -1, the default, chosen
  * from the target's average bucket; 0 a lane per (position, seed) pair;
  * 1 a lane per position, for targets whose tiles span many positions),
- * "gate_tile" (hits per gate warp tile: 64, 128, 256),
+ * "gate_tile" (hits per gate warp tile: 64, 128, 256; unless set, what suits
+ * the gate that runs: 256 for the lockstep gate, 128 for the lane-refill one),
  * "gate_cap" (cells per direction before a hit leaves the gate as a long
  * candidate -- for the lane-per-candidate long kernel after the lockstep
  * gate, for the warp kernel after the lane-refill gate -- multiple of 8,
