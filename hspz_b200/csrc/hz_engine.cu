@@ -359,12 +359,17 @@ struct hz_engine {
   DBuf<SegmentPair> raw;
   HBuf<CallDev> h_calls;
   HBuf<WaveTotals> h_tot;
-  HBuf<hz_segment_pair> h_raw;
-  HBuf<uint32_t> h_raw_scope, h_scope_call;
+  HBuf<uint32_t> h_scope_call;
   // device dedup of the batched form
   bool device_dedup = true;
   uint32_t device_dedup_min = 1u << 16;  // raw HSPs from which a per-call wave dedups on the device
-  DBuf<uint32_t> d_perm_a, d_perm_b, d_keys_a, d_keys_b, d_keep, d_keep_excl, d_hist, d_hpart, d_total;
+  // the wave's different HSPs: the hash set that finds them (2 raw_cap words),
+  // their indices (raw_cap words) and the first kRawPrefix of them; and the
+  // sorts' buffers
+  DBuf<uint32_t> d_set;
+  uint32_t *distinct() const { return d_set.p + 2 * (size_t)raw_cap; }
+  ScopedHspOut *distinct_head() const { return reinterpret_cast<ScopedHspOut *>(d_set.p + ((3 * (size_t)raw_cap + 3) & ~(size_t)3)); }
+  DBuf<uint32_t> d_perm_a, d_perm_b, d_kept, d_total;
   DBuf<ScopedHspOut> d_out;
   HBuf<ScopedHspOut> h_out;
   uint32_t cand_cap = 1u << 20, raw_cap = 1u << 20, scope_cap = 0;
@@ -645,75 +650,44 @@ template <int TW> int launch_gate(hz_engine *e, const GateArgs &ga) {
 // nothing was kept, and the caller reruns the calls in smaller waves.
 constexpr int kSplitWave = 1;
 
-// Runs calls[0..n) as one wave and appends its deduped HSPs, in call order
-// and LASTZ order within each MAX_HITS scope, to *out.  `seeds` (device) is
-// the uploaded seed array of a single-call wave, or null.
-// dedup_and_order of every scope of a wave on the device (hz_dedup.cuh);
-// appends the kept HSPs, in scope order and LASTZ order within each scope.
-int dedup_on_device(hz_engine *e, uint32_t nraw, uint32_t n_scopes, uint32_t call_base, std::vector<WaveRecord> *out,
+// dedup_and_order of every scope of a wave on the device (hz_dedup.cuh): the
+// wave's n different HSPs are sorted, filtered and sorted again; appends the
+// kept ones, in scope order and LASTZ order within each scope.
+int dedup_on_device(hz_engine *e, uint32_t n, uint32_t n_scopes, uint32_t call_base, std::vector<WaveRecord> *out,
                     hz_stats *st) {
   cudaStream_t s = e->st;
-  TRY(e->d_perm_a.ensure(nraw, s));
-  TRY(e->d_perm_b.ensure(nraw, s));
-  TRY(e->d_keys_a.ensure(nraw, s));
-  TRY(e->d_keys_b.ensure(nraw, s));
-  TRY(e->d_keep.ensure(nraw, s));
-  TRY(e->d_keep_excl.ensure(nraw, s));
-  uint64_t rtiles = (nraw + kRadixTile - 1) / kRadixTile;
-  TRY(e->d_hist.ensure(rtiles * kRadixBins, s));
-  TRY(e->d_hpart.ensure(scan_tiles(std::max<uint64_t>(rtiles * kRadixBins, nraw)) + 1, s));
+  TRY(e->d_perm_a.ensure(n, s));
+  TRY(e->d_perm_b.ensure(n, s));
+  TRY(e->d_kept.ensure(n, s));
   TRY(e->d_total.ensure(1, s));
-  const unsigned g = grid_for(nraw, 256);
-  TRY(e->launch("dedup", [&] { iota_kernel<<<g, 256, 0, s>>>(e->d_perm_a.p, nraw); }));
-  uint32_t scope_bytes = 1;
-  while (scope_bytes < 4 && (n_scopes >> (8 * scope_bytes))) scope_bytes++;
-  // stable LSD passes over the fields of a key, least significant first
-  auto sort_by = [&](const int *fields, int nf, uint32_t cnt) -> int {
-    uint64_t tiles = (cnt + kRadixTile - 1) / kRadixTile;
-    for (int fi = 0; fi < nf; fi++) {
-      int f = fields[fi];
-      TRY(e->launch("dedup", [&] {
-        gather_key_kernel<<<grid_for(cnt, 256), 256, 0, s>>>(e->raw.p, e->raw_scope.p, e->d_perm_a.p, cnt, f,
-                                                            e->d_keys_a.p);
-      }));
-      int passes = f == kScope ? (int)scope_bytes : 4;
-      for (int p = 0; p < passes; p++) {
-        int shift = 8 * p;
-        TRY(e->launch("dedup", [&] {
-          radix_hist_kernel<<<(unsigned)tiles, kRadixThreads, 0, s>>>(e->d_keys_a.p, cnt, shift, e->d_hist.p, tiles);
-          exclusive_scan<uint32_t>(e->d_hist.p, e->d_hist.p, tiles * kRadixBins, e->d_hpart.p, e->d_total.p, s);
-          radix_scatter_kernel<<<(unsigned)tiles, kRadixThreads, 0, s>>>(e->d_keys_a.p, e->d_perm_a.p, cnt, shift,
-                                                                        e->d_hist.p, tiles, e->d_keys_b.p,
-                                                                        e->d_perm_b.p);
-        }, 5));
-        std::swap(e->d_keys_a, e->d_keys_b);
-        std::swap(e->d_perm_a, e->d_perm_b);
-      }
-    }
-    return HZ_OK;
-  };
-  static const int by_diagonal_key[5] = {kScoreDesc, kLen, kRefStart, kDiag, kScope};
-  static const int by_lastz_key[5] = {kScoreDesc, kLen, kRefStart, kQueryStart, kScope};
-  TRY(sort_by(by_diagonal_key, 5, nraw));
+  TRY(e->d_out.ensure(n, s));
+  // the kept records come back with their number, unless they are many
+  const uint32_t first = std::min<uint32_t>(n, 1u << 16);
+  TRY(e->h_out.ensure(first));
+  TRY(e->h_scope_call.ensure(n_scopes + 1));
+  CK(cudaMemsetAsync(e->d_total.p, 0, 4, s));
+  const int passes = merge_passes(n);
   TRY(e->launch("dedup", [&] {
-    keep_flag_kernel<<<g, 256, 0, s>>>(e->raw.p, e->raw_scope.p, e->d_perm_a.p, nraw, e->d_keep.p);
-    exclusive_scan<uint32_t>(e->d_keep.p, e->d_keep_excl.p, nraw, e->d_hpart.p, e->d_total.p, s);
-    compact_perm_kernel<<<g, 256, 0, s>>>(e->d_perm_a.p, e->d_keep_excl.p, e->d_keep.p, nraw, e->d_perm_b.p);
-  }, 5));
+    SortArgs<SegmentPair> sa{e->raw.p, e->raw_scope.p, e->distinct(), nullptr, n, nullptr};
+    sort_indices<kByDiagonal>(sa, e->d_perm_a.p, e->d_perm_b.p, s);
+    sa.idx = passes & 1 ? e->d_perm_b.p : e->d_perm_a.p;
+    keep_kernel<<<grid_for(n, 256), 256, 0, s>>>(sa, e->d_kept.p, e->d_total.p);
+    sa.idx = e->d_kept.p;
+    sa.n_dev = e->d_total.p;
+    sort_indices<kByLastz>(sa, e->d_perm_a.p, e->d_perm_b.p, s);
+    emit_scoped_kernel<<<grid_for(n, 256), 256, 0, s>>>(e->raw.p, e->raw_scope.p, e->d_perm_a.p, e->d_perm_b.p,
+                                                       e->d_total.p, e->d_out.p);
+  }, 4 + 2 * passes));
   uint32_t kept = 0;
   CK(cudaMemcpyAsync(&kept, e->d_total.p, 4, cudaMemcpyDeviceToHost, s));
-  TRY(e->sync());
-  std::swap(e->d_perm_a, e->d_perm_b);
-  TRY(sort_by(by_lastz_key, 5, kept));
-  TRY(e->d_out.ensure(kept + 1, s));
-  TRY(e->h_out.ensure(kept + 1));
-  TRY(e->h_scope_call.ensure(n_scopes + 1));
-  TRY(e->launch("dedup", [&] {
-    emit_scoped_kernel<<<grid_for(kept, 256), 256, 0, s>>>(e->raw.p, e->raw_scope.p, e->d_perm_a.p, kept, e->d_out.p);
-  }));
-  CK(cudaMemcpyAsync(e->h_out.p, e->d_out.p, (size_t)kept * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(e->h_out.p, e->d_out.p, (size_t)first * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(e->h_scope_call.p, e->scope_call.p, (size_t)n_scopes * 4, cudaMemcpyDeviceToHost, s));
   TRY(e->sync());
+  if (kept > first) {
+    TRY(e->h_out.ensure(kept));
+    CK(cudaMemcpyAsync(e->h_out.p, e->d_out.p, (size_t)kept * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
+    TRY(e->sync());
+  }
   for (uint32_t i = 0; i < kept; i++) {
     const ScopedHspOut &r = e->h_out.p[i];
     out->push_back(WaveRecord{e->h_scope_call.p[r.scope] + call_base,
@@ -767,19 +741,21 @@ template <typename F> int run_captured(hz_engine *e, F &&chain) {
   return HZ_OK;
 }
 
-// The host side of a wave's dedup: the wave's raw HSPs and their scopes,
-// already read back into e->h_raw / h_raw_scope / h_scope_call, are grouped by
+// The host side of a wave's dedup: the wave's n different HSPs with their
+// scopes, already read back into e->h_out (and e->h_scope_call), are grouped by
 // scope and deduped per scope; the records go to *out in scope order, with
 // their wave-relative call index plus `call_base`.
-void host_dedup(hz_engine *e, uint32_t nraw, uint32_t n_scopes, uint32_t call_base, std::vector<WaveRecord> *out,
+void host_dedup(hz_engine *e, uint32_t n, uint32_t n_scopes, uint32_t call_base, std::vector<WaveRecord> *out,
                 hz_stats *st) {
+  const ScopedHspOut *h = e->h_out.p;
   // counting sort by scope
   std::vector<uint32_t> start(n_scopes + 1, 0);
-  for (uint32_t i = 0; i < nraw; i++) start[e->h_raw_scope.p[i] + 1]++;
+  for (uint32_t i = 0; i < n; i++) start[h[i].scope + 1]++;
   for (uint32_t k = 0; k < n_scopes; k++) start[k + 1] += start[k];
-  std::vector<hz_segment_pair> sorted(nraw);
+  std::vector<hz_segment_pair> sorted(n);
   std::vector<uint32_t> cur(start.begin(), start.end() - 1);
-  for (uint32_t i = 0; i < nraw; i++) sorted[cur[e->h_raw_scope.p[i]]++] = e->h_raw.p[i];
+  for (uint32_t i = 0; i < n; i++)
+    sorted[cur[h[i].scope]++] = hz_segment_pair{h[i].h.ref_start, h[i].h.query_start, h[i].h.len, h[i].h.score};
   for (uint32_t k = 0; k < n_scopes; k++) {
     size_t a = start[k], b = start[k + 1];
     if (a == b) continue;
@@ -794,22 +770,25 @@ void host_dedup(hz_engine *e, uint32_t nraw, uint32_t n_scopes, uint32_t call_ba
 // next call's run_wave, which runs it after launching its own kernels, so the
 // host sort overlaps the device work.  The engine's host read-back buffers
 // stay untouched until then: the next wave refills them only after its sync.
-// Raw HSPs and scopes a plain call reads back with its totals (40 KB).
-constexpr uint32_t kRawPrefix = 2048;
-constexpr uint32_t kScopePrefix = 64;
-
 struct DeferredDedup {
   bool pending = false;
-  uint32_t nraw = 0, n_scopes = 0, call_base = 0;
+  uint32_t n = 0, n_scopes = 0, call_base = 0;
   std::vector<WaveRecord> *out = nullptr;
   hz_stats *st = nullptr;
   void finish(hz_engine *e) {
     if (!pending) return;
     pending = false;
-    host_dedup(e, nraw, n_scopes, call_base, out, st);
+    host_dedup(e, n, n_scopes, call_base, out, st);
   }
 };
 
+// Different HSPs and scopes a plain call reads back with its totals (40 KB).
+constexpr uint32_t kRawPrefix = 2048;
+constexpr uint32_t kScopePrefix = 64;
+
+// Runs calls[0..n) as one wave and appends its deduped HSPs, in call order
+// and LASTZ order within each MAX_HITS scope, to *out.  `seeds` (device) is
+// the uploaded seed array of a single-call wave, or null.
 // With `defer`, a wave deduped on the host leaves that step in *defer (see
 // DeferredDedup) and the records of an earlier deferred wave are emitted once
 // this wave's kernels are queued; `call_base` is added to the call index of
@@ -879,6 +858,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     }
     TRY(e->raw.ensure(e->raw_cap, s));
     TRY(e->raw_scope.ensure(e->raw_cap, s));
+    TRY(e->d_set.ensure(3 * (size_t)e->raw_cap + 4 + kRawPrefix * sizeof(ScopedHspOut) / 4, s));
     TRY(e->tile_first.ensure(e->tile_cap, s));
     TRY(e->tile_call.ensure(e->tile_cap, s));
     // The wave's device chain: no host round trip between its launches, so
@@ -963,24 +943,29 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       TRY(e->launch("exact", [&] {
         exact_kernel<<<(unsigned)(e->sm_count * 8), kExactThreads, 0, s>>>(xa);
       }));
+      const uint32_t set_slots = (uint32_t)std::min<uint64_t>(2ull * e->raw_cap, 0xFFFFFFFFull);
+      CK(cudaMemsetAsync(e->d_set.p, 0, (size_t)set_slots * 4, s));
+      TRY(e->launch("distinct", [&] {
+        unique_kernel<<<(unsigned)(e->sm_count * 4), 256, 0, s>>>(e->raw.p, e->raw_scope.p, &e->tot.p->raw,
+                                                                e->raw_cap, e->d_set.p, set_slots, e->distinct(),
+                                                                &e->tot.p->distinct, e->distinct_head(), kRawPrefix);
+      }));
       CK(cudaMemcpyAsync(e->h_tot.p, e->tot.p, sizeof(WaveTotals), cudaMemcpyDeviceToHost, s));
       return HZ_OK;
     };
     if (graph) TRY(run_captured(e, chain));
     else TRY(chain());
     if (defer) defer->finish(e);  // the previous call's host dedup, while this call's kernels run
-    // A single-call wave (the plain form) reads back the first raw HSPs and
-    // scopes with its totals, so one with few raw HSPs (the usual case) needs
-    // one sync, not two.
+    // A single-call wave (the plain form) reads back the first different HSPs
+    // and scopes with its totals, so one with few of them (the usual case)
+    // needs one sync, not two.
     uint32_t pre_raw = 0, pre_scopes = 0;
     if (n == 1 && !device_dedup) {
-      pre_raw = std::min<uint32_t>(kRawPrefix, e->raw_cap);
+      pre_raw = kRawPrefix;
       pre_scopes = std::min<uint32_t>(kScopePrefix, scope_cap + 1);
-      TRY(e->h_raw.ensure(pre_raw));
-      TRY(e->h_raw_scope.ensure(pre_raw));
+      TRY(e->h_out.ensure(pre_raw));
       TRY(e->h_scope_call.ensure(pre_scopes));
-      CK(cudaMemcpyAsync(e->h_raw.p, e->raw.p, (size_t)pre_raw * sizeof(SegmentPair), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(e->h_raw_scope.p, e->raw_scope.p, (size_t)pre_raw * 4, cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(e->h_out.p, e->distinct_head(), (size_t)pre_raw * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
       CK(cudaMemcpyAsync(e->h_scope_call.p, e->scope_call.p, (size_t)pre_scopes * 4, cudaMemcpyDeviceToHost, s));
     }
     TRY(e->sync());
@@ -1013,39 +998,42 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     if (again) continue;  // a capacity was too small: run the wave again with larger buffers
 
     // per-scope dedup on the host, in scope order
-    uint32_t nraw = t.raw;
     e->cand_seen += t.cand;
     if (st) {
       st->hits += t.hits;
       st->cells += t.cells;
       st->seeds += t.valid * w.per_pos;
-      st->raw_hsps += nraw;
+      st->raw_hsps += t.raw;
       st->calls += n;
     }
-    if (nraw == 0) return HZ_OK;
+    const uint32_t nh = t.distinct;
+    if (nh == 0) return HZ_OK;
     // per-call waves (the plain form) dedup on the host like the reference,
-    // unless the call holds so many raw HSPs that the device sort is faster
-    if (device_dedup || (e->device_dedup && nraw >= e->device_dedup_min))
-      return dedup_on_device(e, nraw, t.n_scopes, call_base, out, st);
-    if (nraw > pre_raw || t.n_scopes > pre_scopes) {  // not all read back with the totals
-      TRY(e->h_raw.ensure(nraw));
-      TRY(e->h_raw_scope.ensure(nraw));
+    // unless the call holds so many HSPs that the device sort is faster
+    if (device_dedup || (e->device_dedup && nh >= e->device_dedup_min))
+      return dedup_on_device(e, nh, t.n_scopes, call_base, out, st);
+    if (nh > pre_raw || t.n_scopes > pre_scopes) {  // not all read back with the totals
+      TRY(e->d_out.ensure(nh, s));
+      TRY(e->h_out.ensure(nh));
       TRY(e->h_scope_call.ensure(t.n_scopes + 1));
-      CK(cudaMemcpyAsync(e->h_raw.p, e->raw.p, (size_t)nraw * sizeof(SegmentPair), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(e->h_raw_scope.p, e->raw_scope.p, (size_t)nraw * 4, cudaMemcpyDeviceToHost, s));
+      TRY(e->launch("dedup", [&] {
+        gather_scoped_kernel<<<grid_for(nh, 256), 256, 0, s>>>(e->raw.p, e->raw_scope.p, e->distinct(), nh,
+                                                              e->d_out.p);
+      }));
+      CK(cudaMemcpyAsync(e->h_out.p, e->d_out.p, (size_t)nh * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
       CK(cudaMemcpyAsync(e->h_scope_call.p, e->scope_call.p, (size_t)t.n_scopes * 4, cudaMemcpyDeviceToHost, s));
       TRY(e->sync());
     }
     if (defer) {
       defer->pending = true;
-      defer->nraw = nraw;
+      defer->n = nh;
       defer->n_scopes = t.n_scopes;
       defer->call_base = call_base;
       defer->out = out;
       defer->st = st;
       return HZ_OK;
     }
-    host_dedup(e, nraw, t.n_scopes, call_base, out, st);
+    host_dedup(e, nh, t.n_scopes, call_base, out, st);
     return HZ_OK;
   }
   return fail(HZ_E_OOM, "wave buffers kept overflowing");
@@ -1333,11 +1321,9 @@ void hz_engine_destroy(hz_engine *e) {
   e->raw.release();
   e->h_calls.release();
   e->h_tot.release();
-  e->h_raw.release();
-  e->h_raw_scope.release();
   e->h_scope_call.release();
-  for (auto *b : {&e->d_perm_a, &e->d_perm_b, &e->d_keys_a, &e->d_keys_b, &e->d_keep, &e->d_keep_excl, &e->d_hist,
-                  &e->d_hpart, &e->d_total, &e->tile_first, &e->tile_call})
+  for (auto *b : {&e->d_set, &e->d_perm_a, &e->d_perm_b, &e->d_kept, &e->d_total, &e->tile_first,
+                  &e->tile_call})
     b->release();
   e->d_out.release();
   e->h_out.release();
@@ -1889,78 +1875,23 @@ int hz_run_batched(hz_engine *e, hz_batch_record **out, uint64_t *n, hz_stats *s
 // program whose own allocator owns the whole device, a serving loop that
 // admits work against a fixed memory budget, or a plugin that must not grow
 // the process's footprint behind its host's back.  For them this entry point
-// runs the batched form's device dedup (radix passes, containment, LASTZ
+// runs the batched form's device dedup (merge sorts, containment, LASTZ
 // order) on a fixed scratch array compiled into this library instead of on
 // engine buffers.
 
 namespace {
 
 constexpr uint32_t kNoAllocMax = HZ_NOALLOC_MAX_HSPS;
-constexpr uint32_t kNoAllocTiles = (kNoAllocMax + kRadixTile - 1) / kRadixTile;
-constexpr uint32_t kNoAllocHist = kNoAllocTiles * kRadixBins;
-constexpr uint32_t kNoAllocPartials = kNoAllocHist / kScanTile + 2;
-// u32 words: perm_a, perm_b, keys_a, keys_b, dropped flags (kNoAllocMax each),
-// radix histograms, scan partials, scan total, kept count
-constexpr size_t kNoAllocWords = 5ull * kNoAllocMax + kNoAllocHist + kNoAllocPartials + 2;
+// u32 words: two index buffers, the kept records' indices, their number
+constexpr size_t kNoAllocWords = 3ull * kNoAllocMax + 1;
 
 }  // namespace
 
-// The scratch: ~6 MB that every GPU which loads this library holds until the
+// The scratch: ~3 MB that every GPU which loads this library holds until the
 // process exits.  Shared by every call; it keeps the last call's contents.
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
 namespace {
-
-// Unaligned-tolerant view of hz_segment_pair (the caller's buffers need only
-// 4-byte alignment).
-struct PlainHsp {
-  uint32_t ref_start, query_start, len;
-  int32_t score;
-};
-
-constexpr int kDroppedField = 6;
-
-__global__ void na_gather_kernel(const PlainHsp *__restrict__ in, const uint32_t *__restrict__ perm,
-                                 const uint32_t *__restrict__ dropped, uint32_t n, int field,
-                                 uint32_t *__restrict__ keys) {
-  uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    uint32_t r = perm[i];
-    if (field == kDroppedField) {
-      keys[i] = dropped[r];
-      continue;
-    }
-    SegmentPair h{in[r].ref_start, in[r].query_start, in[r].len, in[r].score};
-    keys[i] = field_key(h, 0u, field);
-  }
-}
-
-// After the hspComp sort: a record is dropped when it is contained in the
-// previous input record (src/hsp.rs:94-126); kept ones are counted.
-__global__ void na_flag_kernel(const PlainHsp *__restrict__ in, const uint32_t *__restrict__ perm, uint32_t n,
-                               uint32_t *__restrict__ dropped, uint32_t *__restrict__ kept) {
-  uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    uint32_t r = perm[i];
-    bool d = false;
-    if (i > 0) {
-      const PlainHsp &a = in[perm[i - 1]], &b = in[r];
-      d = contained_dev(SegmentPair{a.ref_start, a.query_start, a.len, a.score},
-                        SegmentPair{b.ref_start, b.query_start, b.len, b.score});
-    }
-    dropped[r] = d;
-    if (!d) atomicAdd(kept, 1u);
-  }
-}
-
-__global__ void na_copy_kernel(const PlainHsp *__restrict__ in, const uint32_t *__restrict__ perm,
-                               const uint32_t *__restrict__ kept, PlainHsp *__restrict__ out,
-                               uint32_t *__restrict__ n_out) {
-  const uint32_t k = *kept;
-  uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += stride) out[i] = in[perm[i]];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *n_out = k;
-}
 
 // The unique id of the calling thread's current CUDA context (0 if there is
 // none or the driver cannot say).  Ids are never reused within a process, so
@@ -2040,40 +1971,22 @@ int hz_dedup_and_order_device_noalloc(const hz_segment_pair *d_in, uint32_t n, h
   uint32_t *base = nullptr;
   TRY(noalloc_scratch(device, &base));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  uint32_t *perm_a = base, *perm_b = perm_a + kNoAllocMax, *keys_a = perm_b + kNoAllocMax,
-           *keys_b = keys_a + kNoAllocMax, *dropped = keys_b + kNoAllocMax, *hist = dropped + kNoAllocMax,
-           *partials = hist + kNoAllocHist, *total = partials + kNoAllocPartials, *kept = total + 1;
+  uint32_t *perm_a = base, *perm_b = perm_a + kNoAllocMax, *kept = perm_b + kNoAllocMax, *n_kept = kept + kNoAllocMax;
   // the kept count accumulates and must start at zero; everything else is
   // fully rewritten before it is read
-  CK(cudaMemsetAsync(kept, 0, 4, s));
+  CK(cudaMemsetAsync(n_kept, 0, 4, s));
   const PlainHsp *in = reinterpret_cast<const PlainHsp *>(d_in);
   const unsigned g = grid_for(n, 256, 1024);
-  iota_kernel<<<g, 256, 0, s>>>(perm_a, n);
-  const uint64_t tiles = (n + kRadixTile - 1) / kRadixTile;
-  auto sort_by = [&](const int *fields, int nf) {
-    for (int fi = 0; fi < nf; fi++) {
-      const int f = fields[fi];
-      na_gather_kernel<<<g, 256, 0, s>>>(in, perm_a, dropped, n, f, keys_a);
-      const int passes = f == kDroppedField ? 1 : 4;
-      for (int p = 0; p < passes && n; p++) {
-        radix_hist_kernel<<<(unsigned)tiles, kRadixThreads, 0, s>>>(keys_a, n, 8 * p, hist, tiles);
-        exclusive_scan<uint32_t>(hist, hist, tiles * kRadixBins, partials, total, s);
-        radix_scatter_kernel<<<(unsigned)tiles, kRadixThreads, 0, s>>>(keys_a, perm_a, n, 8 * p, hist, tiles,
-                                                                      keys_b, perm_b);
-        std::swap(keys_a, keys_b);
-        std::swap(perm_a, perm_b);
-      }
-    }
-  };
-  static const int by_diagonal_key[4] = {kScoreDesc, kLen, kRefStart, kDiag};
-  // dropped records last, the kept ones in LASTZ order first
-  static const int by_lastz_key[5] = {kScoreDesc, kLen, kRefStart, kQueryStart, kDroppedField};
   if (n) {
-    sort_by(by_diagonal_key, 4);
-    na_flag_kernel<<<g, 256, 0, s>>>(in, perm_a, n, dropped, kept);
-    sort_by(by_lastz_key, 5);
+    SortArgs<PlainHsp> sa{in, nullptr, nullptr, nullptr, n, nullptr};
+    sort_indices<kByDiagonal>(sa, perm_a, perm_b, s);
+    sa.idx = merge_passes(n) & 1 ? perm_b : perm_a;
+    keep_kernel<<<g, 256, 0, s>>>(sa, kept, n_kept);
+    sa.idx = kept;
+    sa.n_dev = n_kept;
+    sort_indices<kByLastz>(sa, perm_a, perm_b, s);
   }
-  na_copy_kernel<<<g, 256, 0, s>>>(in, perm_a, kept, reinterpret_cast<PlainHsp *>(d_out), d_n_out);
+  emit_plain_kernel<<<g, 256, 0, s>>>(in, perm_a, perm_b, n_kept, reinterpret_cast<PlainHsp *>(d_out), d_n_out);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return fail(HZ_E_CUDA, "dedup launch: %s", cudaGetErrorString(err));
   return HZ_OK;
@@ -2394,8 +2307,7 @@ uint64_t wave_footprint(const hz_engine *w) {
        dbytes(w->scope_call) + dbytes(w->raw_scope) + dbytes(w->tile_first) + dbytes(w->tile_call) +
        dbytes(w->np_excl) + dbytes(w->call_hit_lo) + dbytes(w->scope_lo) + dbytes(w->np_partial) +
        dbytes(w->np_grand) + dbytes(w->tot) + dbytes(w->cand) + dbytes(w->gate_ring) + dbytes(w->raw) + dbytes(w->d_out);
-  for (const DBuf<uint32_t> *x : {&w->d_perm_a, &w->d_perm_b, &w->d_keys_a, &w->d_keys_b, &w->d_keep,
-                                  &w->d_keep_excl, &w->d_hist, &w->d_hpart, &w->d_total})
+  for (const DBuf<uint32_t> *x : {&w->d_set, &w->d_perm_a, &w->d_perm_b, &w->d_kept, &w->d_total})
     b += dbytes(*x);
   return b;
 }
@@ -2410,8 +2322,8 @@ void release_wave_buffers(hz_engine *w) {
   }
   w->qascii.release();
   for (DBuf<uint32_t> *x : {&w->pos_hits, &w->np_pos, &w->call_nz_lo, &w->scope_call, &w->raw_scope, &w->tile_first,
-                            &w->tile_call, &w->pos_kmer, &w->np_kmer, &w->d_perm_a, &w->d_perm_b, &w->d_keys_a, &w->d_keys_b, &w->d_keep,
-                            &w->d_keep_excl, &w->d_hist, &w->d_hpart, &w->d_total})
+                            &w->tile_call, &w->pos_kmer, &w->np_kmer, &w->d_set, &w->d_perm_a,
+                            &w->d_perm_b, &w->d_kept, &w->d_total})
     x->release();
   w->np_excl.release();
   w->call_hit_lo.release();

@@ -63,7 +63,8 @@ struct WaveTotals {
   uint32_t cand;    // gate candidates written (may exceed capacity)
   uint32_t raw;     // accepted HSPs written (may exceed capacity)
   uint32_t long_next;  // long_kernel's cursor over the candidates
-  uint32_t pad[2];
+  uint32_t distinct;   // different ones among the accepted HSPs (unique_kernel)
+  uint32_t pad;
 };
 
 // Gate candidate: a hit whose score bound passes the threshold, or whose

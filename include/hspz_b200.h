@@ -196,7 +196,7 @@ int hz_dedup_and_order(hz_segment_pair *h, uint64_t n, uint64_t *n_out);
  * memory themselves or let a library do it -- e.g. a host whose own
  * allocator owns the whole device, or a serving loop that admits work
  * against a fixed memory budget.  It allocates nothing: its working memory is
- * a fixed array of about 6 MB compiled into this library, which every GPU
+ * a fixed array of about 3 MB compiled into this library, which every GPU
  * that loads the library holds until the process exits.
  *   d_in:    n records on the current device (4-byte aligned), read only;
  *            n <= HZ_NOALLOC_MAX_HSPS, larger n is refused with HZ_E_INVALID.
