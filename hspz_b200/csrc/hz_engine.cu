@@ -336,6 +336,7 @@ struct hz_engine {
   bool aliases_query = false;      // true for the plain form's extra workspaces (see run_pass_multi)
   std::vector<hz_engine *> twins;  // those workspaces, made on first use
   int plain_streams = 4;           // workspaces (host threads and streams) of a plain pass, 1..4
+  int plain_calls = 0;             // calls per wave of a plain pass; 0: as many as fill the device (plain_waves)
   struct Server *server = nullptr;  // the serving loop, while one runs
   // query store
   SeqBuf qstore;
@@ -511,10 +512,24 @@ bool gate2_usable(const hz_engine *e) {
   return e->cfg.xdrop >= 0 && e->cfg.xdrop <= kGate2MaxXdrop && (int64_t)e->cfg.xdrop + kRound * 255 < 32768;
 }
 
-// Hits per warp tile: the knob's, or what suits the gate that runs.  The
-// lane-refill gate stages every hit in shared memory, and beyond 128 hits that
-// costs it the L1 it lives on.
-int wave_tile(const hz_engine *e) { return e->gate_tile ? e->gate_tile : gate2_usable(e) ? 256 : 128; }
+// Hits that `positions` seed positions of `per_pos` seeds are expected to
+// have: the average bucket per seed.
+double expected_hits(const hz_engine *e, uint64_t positions, uint32_t per_pos) {
+  return (double)positions * per_pos * ((double)e->n_pos / (double)(1ull << (2 * e->shape.kmer_size)));
+}
+
+// Hits per warp tile: the knob's, or what suits the gate that runs and the
+// wave.  The lane-refill gate stages every hit in shared memory, and beyond
+// 128 hits that costs it the L1 it lives on.  The lockstep gate pays a setup
+// per tile, so its tiles are large, but a wave of less than a tile or two per
+// warp (4144 of them) then runs on a part of the chip: gate time by tile size
+// 64 / 128 / 256, 0.11 M hits: 37 / 51 / 84 us, 0.52 M: 43 / 41 / 59, 0.86 M:
+// 73 / 72 / 79, 2.1 M: 116 / 116 / 113, 21 M: 732 / 658 / 628.
+int wave_tile(const hz_engine *e, double hits) {
+  if (e->gate_tile) return e->gate_tile;
+  if (!gate2_usable(e)) return 128;
+  return hits < 3e5 ? 64 : hits < 1.2e6 ? 128 : 256;
+}
 
 // Prepares one instance of the lockstep gate for 'smem' bytes of shared
 // memory and returns its blocks per SM.
@@ -551,13 +566,13 @@ template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, Gate2Args
 // pairs against lanes: 4.7: 48.1 / 41.8, 9.5: 37.7 / 35.0, 18.9: 32.2 / 32.6,
 // 42: 29.3 / 32.2, 113: 28.4 / 32.4.  The one-table score lookup when
 // complementary pairs score alike (CostTable).
-int launch_gate2(hz_engine *e, const GateArgs &ga) {
+int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   Gate2Args a2;
   a2.g = ga;
   a2.ref = e->ref_p.half_ptr(0) - kPackPad;
   a2.qry = e->qry_p.half_ptr(0) - kPackPad;
   a2.ring = e->gate_ring.p;
-  a2.tile = (uint32_t)wave_tile(e);
+  a2.tile = (uint32_t)tile;
   a2.soft_codes = 0;
   bool alike = true;
   for (int i = 0; i < kNuc; i++)
@@ -581,8 +596,7 @@ int launch_gate2(hz_engine *e, const GateArgs &ga) {
     }
     a2.min_total = (int32_t)lo;
   }
-  const double per_bucket = (double)e->n_pos / (double)(1ull << (2 * e->shape.kmer_size));
-  const double hits_per_pos = std::max(ga.w.per_pos * per_bucket, 1e-9);
+  const double hits_per_pos = std::max(expected_hits(e, 1, ga.w.per_pos), 1e-9);
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
       e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 7.5 * positions_per_pass;
@@ -843,7 +857,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
   const bool packed_q = e->qry_p.valid && e->shape.size <= 32 && e->qry_p.half >= e->qstore.len;
   w.qp2 = packed_q ? e->qry_p.half_ptr(0) : nullptr;
   w.pos_kmer = e->pos_kmer.p;
-  const int tile = wave_tile(e);
+  const int tile = wave_tile(e, expected_hits(e, npos, w.per_pos));
 
   for (int attempt = 0; attempt < 8; attempt++) {  // each rerun fixes every capacity it found short
     uint32_t scope_cap = std::max<uint32_t>(e->scope_cap, (uint32_t)n * 2 + 16);
@@ -916,7 +930,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       ga.tile_first = e->tile_first.p;
       ga.tile_call = e->tile_call.p;
       if (gate2_usable(e)) {
-        TRY(launch_gate2(e, ga));
+        TRY(launch_gate2(e, ga, tile));
         TRY(launch_long(e, ga));
       } else {
         switch (tile) {
@@ -956,13 +970,13 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     if (graph) TRY(run_captured(e, chain));
     else TRY(chain());
     if (defer) defer->finish(e);  // the previous call's host dedup, while this call's kernels run
-    // A single-call wave (the plain form) reads back the first different HSPs
+    // A wave deduped on the host (the plain form) reads back the first different HSPs
     // and scopes with its totals, so one with few of them (the usual case)
     // needs one sync, not two.
     uint32_t pre_raw = 0, pre_scopes = 0;
-    if (n == 1 && !device_dedup) {
+    if (!device_dedup) {
       pre_raw = kRawPrefix;
-      pre_scopes = std::min<uint32_t>(kScopePrefix, scope_cap + 1);
+      pre_scopes = std::min<uint32_t>(std::max<uint32_t>(kScopePrefix, 2 * (uint32_t)n), scope_cap + 1);
       TRY(e->h_out.ensure(pre_raw));
       TRY(e->h_scope_call.ensure(pre_scopes));
       CK(cudaMemcpyAsync(e->h_out.p, e->distinct_head(), (size_t)pre_raw * sizeof(ScopedHspOut), cudaMemcpyDeviceToHost, s));
@@ -1650,15 +1664,59 @@ void add_stats(hz_stats *a, const hz_stats &b) {
   a->calls += b.calls;
 }
 
-// The plain pass over `k` workspaces: this engine and k - 1 more (each with
-// its own stream and wave buffers over the same target tables and query
-// store), each driven by its own host thread and taking the next call from a
-// shared counter.  While one waits for its call's read-back and dedups it on
-// the host, the others' kernels run, so the device is not idle between calls.
-// Calls are independent, so each call's records are the same as on one
-// workspace; they are put back in call order.
-int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls, std::vector<WaveRecord> *recs,
-                   hz_stats *st) {
+// A plain pass's calls as waves [first, last).  One call leaves the device
+// waiting for its launch chain and its longest extension (~0.3 ms for 2 M
+// hits, of which the gate takes 0.11), so small calls share a wave, up to
+// kPlainHits expected hits -- enough that what does not scale with the hits is
+// a tenth of the wave -- and kPlainPositions seed positions (100 MB of wave
+// buffers).  By calls per wave 1 / 4 / 16 / 32: 80 calls of 10 Mbp against a
+// 10 Mbp bin (2.1 M hits each) 11.1 / 8.3 / 7.5 / 7.2 ms, 8 calls of a 1 Mbp
+// pair 0.84 / 0.61 / 0.60 / 0.60; a call against a 200 Mbp target has 33 M
+// hits and stays alone.  Calls are independent, so their records are the same
+// in any wave.
+constexpr double kPlainHits = 5e7;
+constexpr uint64_t kPlainPositions = 1ull << 22;
+std::vector<std::pair<size_t, size_t>> plain_waves(const hz_engine *e, const std::vector<HostCall> &calls) {
+  std::vector<std::pair<size_t, size_t>> out;
+  for (size_t i = 0; i < calls.size();) {
+    size_t j = i;
+    uint64_t pos = 0;
+    while (j < calls.size()) {
+      const uint64_t more = pos + (calls[j].end - calls[j].start);
+      if (j > i && (e->plain_calls ? j - i >= (size_t)e->plain_calls
+                                   : more > kPlainPositions ||
+                                         expected_hits(e, more, e->per_pos(e->cfg.transitions)) > kPlainHits))
+        break;
+      pos = more;
+      j++;
+    }
+    out.push_back({i, j});
+    i = j;
+  }
+  return out;
+}
+
+// One wave of a plain pass; one that holds too many hits runs call by call.
+int run_plain_wave(hz_engine *e, const std::vector<HostCall> &calls, std::pair<size_t, size_t> wave,
+                   std::vector<WaveRecord> *recs, hz_stats *st, DeferredDedup *defer = nullptr) {
+  const size_t n = wave.second - wave.first;
+  int rc = run_wave(e, &calls[wave.first], n, nullptr, e->cfg.transitions, recs, st, false, false, defer,
+                    (uint32_t)wave.first);
+  if (rc != kSplitWave) return rc;
+  for (size_t i = wave.first; i < wave.second; i++)
+    TRY(run_wave(e, &calls[i], 1, nullptr, e->cfg.transitions, recs, st, false, false, defer, (uint32_t)i));
+  return HZ_OK;
+}
+
+// The plain pass's waves over `k` workspaces: this engine and k - 1 more (each
+// with its own stream and wave buffers over the same target tables and query
+// store), each driven by its own host thread and taking the next wave from a
+// shared counter.  While one waits for its read-back and dedups on the host,
+// the others' kernels run, so the device is not idle between waves.  Each
+// wave's records are the same as on one workspace; they are put back in call
+// order.
+int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls,
+                   const std::vector<std::pair<size_t, size_t>> &waves, std::vector<WaveRecord> *recs, hz_stats *st) {
   while ((int)e->twins.size() < k - 1) {
     hz_engine *w = nullptr;
     TRY(clone_shared(e, &w));
@@ -1683,10 +1741,10 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls, std:
   std::vector<uint64_t> launches0(ws.size());
   for (size_t j = 0; j < ws.size(); j++) launches0[j] = ws[j]->launches;
 
-  std::vector<std::vector<WaveRecord>> per(calls.size());
+  std::vector<std::vector<WaveRecord>> per(waves.size());
   std::atomic<size_t> next{0};
   std::atomic<bool> stop{false};
-  // calls an extra workspace could not finish for lack of device memory;
+  // waves an extra workspace could not finish for lack of device memory;
   // this engine runs them once the others are done
   std::vector<size_t> orphans;
   std::mutex orphans_mu;
@@ -1694,12 +1752,11 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls, std:
     for (;;) {
       if (stop.load()) return HZ_OK;
       size_t i = next.fetch_add(1);
-      if (i >= calls.size()) return HZ_OK;
-      hz_stats one;  // counted only once the call has finished
+      if (i >= waves.size()) return HZ_OK;
+      hz_stats one;  // counted only once the wave has finished
       memset(&one, 0, sizeof one);
-      int rc = run_wave(x, &calls[i], 1, nullptr, x->cfg.transitions, &per[i], &one, false, false, nullptr,
-                        (uint32_t)i);
-      if (rc == HZ_E_OOM && extra) {  // this workspace stops; its call moves on
+      int rc = run_plain_wave(x, calls, waves[i], &per[i], &one);
+      if (rc == HZ_E_OOM && extra) {  // this workspace stops; its wave moves on
         per[i].clear();
         std::lock_guard<std::mutex> lock(orphans_mu);
         orphans.push_back(i);
@@ -1740,8 +1797,7 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls, std:
     for (size_t i : orphans) {
       hz_stats one;
       memset(&one, 0, sizeof one);
-      rcs[0] = run_wave(e, &calls[i], 1, nullptr, e->cfg.transitions, &per[i], &one, false, false, nullptr,
-                        (uint32_t)i);
+      rcs[0] = run_plain_wave(e, calls, waves[i], &per[i], &one);
       if (rcs[0] != HZ_OK) break;
       add_stats(&sts[0], one);
     }
@@ -1779,8 +1835,8 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls, std:
 }
 }  // namespace
 
-// The plain per-chunk form: one wave (launch chain + read-back + host dedup)
-// per seed_and_filter call, in the reference's call order.
+// The plain form: waves of one or a few seed_and_filter calls (launch chain,
+// read-back, host dedup), in the reference's call order.
 int hz_run_pass(hz_engine *e, hz_pass_record **out, uint64_t *n, hz_stats *stats) {
   if (!e || !out || !n) return fail(HZ_E_INVALID, "bad argument");
   *out = nullptr;
@@ -1793,13 +1849,13 @@ int hz_run_pass(hz_engine *e, hz_pass_record **out, uint64_t *n, hz_stats *stats
   std::vector<HostCall> calls;
   query_calls(e, e->cur_query, &calls);
   std::vector<WaveRecord> recs;
+  const std::vector<std::pair<size_t, size_t>> waves = plain_waves(e, calls);
   // (on a caller's stream, every call stays on that stream)
-  if (e->plain_streams >= 2 && calls.size() >= 2 && e->st == e->own_st) {
-    TRY(run_pass_multi(e, e->plain_streams, calls, &recs, &local));
+  if (e->plain_streams >= 2 && waves.size() >= 2 && e->st == e->own_st) {
+    TRY(run_pass_multi(e, (int)std::min<size_t>((size_t)e->plain_streams, waves.size()), calls, waves, &recs, &local));
   } else {
-    DeferredDedup defer;  // call i's host dedup runs while call i + 1's kernels do
-    for (size_t i = 0; i < calls.size(); i++)
-      TRY(run_wave(e, &calls[i], 1, nullptr, e->cfg.transitions, &recs, &local, false, false, &defer, (uint32_t)i));
+    DeferredDedup defer;  // wave i's host dedup runs while wave i + 1's kernels do
+    for (const auto &wave : waves) TRY(run_plain_wave(e, calls, wave, &recs, &local, &defer));
     defer.finish(e);
   }
   // records of one interval: plus calls before minus calls (call order already)
@@ -2132,6 +2188,9 @@ int hz_engine_set_tuning(hz_engine *e, const char *key, int64_t value) {
       hz_engine_destroy(e->twins.back());
       e->twins.pop_back();
     }
+  } else if (k == "plain_calls") {
+    if (value < 0 || value > 1000000) return fail(HZ_E_INVALID, "plain_calls must be 0..1000000");
+    e->plain_calls = (int)value;
   } else if (k == "tile_cap" || k == "cand_cap" || k == "raw_cap") {
     // starting capacities; a wave that needs more grows them and runs again
     if (value < 16 || value > 0x7FFFFFFFll) return fail(HZ_E_INVALID, "%s must be 16..2^31-1", key);
@@ -2215,7 +2274,7 @@ int hz_engine_autotune(hz_engine *e, uint64_t sample_positions, hz_tuning *out) 
     e->use_graph = start.graph;
     return rc;
   }
-  out->gate_tile = wave_tile(e);
+  out->gate_tile = pick.tile ? pick.tile : wave_tile(e, 1e9);
   out->gate_cap = (int32_t)pick.cap;
   out->gate_blocks_per_sm = e->gate_blocks_per_sm;
   out->graph = pick.graph ? 1 : 0;
@@ -2375,6 +2434,7 @@ void share_target(hz_engine *w, const hz_engine *e) {
   w->ref_p = e->ref_p;
   w->has_target = true;
   w->owns_target = false;
+  w->plain_calls = e->plain_calls;
   w->gate_version = e->gate_version;
   w->gate_sparse = e->gate_sparse;
   w->gate_tile = e->gate_tile;

@@ -124,11 +124,12 @@ int hz_generate_seeds(hz_engine *e, uint32_t slot, int rev, uint32_t start, uint
 int hz_seed_and_filter(hz_engine *e, uint32_t slot, int rev, hz_segment_pair **out, uint64_t *n,
                        hz_stats *stats);
 
-/* seed_and_filter_all (src/run.rs:266-495), plain per-chunk form: every
- * interval x strand x WGA chunk of the swapped-in query, one launch chain per
- * call.  Records are grouped per interval, plus before minus, in call order.
- * By default the calls run on four workspaces at once (tuning knob
- * "plain_streams"); the records do not depend on it. */
+/* seed_and_filter_all (src/run.rs:266-495), plain form: every interval x
+ * strand x WGA chunk of the swapped-in query.  Small calls share a launch
+ * chain (tuning knob "plain_calls"; 1 is the reference's one chain per call).
+ * Records are grouped per interval, plus before minus, in call order.
+ * By default the chains run on four workspaces at once (tuning knob
+ * "plain_streams"); the records do not depend on either. */
 int hz_run_pass(hz_engine *e, hz_pass_record **out, uint64_t *n, hz_stats *stats);
 
 /* One query block for the batched form (ASCII, records joined by '&'). */
@@ -248,7 +249,9 @@ int hz_engine_profile_reset(hz_engine *e);
  * host, as the reference does),
  * "graph" (1: the batched form captures each wave's kernel chain as a CUDA
  * graph and replays it, updating the instantiated graph in place),
- * "plain_streams" (1..4, default 4: hz_run_pass runs its calls on this
+ * "plain_calls" (calls that share a launch chain of hz_run_pass, 0..1000000;
+ * 0, the default: as many as fill the device; 1: one chain per call),
+ * "plain_streams" (1..4, default 4: hz_run_pass runs its chains on this
  * engine and plain_streams - 1 more workspaces over the same target, each
  * with its own host thread and stream, so one call's read-back and host dedup
  * overlap other calls' kernels; 1: one call at a time on this engine; an
