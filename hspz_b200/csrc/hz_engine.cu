@@ -531,6 +531,15 @@ int wave_tile(const hz_engine *e, double hits) {
   return hits < 3e5 ? 64 : hits < 1.2e6 ? 128 : 256;
 }
 
+// Whether complementary ACGT pairs score alike: one score per index of the
+// packed kernels' lookup (CostTable).
+bool strands_alike(const int32_t *sub) {
+  for (int i = 0; i < 4; i++)
+    for (int j = 0; j < 4; j++)
+      if (sub[i * kNuc + j] != sub[(i ^ 3) * kNuc + (j ^ 3)]) return false;
+  return true;
+}
+
 // Prepares one instance of the lockstep gate for 'smem' bytes of shared
 // memory and returns its blocks per SM.
 template <bool SPARSE, bool GENERAL> int gate2_blocks(hz_engine *e, size_t smem, int *per_sm) {
@@ -574,11 +583,9 @@ int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   a2.ring = e->gate_ring.p;
   a2.tile = (uint32_t)tile;
   a2.soft_codes = 0;
-  bool alike = true;
   for (int i = 0; i < kNuc; i++)
     for (int j = 0; j < kNuc; j++) {
       const int32_t v = ga.sub[i * kNuc + j];
-      if (i < 4 && j < 4) alike = alike && v == ga.sub[(i ^ 3) * kNuc + (j ^ 3)];
       // a code ends every extension that meets it when all its scores drop
       // below -xdrop
       if ((int64_t)v + ga.xdrop < 0) continue;
@@ -600,26 +607,30 @@ int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
       e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 7.5 * positions_per_pass;
-  if (alike) return sparse ? launch_gate2_as<true, false>(e, a2) : launch_gate2_as<false, false>(e, a2);
+  if (strands_alike(ga.sub)) return sparse ? launch_gate2_as<true, false>(e, a2) : launch_gate2_as<false, false>(e, a2);
   return sparse ? launch_gate2_as<true, true>(e, a2) : launch_gate2_as<false, true>(e, a2);
 }
 
-// The long candidates of a wave, extended to their ends in lockstep over the
-// packed sequences (long_kernel); runs only where the packed gate runs.
-int launch_long(hz_engine *e, const GateArgs &ga) {
+// The candidates of a wave, extended to their ends over the packed sequences
+// (long_kernel); runs only where the packed gate runs.
+template <bool GENERAL> int launch_long_as(hz_engine *e, const LongArgs &la) {
   static bool configured[64] = {false};
   static std::mutex mu;
   const size_t smem = sizeof(LongSmem);
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!configured[e->device & 63]) {
-      CK(cudaFuncSetAttribute(long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      CK(cudaFuncSetAttribute(long_kernel<GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       configured[e->device & 63] = true;
     }
   }
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, long_kernel, kGateThreads, smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, long_kernel<GENERAL>, kGateThreads, smem));
   if (per_sm < 1) per_sm = 1;
+  const unsigned grid = (unsigned)(e->sm_count * per_sm);
+  return e->launch("long", [&] { long_kernel<GENERAL><<<grid, kGateThreads, smem, e->st>>>(la); });
+}
+int launch_long(hz_engine *e, const GateArgs &ga) {
   LongArgs la;
   la.ref = e->ref_p.half_ptr(0);
   la.refr = e->ref_p.half_ptr(1);
@@ -636,8 +647,11 @@ int launch_long(hz_engine *e, const GateArgs &ga) {
   memcpy(la.sub, ga.sub, sizeof(la.sub));
   la.xdrop = ga.xdrop;
   la.late_max_safe = ga.late_max_safe;
-  const unsigned grid = (unsigned)(e->sm_count * per_sm);
-  return e->launch("long", [&] { long_kernel<<<grid, kGateThreads, smem, e->st>>>(la); });
+  // half a warp per direction takes 28 us for 2 300 candidates and 4 ns more for
+  // each, a lane per direction 96 us (its longest extension) and 1 ns:
+  // 60 000 candidates 222 / 167 us, 105 000 379 / 170
+  la.wide_max = 32768;
+  return strands_alike(ga.sub) ? launch_long_as<false>(e, la) : launch_long_as<true>(e, la);
 }
 
 template <int TW> int launch_gate(hz_engine *e, const GateArgs &ga) {

@@ -1,25 +1,26 @@
-// Long candidates extended in lockstep (included by hz_wave.cuh after
-// hz_gate2.cuh).
+// Candidates extended exactly (included by hz_wave.cuh after hz_gate2.cuh).
 //
-// A hit whose extension runs past the score gate's cell cap is a "long"
-// candidate: the gate stops scoring it and the exact kernel has to redo both
-// directions from the anchor (src/gpu/kernels.rs:1279-1406 does this
-// warp-wide for every hit).  On repeat-dense input these extensions run to
-// hundreds or thousands of cells.  long_kernel extends every long candidate
-// of a wave to its end, one lane per candidate-direction, in the gate's
-// rounds of kRound cells over the 2-bit packed sequences, and finds in each
-// direction the maximum and the first cell that reaches it.  It writes them
-// into the candidate and marks it kDoneFlag, so the exact kernel is left
-// with the entropy and the accept.
+// The lockstep gate hands on every hit whose extensions may reach the
+// threshold, and those that run past its cell cap (src/gpu/kernels.rs:1279-1406
+// extends every hit warp-wide).  long_kernel extends each candidate of a wave
+// to its end over the 2-bit packed sequences and finds in each direction the
+// maximum and the first cell that reaches it.  It writes them into the
+// candidate and marks it kDoneFlag, so the exact kernel is left with the
+// entropy and the accept.
 //
-// The maximum's position is found without a per-cell test: in a round whose
-// cells are all valid the main pass notes the last eight-cell group in which
-// the running maximum rose (the first cell reaching the round's final
-// maximum lies in it) together with that group's starting sum, and only
-// when the direction ends is that one group rescored.  A round that stops
-// early (a drop, a special base, the edge) searches its own valid groups at
-// once, from the group states it keeps in shared memory and the codes it
-// still holds in registers.
+// Few candidates (LongArgs::wide_max) go half a warp per direction, 256 cells
+// per step (long_wide): their time is that of the longest extension.  More go
+// one lane per candidate-direction, in rounds of kRound cells, which takes
+// fewer instructions per cell.  There the maximum's position is found without
+// a per-cell test: in a round whose cells are all valid the main pass notes
+// the last eight-cell group in which the running maximum rose (the first cell
+// reaching the round's final maximum lies in it) together with that group's
+// starting sum, and only when the direction ends is that one group rescored.
+// A round that stops early (a drop, a special base, the edge) searches its own
+// valid groups at once, from the group states it keeps in shared memory and
+// the codes it still holds in registers.  Scores come from the gate's lookup
+// (costs by byte permute, sums by dot product): 3.5 M candidates 2.76 ms, with
+// a shared-memory lookup per cell 3.13.
 //
 // Semantics are exact_dir4's: cells counted up to and including the first
 // dropping cell (or to the edge); the right position is the cell offset of
@@ -59,23 +60,15 @@ __device__ __forceinline__ void window_round(const uint4 *__restrict__ blk, uint
   *sp_hi = kRound > 32 ? __funnelshift_r(r[1].z, r[kRec - 1].z, o) : 0u;
 }
 
-// The four index words of 16 cells: word j holds cells j, j+4, j+8, j+12 in
-// its bytes 0..3, each byte being that cell's table index (reference code |
-// query code << 2) with its upper four bits clear.  Every lane's score lookup
-// then falls in the same 16 bytes of shared memory, four banks, so a warp's
-// lookup is one wavefront whatever the codes.
-__device__ __forceinline__ void pair_words(uint32_t r, uint32_t q, uint32_t t[4]) {
-  const uint32_t x = (r & 0x33333333u) | ((q << 2) & 0xCCCCCCCCu);  // nibble n: index of cell 2n
-  const uint32_t y = ((r >> 2) & 0x33333333u) | (q & 0xCCCCCCCCu);  // nibble n: index of cell 2n + 1
-  t[0] = x & 0x0F0F0F0Fu;
-  t[1] = y & 0x0F0F0F0Fu;
-  t[2] = (x >> 4) & 0x0F0F0F0Fu;
-  t[3] = (y >> 4) & 0x0F0F0F0Fu;
+// The costs (negated scores) of the eight cells whose codes are the low 16 bits
+// of r and q: even cells in .x, odd ones in .y, a byte each; and s plus the
+// score of cell k of them.
+template <typename TAB> __device__ __forceinline__ uint2 costs8(const TAB &tab, uint32_t r, uint32_t q) {
+  const uint2 sel = TAB::index(r, q);
+  return make_uint2(tab.costs(sel.x), tab.costs(sel.y));
 }
-
-// Score of cell k (0..15) of the 16 cells whose index words are t.
-__device__ __forceinline__ int32_t cell_score(const int8_t *tbl, const uint32_t t[4], int k) {
-  return tbl[__byte_perm(t[k & 3], 0u, 0x4440u + (uint32_t)(k >> 2))];
+__device__ __forceinline__ int32_t add_score(int32_t s, const uint2 &c, int k) {
+  return __dp4a((int)(k & 1 ? c.y : c.x), (int)(0xFFu << (8 * (k >> 1))), s);
 }
 
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
@@ -103,6 +96,7 @@ struct LongArgs {
   int32_t sub[64];
   int32_t xdrop;
   uint32_t late_max_safe;  // as GateArgs::late_max_safe
+  uint32_t wide_max;       // candidates up to which half a warp extends each direction
 };
 
 struct LongWarp {
@@ -111,37 +105,177 @@ struct LongWarp {
 };
 
 struct LongSmem {
-  int32_t sub[64];
-  int8_t tbl[16];
   LongWarp warp[kGateWarps];
 };
 
 // The first of the eight cells whose codes are the low 16 bits of r and q at
 // which the running sum, starting from s, equals target (8 if none does).
-__device__ __forceinline__ uint32_t first_reach(const int8_t *tbl, uint32_t r, uint32_t q, int32_t s,
-                                                int32_t target) {
-  uint32_t tw[4];
-  pair_words(r & 0xFFFFu, q & 0xFFFFu, tw);
+template <typename TAB>
+__device__ __forceinline__ uint32_t first_reach(const TAB &tab, uint32_t r, uint32_t q, int32_t s, int32_t target) {
+  const uint2 cost = costs8(tab, r, q);
   uint32_t c = 8;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    s = wadd(s, cell_score(tbl, tw, i));
+    s = add_score(s, cost, i);
     if (c == 8 && s == target) c = (uint32_t)i;
   }
   return c;
 }
 
-__global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
+// Few candidates: half a warp per direction, sixteen cells per lane, 256 per
+// step.  A wave's time here is that of its longest extension, and lanes on
+// their own need a 48-cell round for what a step does for 256 cells.  A lane
+// sums its cells' costs A (negated scores), and notes their minimum, maximum
+// and largest rise over an earlier minimum; scans over the half warp give the
+// cost and the minimum before its cells, and with them whether one of its
+// cells drops.  The first lane that has one finds which; the minimum's first
+// cell is looked for where a step lowers it.
+template <bool GENERAL> __device__ __forceinline__ void long_wide(const LongArgs &a, uint32_t ncand) {
+  const uint32_t lane = threadIdx.x & 31, l = lane & 15u, half = lane >> 4;  // half 0: right, 1: left
+  const CostTable<GENERAL> tab(a.sub);
+  const int32_t X = a.xdrop;
+  const uint4 *const rseq = half ? a.refr : a.ref, *const qseq = half ? a.qryr : a.qry;
+  unsigned long long cells_acc = 0;
+  uint32_t i = 0;
+  if (lane == 0) i = atomicAdd(&a.tot->long_next, 1u);
+  i = __shfl_sync(0xffffffffu, i, 0);
+  while (i < ncand) {
+    uint32_t next = 0;  // claimed while this one is extended
+    if (lane == 0) next = atomicAdd(&a.tot->long_next, 1u);
+    const Cand c = a.cand[i];
+    const CallDev cd = a.calls[c.call & ~(kLongFlag | kDoneFlag)];
+    const uint32_t edge = !(c.call & kLongFlag) ? 0u
+                          : half                ? min(c.r0, c.q0 - cd.qoff)
+                                                : min(a.rlen - c.r0, cd.qoff + cd.qlen - c.q0);
+    const uint32_t rp = half ? a.rlen - c.r0 : c.r0, qp = half ? a.qtotal - c.q0 : c.q0;
+    // the half's state: cost and minimum at the step's start, the minimum's
+    // cell (-1: none yet), cells scored
+    int32_t at = 0, low = 0, pos = -1;
+    uint32_t cells = 0;
+    bool done = edge == 0;
+    for (uint32_t step = 0; __any_sync(0xffffffffu, !done); step += 256) {
+      const uint32_t k0 = step + 16 * l;
+      const uint32_t v = done || k0 >= edge ? 0u : min(edge - k0, 16u);  // the lane's cells
+      uint32_t rlo, rhi, rsp, qlo, qhi, qsp;
+      window32(rseq, v ? rp + k0 : 0u, &rlo, &rhi, &rsp);
+      window32(qseq, v ? qp + k0 : 0u, &qlo, &qhi, &qsp);
+      const uint2 sel = CostTable<GENERAL>::index(rlo, qlo);
+      const uint32_t e[2] = {tab.costs(sel.x), tab.costs(sel.x >> 16)},
+                     o[2] = {tab.costs(sel.y), tab.costs(sel.y >> 16)};
+      int32_t A[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const int32_t cost = (int32_t)(int8_t)((j & 1 ? o[j >> 3] : e[j >> 3]) >> (8 * ((j & 7) >> 1)));
+        A[j] = (uint32_t)j < v ? cost : 0;
+      }
+      uint32_t sp = (rsp | qsp) & ((1u << v) - 1u);
+      if (__any_sync(0xffffffffu, sp != 0)) {  // special bases: their scores from the 8-bit codes
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+          if (sp >> j & 1u) {
+            const uint32_t pr = rp + k0 + j, pq = qp + k0 + j;
+            A[j] = -a.sub[a.ref8[half ? a.rlen - 1u - pr : pr] * kNuc + a.qry8[half ? a.qtotal - 1u - pq : pq]];
+          }
+      }
+      int32_t lm = 0x7FFFFFFF, hi = -0x7FFFFFFF, rise = 0;
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        if (j) A[j] = wadd(A[j], A[j - 1]);
+        lm = min(lm, A[j]);
+        hi = max(hi, A[j]);
+        rise = max(rise, A[j] - lm);
+      }
+      if (v == 0) lm = 0x3FFFFFFF;  // no cells: never the minimum, never a drop
+      int32_t incl = A[15];
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) {
+        const int32_t up = __shfl_up_sync(0xffffffffu, incl, d, 16);
+        if (l >= (uint32_t)d) incl = wadd(incl, up);
+      }
+      const int32_t mine = wadd(at, incl - A[15]);  // the cost before the lane's cells
+      int32_t upto = v ? wadd(mine, lm) : 0x7FFFFFFF;
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) upto = min(upto, __shfl_up_sync(0xffffffffu, upto, d, 16));
+      int32_t before = __shfl_up_sync(0xffffffffu, upto, 1, 16);
+      before = l ? min(before, low) : low;  // the minimum before them
+      const int32_t D = mine - before;
+      const bool drops = v && (hi > X - D || rise > X);
+      const uint32_t fl = __ballot_sync(0xffffffffu, drops) >> (16 * half) & 0xFFFFu;
+      const uint32_t f = fl ? (uint32_t)(__ffs((int)fl) - 1) : 16u;  // the first lane with a drop
+      // the cells before the drop: their number, and the lowest cost
+      uint32_t n = l < f ? v : 0u;
+      if (l == f) {
+        int32_t m = -D, best = 0x3FFFFFFF;
+        uint32_t hit = 16;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          m = min(m, A[j]);
+          if (hit == 16) {
+            if (A[j] - m > X && (uint32_t)j < v) hit = (uint32_t)j;
+            else best = min(best, A[j]);
+          }
+        }
+        n = hit;
+        lm = best;
+      }
+      const int32_t least = n ? wadd(mine, lm) : 0x7FFFFFFF;
+      int32_t all = least;
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) all = min(all, __shfl_xor_sync(0xffffffffu, all, d));
+      if (__any_sync(0xffffffffu, !done && all < low)) {  // a new minimum: its first cell
+        uint32_t first = 16;
+#pragma unroll
+        for (int j = 15; j >= 0; j--)
+          if ((uint32_t)j < n && wadd(mine, A[j]) == all) first = (uint32_t)j;
+        const uint32_t has = __ballot_sync(0xffffffffu, first < 16) >> (16 * half) & 0xFFFFu;
+        const uint32_t g = has ? (uint32_t)(__ffs((int)has) - 1) : 0u;
+        const uint32_t cell = step + 16 * g + __shfl_sync(0xffffffffu, first, g, 16);
+        if (!done && all < low) {
+          low = all;
+          pos = (int32_t)cell;
+        }
+      }
+      const uint32_t in_f = __shfl_sync(0xffffffffu, n, f & 15u, 16);
+      at = wadd(at, __shfl_sync(0xffffffffu, incl, 15, 16));
+      if (!done) {
+        if (f < 16) {
+          cells = step + 16 * f + in_f + 1;
+          done = true;
+        } else if (step + 256 >= edge) {
+          cells = edge;
+          done = true;
+        }
+      }
+    }
+    const int32_t lmax = __shfl_sync(0xffffffffu, -low, 16), lpos = __shfl_sync(0xffffffffu, pos, 16);
+    const uint32_t lcells = __shfl_sync(0xffffffffu, cells, 16);
+    if (lane == 0 && (c.call & kLongFlag)) {
+      Cand &out = a.cand[i];
+      out.rmax = -low;
+      out.lmax = lmax;
+      out.rpos = pos;
+      out.lpos = lpos + 1;
+      out.call = c.call | kDoneFlag;
+      cells_acc += cells + lcells;
+    }
+    i = __shfl_sync(0xffffffffu, next, 0);
+  }
+  if (lane == 0 && cells_acc) atomicAdd(&a.tot->cells, cells_acc);
+}
+
+template <bool GENERAL>
+__global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constant__ LongArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   LongSmem &sm = *reinterpret_cast<LongSmem *>(smem_raw);
-  if (threadIdx.x < 64) sm.sub[threadIdx.x] = a.sub[threadIdx.x];
-  if (threadIdx.x < 16) sm.tbl[threadIdx.x] = (int8_t)a.sub[(threadIdx.x & 3u) * kNuc + (threadIdx.x >> 2)];
-  __syncthreads();  // the block's only barrier
+  const uint32_t ncand = min(a.tot->cand, a.cand_cap);
+  if (ncand <= a.wide_max) {
+    long_wide<GENERAL>(a, ncand);
+    return;
+  }
   LongWarp &wp = sm.warp[threadIdx.x >> 5];
-  const int8_t *tbl = sm.tbl;
+  const CostTable<GENERAL> tab(a.sub);
   const uint32_t lane = threadIdx.x & 31;
   const int32_t X = a.xdrop;
-  const uint32_t ncand = min(a.tot->cand, a.cand_cap);
   unsigned long long cells_acc = 0;
   uint32_t qn = 0;  // candidates in the warp's queue (warp-uniform)
   bool exhausted = false;
@@ -221,19 +355,18 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
     int32_t gi = -1;
 #pragma unroll
     for (int h = 0; h < kChunks; h++) {
-      uint32_t tw[4];
-      pair_words(Rc[h], Qc[h], tw);
+      const uint2 sel = CostTable<GENERAL>::index(Rc[h], Qc[h]);
 #pragma unroll
       for (int gg = 0; gg < 2; gg++) {
         const int g = 2 * h + gg;
         wp.grp[g][lane] = __byte_perm((uint32_t)S, (uint32_t)M, 0x5410u);
         const int32_t Mg = M;
+        const uint2 cost = make_uint2(tab.costs(gg ? sel.x >> 16 : sel.x), tab.costs(gg ? sel.y >> 16 : sel.y));
         int32_t lo = 0x7FFFFFFF;
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
-          const int k = 8 * gg + i;
-          const int32_t S1 = wadd(S, cell_score(tbl, tw, k));
-          const int32_t S2 = wadd(S1, cell_score(tbl, tw, k + 1));
+          const int32_t S1 = add_score(S, cost, i);
+          const int32_t S2 = add_score(S1, cost, i + 1);
           M = __vimax3_s32(M, S1, S2);
           lo = __vimin3_s32(lo, S1, S2);
           S = S2;
@@ -264,14 +397,13 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
             qw = Qc[k];
           }
         const uint32_t sh = (g & 1u) << 4;
-        uint32_t tw[4];
-        pair_words((hw >> sh) & 0xFFFFu, (qw >> sh) & 0xFFFFu, tw);
+        const uint2 cost = costs8(tab, hw >> sh, qw >> sh);
         if (a.late_max_safe && g != gv) {
           int32_t D = (int32_t)((uint32_t)Me - (uint32_t)Se);
           uint32_t dm = 0;
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            D = max((int32_t)((uint32_t)D - (uint32_t)cell_score(tbl, tw, i)), 0);
+            D = max(__dp4a((int)(i & 1 ? cost.y : cost.x), 1 << (8 * (i >> 1)), D), 0);
             dm |= (uint32_t)(D > X) << i;
           }
           if (dm) {
@@ -286,7 +418,7 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
         uint32_t d = 8;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          const int32_t Sx = wadd(Se, cell_score(tbl, tw, i));
+          const int32_t Sx = add_score(Se, cost, i);
           const int32_t Mx = max(Me, Sx);
           if ((uint32_t)i < lim && d == 8) {
             if ((int32_t)((uint32_t)Mx - (uint32_t)Sx) > X) {
@@ -315,7 +447,7 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
       if (!dropped && vv < (uint32_t)kRound && vv < v) {  // a special base at cell vv
         const uint32_t pr = rp + vv, pq = qp + vv;
         const uint32_t r8 = dir ? a.rlen - 1u - pr : pr, q8 = dir ? a.qtotal - 1u - pq : pq;
-        const int32_t Sx = wadd(Sf, sm.sub[a.ref8[r8] * kNuc + a.qry8[q8]]);
+        const int32_t Sx = wadd(Sf, a.sub[a.ref8[r8] * kNuc + a.qry8[q8]]);
         const int32_t Mx = max(Mf, Sx);
         used = vv + 1;
         if ((int32_t)((uint32_t)Mx - (uint32_t)Sx) > X) {
@@ -345,7 +477,7 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
           const uint32_t qw = (g >> 1) == 0 ? Qc[0] : (g >> 1) == 1 ? Qc[1] : Qc[2];
           const uint32_t sh = (g & 1u) << 4;
           mpos = (int32_t)(cells + 8u * g +
-                           first_reach(tbl, hw >> sh, qw >> sh, near16(S, wp.grp[g][lane] & 0xFFFFu), Mr));
+                           first_reach(tab, hw >> sh, qw >> sh, near16(S, wp.grp[g][lane] & 0xFFFFu), Mr));
           pbase = -1;
         }
       }
@@ -368,7 +500,7 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(LongArgs a) {
         uint32_t rlo, rhi, rsp, qlo, qhi, qsp;
         window32(dir ? a.refr : a.ref, rp + at, &rlo, &rhi, &rsp);
         window32(dir ? a.qryr : a.qry, qp + at, &qlo, &qhi, &qsp);
-        mpos = pbase + (int32_t)first_reach(tbl, rlo, qlo, pS, res);
+        mpos = pbase + (int32_t)first_reach(tab, rlo, qlo, pS, res);
         pbase = -1;
       }
       tcells += cells;
