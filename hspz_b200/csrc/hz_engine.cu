@@ -497,19 +497,35 @@ int pack_seq(hz_engine *e, const uint8_t *codes, uint64_t n, Packed *p) {
   return HZ_OK;
 }
 
-// The lockstep gate reads each cell's cost (the negated score) as a signed
-// byte and keeps positions in 32 bits; otherwise the lane-refill gate runs.
+// How the lockstep gate looks this matrix's scores up (CostMode), or -1 when
+// they don't fit it and the lane-refill gate runs.
+int cost_mode(const hz_engine *e) {
+  const int32_t *sub = e->cfg.sub_mat;
+  const int64_t X = e->cfg.xdrop;
+  int64_t top = 0, cost = 0;  // the largest score and cost
+  bool alike = true;          // complementary pairs score alike
+  for (int r = 0; r < 4; r++)
+    for (int q = 0; q < 4; q++) {
+      const int64_t v = sub[r * kNuc + q];
+      top = std::max(top, v);
+      cost = std::max(cost, -v);
+      alike = alike && v == sub[(r ^ 3) * kNuc + (q ^ 3)];
+    }
+  if (X < 0) return -1;
+  // drawdowns are kept in 16 bits (gate2_kernel), and long_kernel's group
+  // states modulo 2^16 (near16)
+  if (top <= 127 && cost <= 127) return X <= kGate2MaxXdrop && X + kRound * 255 < 32768 ? (alike ? kAlike : kGeneral) : -1;
+  // costs of 16 bits: the drop test's word holds kLeft costs above bit 15, the
+  // running costs a round's rise above xdrop, the rescoring a score below it
+  if (alike && cost * kLeft <= 32768 && top * kLeft + X + cost * kLeft <= 65535 && X + top <= 32767) return kWide;
+  return -1;
+}
+
+// The lockstep gate needs packed sequences and 32-bit positions.
 bool gate2_usable(const hz_engine *e) {
   if (e->gate_version != 2 || !e->ref_p.valid || !e->qry_p.valid) return false;
   if ((uint64_t)e->rlen + 128 >= (1ull << 32) || (uint64_t)e->qstore.len + 128 >= (1ull << 32)) return false;
-  for (int r = 0; r < 4; r++)
-    for (int q = 0; q < 4; q++) {
-      const int32_t v = e->cfg.sub_mat[r * kNuc + q];
-      if (v < -127 || v > 127) return false;
-    }
-  // drawdowns are kept in 16 bits (gate2_kernel), and long_kernel's group
-  // states modulo 2^16 (near16)
-  return e->cfg.xdrop >= 0 && e->cfg.xdrop <= kGate2MaxXdrop && (int64_t)e->cfg.xdrop + kRound * 255 < 32768;
+  return cost_mode(e) >= 0;
 }
 
 // Hits that `positions` seed positions of `per_pos` seeds are expected to
@@ -531,41 +547,32 @@ int wave_tile(const hz_engine *e, double hits) {
   return hits < 3e5 ? 64 : hits < 1.2e6 ? 128 : 256;
 }
 
-// Whether complementary ACGT pairs score alike: one score per index of the
-// packed kernels' lookup (CostTable).
-bool strands_alike(const int32_t *sub) {
-  for (int i = 0; i < 4; i++)
-    for (int j = 0; j < 4; j++)
-      if (sub[i * kNuc + j] != sub[(i ^ 3) * kNuc + (j ^ 3)]) return false;
-  return true;
-}
-
 // Prepares one instance of the lockstep gate for 'smem' bytes of shared
 // memory and returns its blocks per SM.
-template <bool SPARSE, bool GENERAL> int gate2_blocks(hz_engine *e, size_t smem, int *per_sm) {
+template <bool SPARSE, int MODE> int gate2_blocks(hz_engine *e, size_t smem, int *per_sm) {
   static size_t configured[64] = {0};
   static std::mutex mu;  // serving workers launch from several host threads
   {
     std::lock_guard<std::mutex> lock(mu);
     if (configured[e->device & 63] < smem) {
-      CK(cudaFuncSetAttribute(gate2_kernel<SPARSE, GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      CK(cudaFuncSetAttribute(gate2_kernel<SPARSE, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       configured[e->device & 63] = smem;
     }
   }
   *per_sm = e->gate_blocks_per_sm;
   if (*per_sm <= 0) {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, gate2_kernel<SPARSE, GENERAL>, kGate2Threads, smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, gate2_kernel<SPARSE, MODE>, kGate2Threads, smem));
     if (*per_sm < 1) *per_sm = 1;
   }
   return HZ_OK;
 }
 
-template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, Gate2Args &a2) {
+template <bool SPARSE, int MODE> int launch_gate2_as(hz_engine *e, Gate2Args &a2) {
   const size_t smem = gate2_smem((int)a2.tile);
   int per_sm = 0;
-  TRY((gate2_blocks<SPARSE, GENERAL>(e, smem, &per_sm)));
+  TRY((gate2_blocks<SPARSE, MODE>(e, smem, &per_sm)));
   const unsigned grid = std::min<unsigned>((unsigned)(e->sm_count * per_sm), e->gate_ring_blocks);
-  return e->launch("gate", [&] { gate2_kernel<SPARSE, GENERAL><<<grid, kGate2Threads, smem, e->st>>>(a2); });
+  return e->launch("gate", [&] { gate2_kernel<SPARSE, MODE><<<grid, kGate2Threads, smem, e->st>>>(a2); });
 }
 
 // The sparse tile setup (a lane per position) when a tile is expected to span
@@ -573,8 +580,7 @@ template <bool SPARSE, bool GENERAL> int launch_gate2_as(hz_engine *e, Gate2Args
 // each), from the hits per query position: seeds per position times the
 // average bucket.  256-hit tiles, 13 seeds, ps per hit by hits per position,
 // pairs against lanes: 4.7: 48.1 / 41.8, 9.5: 37.7 / 35.0, 18.9: 32.2 / 32.6,
-// 42: 29.3 / 32.2, 113: 28.4 / 32.4.  The one-table score lookup when
-// complementary pairs score alike (CostTable).
+// 42: 29.3 / 32.2, 113: 28.4 / 32.4.
 int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   Gate2Args a2;
   a2.g = ga;
@@ -607,28 +613,34 @@ int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
       e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 7.5 * positions_per_pass;
-  if (strands_alike(ga.sub)) return sparse ? launch_gate2_as<true, false>(e, a2) : launch_gate2_as<false, false>(e, a2);
-  return sparse ? launch_gate2_as<true, true>(e, a2) : launch_gate2_as<false, true>(e, a2);
+  int32_t top = 0;
+  for (int i = 0; i < 16; i++) top = std::max(top, ga.sub[(i >> 2) * kNuc + (i & 3)]);
+  a2.cost_base = (uint32_t)(kLeft * top);
+  switch (cost_mode(e)) {
+    case kAlike: return sparse ? launch_gate2_as<true, kAlike>(e, a2) : launch_gate2_as<false, kAlike>(e, a2);
+    case kGeneral: return sparse ? launch_gate2_as<true, kGeneral>(e, a2) : launch_gate2_as<false, kGeneral>(e, a2);
+    default: return sparse ? launch_gate2_as<true, kWide>(e, a2) : launch_gate2_as<false, kWide>(e, a2);
+  }
 }
 
 // The candidates of a wave, extended to their ends over the packed sequences
 // (long_kernel); runs only where the packed gate runs.
-template <bool GENERAL> int launch_long_as(hz_engine *e, const LongArgs &la) {
+template <int MODE> int launch_long_as(hz_engine *e, const LongArgs &la) {
   static bool configured[64] = {false};
   static std::mutex mu;
   const size_t smem = sizeof(LongSmem);
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!configured[e->device & 63]) {
-      CK(cudaFuncSetAttribute(long_kernel<GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      CK(cudaFuncSetAttribute(long_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       configured[e->device & 63] = true;
     }
   }
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, long_kernel<GENERAL>, kGateThreads, smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, long_kernel<MODE>, kGateThreads, smem));
   if (per_sm < 1) per_sm = 1;
   const unsigned grid = (unsigned)(e->sm_count * per_sm);
-  return e->launch("long", [&] { long_kernel<GENERAL><<<grid, kGateThreads, smem, e->st>>>(la); });
+  return e->launch("long", [&] { long_kernel<MODE><<<grid, kGateThreads, smem, e->st>>>(la); });
 }
 int launch_long(hz_engine *e, const GateArgs &ga) {
   LongArgs la;
@@ -651,7 +663,11 @@ int launch_long(hz_engine *e, const GateArgs &ga) {
   // each, a lane per direction 96 us (its longest extension) and 1 ns:
   // 60 000 candidates 222 / 167 us, 105 000 379 / 170
   la.wide_max = 32768;
-  return strands_alike(ga.sub) ? launch_long_as<false>(e, la) : launch_long_as<true>(e, la);
+  switch (cost_mode(e)) {
+    case kAlike: return launch_long_as<kAlike>(e, la);
+    case kGeneral: return launch_long_as<kGeneral>(e, la);
+    default: la.wide_max = 0xFFFFFFFFu; return launch_long_as<kWide>(e, la);
+  }
 }
 
 template <int TW> int launch_gate(hz_engine *e, const GateArgs &ga) {

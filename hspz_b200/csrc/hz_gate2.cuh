@@ -71,9 +71,10 @@ constexpr uint32_t kMaxTile = 256;
 constexpr int kGate2Threads = 128;
 constexpr int kGate2Warps = kGate2Threads / 32;
 constexpr int kGate2BlocksPerSm = 7;
-// Running costs are kept as kCostBase + A in 16 unsigned bits.  A falls by at
-// most kLeft * 127 in a round and rises by at most kLeft * 128 above
-// kCostBase + xdrop.
+// Running costs are kept as kCostBase + A in 16 unsigned bits (kWide: as
+// Gate2Args::cost_base + A).  A falls by at most kLeft times the largest score
+// in a round and rises by at most kLeft times the largest cost above the base
+// + xdrop; a direction that has ended starts later rounds at the base.
 constexpr uint32_t kCostBase = kLeft * 128;
 static_assert(kWindow == 96, "a window is read as four 32-base records, at any offset in the first");
 static_assert(kLeft % 8 == 0 && kRight % 8 == 0 && kLeft > kRight, "groups of eight cells; the left extension is longer");
@@ -125,6 +126,7 @@ struct Gate2Args {
   uint32_t *ring;       // gate2_ring_words words
   uint32_t tile;        // hits per warp tile, a multiple of 32, at most kMaxTile
   uint32_t soft_codes;  // bit c: code c (4..7) does not end every extension that meets it
+  uint32_t cost_base;   // kLeft * (largest score), for kWide matrices
   int32_t min_total;    // the smallest total with (i32)(f32)total >= hspthresh
 };
 
@@ -168,24 +170,40 @@ __device__ __forceinline__ void window_codes(const uint4 r[4], uint32_t a, uint3
   for (int k = 0; k < 3; k++) sp[k] = __funnelshift_r(r[k].z, r[k + 1].z, o);
 }
 
-// Costs (negated scores) of ACGT pairs as table bytes.  The index of a pair
-// is reference ^ query | parity << 2, parity the xor of the reference code's
-// two bits: with A C G T = 0..3 a complement flips both bits, so a matrix
-// with equal scores for complementary pairs -- HOXD70, and any matrix that
-// treats the strands alike -- has one score per index.  GENERAL matrices add
-// the reference code's low bit as bit 3 and hold a second table for it.
-template <bool GENERAL>
+// How a matrix's ACGT scores are looked up.  kAlike: complementary pairs score
+// alike and costs fit a signed byte; kGeneral: any byte scores; kWide: alike,
+// costs of 16 bits.
+enum CostMode : int { kAlike, kGeneral, kWide };
+
+// The costs of eight cells: bytes of the even cells, of the odd cells (kAlike,
+// kGeneral); 16-bit pairs of cells 0 2, 4 6, 1 3, 5 7 (kWide).
+template <int MODE> struct Cells8 {
+  uint32_t w[MODE == kWide ? 4 : 2];
+};
+
+// Costs (negated scores) of ACGT pairs.  The index of a pair is reference ^
+// query | parity << 2, parity the xor of the reference code's two bits: with
+// A C G T = 0..3 a complement flips both bits, so a matrix with equal scores
+// for complementary pairs -- HOXD70, and any matrix that treats the strands
+// alike -- has one score per index, and eight bytes hold them.  kGeneral
+// matrices add the reference code's low bit as bit 3 and hold a second table
+// for it; kWide ones look low and high bytes up apart and pair them, three
+// more permutes for four cells (a close-species score set, mismatches down to
+// -356, 68 M hits against a 10 Mbp bin: 3.7 ms in the lane-refill gate, 2.5
+// here).
+template <int MODE>
 struct CostTable {
-  uint32_t t[GENERAL ? 4 : 2];
+  uint32_t t[MODE == kAlike ? 2 : 4];
   __device__ __forceinline__ explicit CostTable(const int32_t *sub) {
 #pragma unroll
-    for (int i = 0; i < (GENERAL ? 4 : 2); i++) {
+    for (int i = 0; i < (MODE == kAlike ? 2 : 4); i++) {
       t[i] = 0;
 #pragma unroll
       for (int x = 0; x < 4; x++) {
-        const int low = i >> 1, parity = i & 1;
+        const int low = MODE == kGeneral ? i >> 1 : 0, parity = i & 1;
         const int r = (parity ^ low) << 1 | low;
-        t[i] |= (uint32_t)(uint8_t)(-sub[r * kNuc + (r ^ x)]) << (8 * x);
+        const uint32_t cost = (uint32_t)-sub[r * kNuc + (r ^ x)];
+        t[i] |= (cost >> (MODE == kWide && i >= 2 ? 8 : 0) & 0xFFu) << (8 * x);
       }
     }
   }
@@ -196,40 +214,66 @@ struct CostTable {
     uint2 e;
     e.x = (x & 0x33333333u) | ((p << 2) & ~0x33333333u);
     e.y = ((x >> 2) & 0x33333333u) | (p & ~0x33333333u);
-    if (GENERAL) {
+    if (MODE == kGeneral) {
       e.x |= (r & 0x11111111u) << 3;
       e.y |= (r << 1) & 0x88888888u;
     }
     return e;
   }
-  // The costs of the four cells whose indices are the low nibbles of s.
-  __device__ __forceinline__ uint32_t costs(uint32_t s) const {
-    if (!GENERAL) return permute(t[0], t[1], s);
+  // The cost bytes of the four cells whose indices are the low nibbles of s.
+  __device__ __forceinline__ uint32_t bytes(uint32_t s) const {
+    if (MODE != kGeneral) return permute(t[0], t[1], s);
     const uint32_t lo = s & 0x7777u;
     // bit 3 of each nibble as a byte mask: nibble 9 takes the sign of byte 1
     const uint32_t m = permute(0x00008000u, 0u, ((s >> 3) & 0x1111u) * 9u);
-    return (permute(t[0], t[1], lo) & ~m) | (permute(t[GENERAL ? 2 : 0], t[GENERAL ? 3 : 1], lo) & m);
+    return (permute(t[0], t[1], lo) & ~m) | (permute(t[MODE == kAlike ? 0 : 2], t[MODE == kAlike ? 1 : 3], lo) & m);
+  }
+  // The costs of eight cells from the indices of the even and the odd ones.
+  __device__ __forceinline__ Cells8<MODE> cells(uint32_t even, uint32_t odd) const {
+    Cells8<MODE> c;
+    if constexpr (MODE == kWide) {
+      const uint32_t el = permute(t[0], t[1], even), eh = permute(t[2], t[3], even);
+      const uint32_t ol = permute(t[0], t[1], odd), oh = permute(t[2], t[3], odd);
+      c.w[0] = permute(el, eh, 0x5140u);
+      c.w[1] = permute(el, eh, 0x7362u);
+      c.w[2] = permute(ol, oh, 0x5140u);
+      c.w[3] = permute(ol, oh, 0x7362u);
+    } else {
+      c.w[0] = bytes(even);
+      c.w[1] = bytes(odd);
+    }
+    return c;
   }
 };
 
-// Cell k (0..7) of an eight-cell group whose costs are e (even bases) and o
-// (odd bases): ascending bases for the right extension, descending for the
-// left one.  Which word, and which of its bytes.
-__device__ __forceinline__ constexpr int right_byte(int k) { return k >> 1; }
-__device__ __forceinline__ constexpr int left_byte(int k) { return 3 - (k >> 1); }
-__device__ __forceinline__ uint32_t right_word(int k, uint32_t e, uint32_t o) { return k & 1 ? o : e; }
-__device__ __forceinline__ uint32_t left_word(int k, uint32_t e, uint32_t o) { return k & 1 ? e : o; }
-
-// acc + the signed byte b of word.
-__device__ __forceinline__ uint32_t add_byte(uint32_t word, int b, uint32_t acc) {
-  return (uint32_t)__dp4a((int)word, 1 << (8 * b), (int)acc);
+// Of base b (0..7) of a group: the word of its cost, and the byte or half.
+template <int MODE> __device__ __forceinline__ uint32_t cost_word(const Cells8<MODE> &c, int b) {
+  return MODE == kWide ? c.w[MODE == kWide ? (b & 1) * 2 + (b >> 2) : 0] : c.w[b & 1];
+}
+// acc + the cost of base b.
+template <int MODE> __device__ __forceinline__ uint32_t add_cost(const Cells8<MODE> &c, int b, uint32_t acc) {
+  if (MODE == kWide) return (uint32_t)__dp2a_lo((int)cost_word(c, b), b & 2 ? 0x100 : 1, (int)acc);
+  return (uint32_t)__dp4a((int)cost_word(c, b), 1 << (8 * (b >> 1)), (int)acc);
+}
+// The costs of base br of one group and base bl of another, as 16-bit halves.
+template <int MODE>
+__device__ __forceinline__ uint32_t cost_pair(const Cells8<MODE> &r, int br, const Cells8<MODE> &l, int bl) {
+  uint32_t s;
+  if (MODE == kWide) {
+    const uint32_t x = br & 2u, y = 4u + (bl & 2u);
+    s = x | (x + 1) << 4 | y << 8 | (y + 1) << 12;
+  } else {
+    const uint32_t x = (uint32_t)br >> 1, y = 4u + ((uint32_t)bl >> 1);
+    s = x | (8u | x) << 4 | y << 8 | (8u | y) << 12;
+  }
+  return permute(cost_word(r, br), cost_word(l, bl), s);
 }
 
 // SPARSE: the setup for targets whose buckets hold few positions, where a
 // 128-hit tile spans many query positions (10-20 Mbp bins): a lane per
 // position instead of per (position, seed) pair.  The engine picks it from
-// the target's average bucket size.  GENERAL: see CostTable.
-template <bool SPARSE, bool GENERAL>
+// the target's average bucket size.  MODE: see CostMode.
+template <bool SPARSE, int MODE>
 __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel(const __grid_constant__ Gate2Args a2) {
   const GateArgs &a = a2.g;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -243,7 +287,8 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
   uint32_t *const slot_x = reinterpret_cast<uint32_t *>(mine + sizeof(GateWarp));
   uint32_t *const slot_q = slot_x + tile, *const slot_call = slot_q + tile;
   const uint32_t lane = threadIdx.x & 31;
-  const CostTable<GENERAL> tab(a.sub);
+  const CostTable<MODE> tab(a.sub);
+  const uint32_t cost_base = MODE == kWide ? a2.cost_base : kCostBase;
   const uint32_t thr = 0x7FFFu - (uint32_t)a.xdrop;  // drawdown + thr has bit 15 set when it exceeds xdrop
   const uint32_t thr2 = thr * 0x10001u;
   const bool soft = ((a2.ref[0].w | a2.qry[0].w) & a2.soft_codes) != 0;
@@ -457,7 +502,7 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
     uint2 sel[kWinChunks];
 #pragma unroll
     for (int c = 0; c < kWinChunks; c++) {
-      sel[c] = CostTable<GENERAL>::index(Rc[c], Qc[c]);
+      sel[c] = CostTable<MODE>::index(Rc[c], Qc[c]);
       wt.sel[c][lane] = sel[c];
     }
     // Every lane scores the whole window.  Per eight-cell group it keeps the
@@ -467,40 +512,40 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
     // 15 - kSolo - g.
     uint32_t flags = 0;
     {
-      uint32_t Ar = kCostBase + (draw & 0xFFFFu), Al = kCostBase + (draw >> 16), ml = kCostBase;
+      uint32_t Ar = cost_base + (draw & 0xFFFFu), Al = cost_base + (draw >> 16), ml = cost_base;
 #pragma unroll
       for (int g = 0; g < kSolo; g++) {  // the left extension's first groups
         const int f = kGroupsL - 1 - g;  // the group's place in the window
-        const uint32_t e = tab.costs((f & 1) ? sel[f >> 1].x >> 16 : sel[f >> 1].x),
-                       o = tab.costs((f & 1) ? sel[f >> 1].y >> 16 : sel[f >> 1].y);
+        const Cells8<MODE> lc = tab.cells((f & 1) ? sel[f >> 1].x >> 16 : sel[f >> 1].x,
+                                          (f & 1) ? sel[f >> 1].y >> 16 : sel[f >> 1].y);
         wt.grp[g][lane] = (Al - ml + thr) << 16;
         uint32_t hi = 0;
 #pragma unroll
         for (int k = 0; k < 8; k += 2) {
-          const uint32_t A1 = add_byte(left_word(k, e, o), left_byte(k), Al);
-          Al = add_byte(left_word(k + 1, e, o), left_byte(k + 1), A1);
+          const uint32_t A1 = add_cost(lc, 7 - k, Al);
+          Al = add_cost(lc, 6 - k, A1);
           ml = (uint32_t)__vimin3_s32((int)ml, (int)A1, (int)Al);
           hi = (uint32_t)__vimax3_s32((int)hi, (int)A1, (int)Al);
         }
         flags |= ((hi - ml + thr) & 0x8000u) << (16 - g);
       }
-      m2 = ml << 16 | kCostBase;
+      m2 = ml << 16 | cost_base;
       P = Al * 0x10000u + Ar;
 #pragma unroll
       for (int g = 0; g < kGroupsR; g++) {
         const int fl = kGroupsL - 1 - kSolo - g, fr = kGroupsL + g;
-        const uint32_t le = tab.costs((fl & 1) ? sel[fl >> 1].x >> 16 : sel[fl >> 1].x),
-                       lo = tab.costs((fl & 1) ? sel[fl >> 1].y >> 16 : sel[fl >> 1].y),
-                       re = tab.costs((fr & 1) ? sel[fr >> 1].x >> 16 : sel[fr >> 1].x),
-                       ro = tab.costs((fr & 1) ? sel[fr >> 1].y >> 16 : sel[fr >> 1].y);
+        const Cells8<MODE> lc = tab.cells((fl & 1) ? sel[fl >> 1].x >> 16 : sel[fl >> 1].x,
+                                          (fl & 1) ? sel[fl >> 1].y >> 16 : sel[fl >> 1].y);
+        const Cells8<MODE> rc = tab.cells((fr & 1) ? sel[fr >> 1].x >> 16 : sel[fr >> 1].x,
+                                          (fr & 1) ? sel[fr >> 1].y >> 16 : sel[fr >> 1].y);
         wt.grp[g + kSolo][lane] = P - m2 + thr2;
         uint32_t hi = 0;
 #pragma unroll
         for (int k = 0; k < 8; k += 2) {
-          const uint32_t Al1 = add_byte(left_word(k, le, lo), left_byte(k), Al);
-          const uint32_t Ar1 = add_byte(right_word(k, re, ro), right_byte(k), Ar);
-          Al = add_byte(left_word(k + 1, le, lo), left_byte(k + 1), Al1);
-          Ar = add_byte(right_word(k + 1, re, ro), right_byte(k + 1), Ar1);
+          const uint32_t Al1 = add_cost(lc, 7 - k, Al);
+          const uint32_t Ar1 = add_cost(rc, k, Ar);
+          Al = add_cost(lc, 6 - k, Al1);
+          Ar = add_cost(rc, k + 1, Ar1);
           const uint32_t P1 = Al1 * 0x10000u + Ar1;
           P = Al * 0x10000u + Ar;
           m2 = __vimin3_u16x2(m2, P1, P);
@@ -525,18 +570,13 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
       const uint32_t fl = kGroupsL - 1 - gl, fr = kGroupsL - kSolo + gr;
       const uint2 wl = wt.sel[fl >> 1][lane], wr = wt.sel[fr >> 1][lane];
       const uint32_t shl = (fl & 1u) << 4, shr = (fr & 1u) << 4;
-      const uint32_t le = tab.costs(wl.x >> shl), lo = tab.costs(wl.y >> shl), re = tab.costs(wr.x >> shr),
-                     ro = tab.costs(wr.y >> shr);
+      const Cells8<MODE> lc = tab.cells(wl.x >> shl, wl.y >> shl), rc = tab.cells(wr.x >> shr, wr.y >> shr);
       uint32_t E = permute(wt.grp[gr][lane], wt.grp[gl][lane], 0x7610u);
       uint32_t F = 0;      // bits 15 and 31: the direction has dropped
       uint32_t after = 0;  // 128 * (cells from the drop on: right + 16 * left)
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        // both cells' costs, sign-extended to 16 bits
-        const uint32_t rb = (uint32_t)right_byte(k), lb = 4u + (uint32_t)left_byte(k);
-        const uint32_t c2 = permute(right_word(k, re, ro), left_word(k, le, lo),
-                                    rb | (8u | rb) << 4 | lb << 8 | (8u | lb) << 12);
-        E = __viaddmax_u16x2(E, c2, thr2);
+        E = __viaddmax_u16x2(E, cost_pair(rc, k, lc, 7 - k), thr2);
         F = (F | E) & 0x80008000u;
         after = __dp4a(F, 0x10000100u, after);
       }
@@ -628,13 +668,14 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
         if (sp_l <= (uint32_t)kLeft && sp_l == use >> 16) exact |= soft_end(vr - sp_l, vq - sp_l);
       }
       const uint32_t cells = (use & 0xFFFFu) + (use >> 16) - (more_r ? 1u : 0u) - (more_l ? 1u : 0u);
-      const int32_t bound = (int32_t)(2u * kCostBase - (m2 & 0xFFFFu) - (m2 >> 16));
+      const int32_t bound = (int32_t)(2u * cost_base - (m2 & 0xFFFFu) - (m2 >> 16));
       const bool on = have && more && !exact;
       const bool cand = have && !on && (exact || bound >= a2.min_total);
       cells_acc += have && !on && !cand ? cells : 0u;
       if (cand) emit(hit * 32ull + lane, vr, vq, call);
       // the right extension goes on first; the left one waits if it does too
-      push(on, vr, vq, call, hit, more_r ? (uint32_t)kRight : (uint32_t)-kLeft, P - m2, bound,
+      push(on, vr, vq, call, hit, more_r ? (uint32_t)kRight : (uint32_t)-kLeft,
+           (P - m2) & ((more_r ? 0xFFFFu : 0u) | (more_l ? 0xFFFF0000u : 0u)), bound,
            (more_r ? kGoRight | (more_l ? kWaitLeft : 0u) : kGoLeft) | lane << 3 | cells << 8);
     } else if (ring_n) {
       // up to 32 waiting hits, from where they stand
@@ -675,7 +716,7 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
         if (on_l && ends_l == special >> 16 && use_l == ends_l && !more_l) exact |= soft_end(vr - use_l, vq - use_l);
       }
       const uint32_t cells = (state >> 8) + use_r + use_l - (more_r ? 1u : 0u) - (more_l ? 1u : 0u);
-      bound += (int32_t)((on_r ? kCostBase - (m2 & 0xFFFFu) : 0u) + (on_l ? kCostBase - (m2 >> 16) : 0u));
+      bound += (int32_t)((on_r ? cost_base - (m2 & 0xFFFFu) : 0u) + (on_l ? cost_base - (m2 >> 16) : 0u));
       const bool waits = (state & kWaitLeft) != 0;
       const bool on = have && !exact && (more_r || more_l || waits);
       const bool cand = have && !on && (exact || bound >= a2.min_total);
@@ -683,7 +724,7 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
       if (cand) emit(hit * 32ull + (state >> 3 & 31u), r0, q0, call);
       const uint32_t m = (on_r ? 0xFFFFu : 0u) | (on_l ? 0xFFFF0000u : 0u);
       push(on, r0, q0, call, hit, more_r ? off + kRight : waits ? (uint32_t)-kLeft : off - kLeft,
-           ((P - m2) & m) | (was & ~m), bound,
+           ((P - m2) & ((more_r ? 0xFFFFu : 0u) | (more_l ? 0xFFFF0000u : 0u))) | (was & ~m), bound,
            (more_r ? kGoRight | (state & kWaitLeft) : kGoLeft) | (state & 31u << 3) | cells << 8);
     } else {
       break;

@@ -8,7 +8,8 @@
 // candidate and marks it kDoneFlag, so the exact kernel is left with the
 // entropy and the accept.
 //
-// Few candidates (LongArgs::wide_max) go half a warp per direction, 256 cells
+// Few candidates (LongArgs::wide_max; all of them where scores are kWide, whose
+// group states would not fit 16 bits) go half a warp per direction, 256 cells
 // per step (long_wide): their time is that of the longest extension.  More go
 // one lane per candidate-direction, in rounds of kRound cells, which takes
 // fewer instructions per cell.  There the maximum's position is found without
@@ -61,14 +62,15 @@ __device__ __forceinline__ void window_round(const uint4 *__restrict__ blk, uint
 }
 
 // The costs (negated scores) of the eight cells whose codes are the low 16 bits
-// of r and q: even cells in .x, odd ones in .y, a byte each; and s plus the
-// score of cell k of them.
-template <typename TAB> __device__ __forceinline__ uint2 costs8(const TAB &tab, uint32_t r, uint32_t q) {
-  const uint2 sel = TAB::index(r, q);
-  return make_uint2(tab.costs(sel.x), tab.costs(sel.y));
+// of r and q; and s plus the score of cell k of them.
+template <int MODE>
+__device__ __forceinline__ Cells8<MODE> costs8(const CostTable<MODE> &tab, uint32_t r, uint32_t q) {
+  const uint2 sel = CostTable<MODE>::index(r, q);
+  return tab.cells(sel.x, sel.y);
 }
-__device__ __forceinline__ int32_t add_score(int32_t s, const uint2 &c, int k) {
-  return __dp4a((int)(k & 1 ? c.y : c.x), (int)(0xFFu << (8 * (k >> 1))), s);
+template <int MODE> __device__ __forceinline__ int32_t add_score(int32_t s, const Cells8<MODE> &c, int k) {
+  if (MODE == kWide) return __dp2a_lo((int)cost_word(c, k), k & 2 ? 0xFF00 : 0xFF, s);
+  return __dp4a((int)cost_word(c, k), (int)(0xFFu << (8 * (k >> 1))), s);
 }
 
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
@@ -110,9 +112,9 @@ struct LongSmem {
 
 // The first of the eight cells whose codes are the low 16 bits of r and q at
 // which the running sum, starting from s, equals target (8 if none does).
-template <typename TAB>
-__device__ __forceinline__ uint32_t first_reach(const TAB &tab, uint32_t r, uint32_t q, int32_t s, int32_t target) {
-  const uint2 cost = costs8(tab, r, q);
+template <int MODE>
+__device__ __forceinline__ uint32_t first_reach(const CostTable<MODE> &tab, uint32_t r, uint32_t q, int32_t s, int32_t target) {
+  const Cells8<MODE> cost = costs8(tab, r, q);
   uint32_t c = 8;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
@@ -130,9 +132,9 @@ __device__ __forceinline__ uint32_t first_reach(const TAB &tab, uint32_t r, uint
 // cost and the minimum before its cells, and with them whether one of its
 // cells drops.  The first lane that has one finds which; the minimum's first
 // cell is looked for where a step lowers it.
-template <bool GENERAL> __device__ __forceinline__ void long_wide(const LongArgs &a, uint32_t ncand) {
+template <int MODE> __device__ __forceinline__ void long_wide(const LongArgs &a, uint32_t ncand) {
   const uint32_t lane = threadIdx.x & 31, l = lane & 15u, half = lane >> 4;  // half 0: right, 1: left
-  const CostTable<GENERAL> tab(a.sub);
+  const CostTable<MODE> tab(a.sub);
   const int32_t X = a.xdrop;
   const uint4 *const rseq = half ? a.refr : a.ref, *const qseq = half ? a.qryr : a.qry;
   unsigned long long cells_acc = 0;
@@ -159,13 +161,12 @@ template <bool GENERAL> __device__ __forceinline__ void long_wide(const LongArgs
       uint32_t rlo, rhi, rsp, qlo, qhi, qsp;
       window32(rseq, v ? rp + k0 : 0u, &rlo, &rhi, &rsp);
       window32(qseq, v ? qp + k0 : 0u, &qlo, &qhi, &qsp);
-      const uint2 sel = CostTable<GENERAL>::index(rlo, qlo);
-      const uint32_t e[2] = {tab.costs(sel.x), tab.costs(sel.x >> 16)},
-                     o[2] = {tab.costs(sel.y), tab.costs(sel.y >> 16)};
+      const uint2 sel = CostTable<MODE>::index(rlo, qlo);
+      const Cells8<MODE> c8[2] = {tab.cells(sel.x, sel.y), tab.cells(sel.x >> 16, sel.y >> 16)};
       int32_t A[16];
 #pragma unroll
       for (int j = 0; j < 16; j++) {
-        const int32_t cost = (int32_t)(int8_t)((j & 1 ? o[j >> 3] : e[j >> 3]) >> (8 * ((j & 7) >> 1)));
+        const int32_t cost = (int32_t)add_cost(c8[j >> 3], j & 7, 0u);
         A[j] = (uint32_t)j < v ? cost : 0;
       }
       uint32_t sp = (rsp | qsp) & ((1u << v) - 1u);
@@ -263,17 +264,17 @@ template <bool GENERAL> __device__ __forceinline__ void long_wide(const LongArgs
   if (lane == 0 && cells_acc) atomicAdd(&a.tot->cells, cells_acc);
 }
 
-template <bool GENERAL>
+template <int MODE>
 __global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constant__ LongArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   LongSmem &sm = *reinterpret_cast<LongSmem *>(smem_raw);
   const uint32_t ncand = min(a.tot->cand, a.cand_cap);
   if (ncand <= a.wide_max) {
-    long_wide<GENERAL>(a, ncand);
+    long_wide<MODE>(a, ncand);
     return;
   }
   LongWarp &wp = sm.warp[threadIdx.x >> 5];
-  const CostTable<GENERAL> tab(a.sub);
+  const CostTable<MODE> tab(a.sub);
   const uint32_t lane = threadIdx.x & 31;
   const int32_t X = a.xdrop;
   unsigned long long cells_acc = 0;
@@ -355,13 +356,13 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constan
     int32_t gi = -1;
 #pragma unroll
     for (int h = 0; h < kChunks; h++) {
-      const uint2 sel = CostTable<GENERAL>::index(Rc[h], Qc[h]);
+      const uint2 sel = CostTable<MODE>::index(Rc[h], Qc[h]);
 #pragma unroll
       for (int gg = 0; gg < 2; gg++) {
         const int g = 2 * h + gg;
         wp.grp[g][lane] = __byte_perm((uint32_t)S, (uint32_t)M, 0x5410u);
         const int32_t Mg = M;
-        const uint2 cost = make_uint2(tab.costs(gg ? sel.x >> 16 : sel.x), tab.costs(gg ? sel.y >> 16 : sel.y));
+        const Cells8<MODE> cost = tab.cells(gg ? sel.x >> 16 : sel.x, gg ? sel.y >> 16 : sel.y);
         int32_t lo = 0x7FFFFFFF;
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
@@ -397,13 +398,13 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constan
             qw = Qc[k];
           }
         const uint32_t sh = (g & 1u) << 4;
-        const uint2 cost = costs8(tab, hw >> sh, qw >> sh);
+        const Cells8<MODE> cost = costs8(tab, hw >> sh, qw >> sh);
         if (a.late_max_safe && g != gv) {
           int32_t D = (int32_t)((uint32_t)Me - (uint32_t)Se);
           uint32_t dm = 0;
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            D = max(__dp4a((int)(i & 1 ? cost.y : cost.x), 1 << (8 * (i >> 1)), D), 0);
+            D = max((int32_t)add_cost(cost, i, (uint32_t)D), 0);
             dm |= (uint32_t)(D > X) << i;
           }
           if (dm) {

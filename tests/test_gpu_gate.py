@@ -40,6 +40,15 @@ def matrix(kind: str, xdrop: int):
         from hspz_b200 import build_sub_mat
         return build_sub_mat("n", xdrop)
     m = list(m)
+    if kind == "wide":  # a close-species score set: mismatches beyond a byte
+        rows = [[90, -330, -236, -356], [-330, 100, -318, -236], [-236, -318, 100, -330], [-356, -236, -330, 90]]
+        for r in range(4):
+            for c in range(4):
+                m[r * 8 + c] = rows[r][c]
+    if kind == "widest":  # the largest cost the lockstep gate takes
+        for r in range(4):
+            for c in range(4):
+                m[r * 8 + c] = 130 if r == c else -585
     if kind == "general":  # no two of the sixteen ACGT scores are tied by strand
         rng = np.random.default_rng(5)
         for r in range(4):
@@ -53,6 +62,8 @@ def matrix(kind: str, xdrop: int):
     ("default", 910, 96, 0), ("default", 910, 8, 0), ("default", 910, 65528, 0), ("default", 120, 128, 0),
     ("default", 0, 128, 0), ("default", 9000, 1024, 1), ("default", 20000, 256, 0),
     ("general", 910, 128, 0), ("general", 910, 104, 1), ("general", 150, 128, 0), ("ambiguous", 910, 128, 0),
+    ("wide", 910, 128, 0), ("wide", 910, 128, 1), ("wide", 910, 8, 0), ("wide", 300, 104, 0), ("wide", 20000, 1024, 1),
+    ("widest", 910, 128, 0), ("widest", 25000, 512, 0), ("widest", 32637, 256, 1),
     ("ambiguous", 910, 4096, 1)])
 def test_gate_edges_match_the_oracle(kind, xdrop, cap, sparse):
     t, q = sequences(xdrop + cap)
