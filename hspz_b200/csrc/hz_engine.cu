@@ -352,7 +352,7 @@ struct hz_engine {
   DBuf<uint32_t> pos_kmer, np_kmer;  // k-mer of every seed position, and of every position with hits
   uint32_t tile_cap = 1u << 23;  // entries of the gate's tile table (grows when a wave needs more)
   DBuf<unsigned long long> np_excl, call_hit_lo, scope_lo;
-  DBuf<HitNz> np_partial, np_grand;
+  DBuf<HitNz> np_partial;
   DBuf<WaveTotals> tot;
   DBuf<Cand> cand;
   DBuf<uint32_t> gate_ring;       // the lockstep gate's waiting hits, for gate_ring_blocks blocks
@@ -857,9 +857,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
   if (npos >= 0x7FFFFFFFull) return fail(HZ_E_INVALID, "a wave of %llu seed positions exceeds 2^31", (unsigned long long)npos);
   TRY(e->calls.ensure(n, s));
   TRY(e->pos_hits.ensure(npos, s));
-  uint64_t tiles = scan_tiles(npos);
-  TRY(e->np_partial.ensure(tiles + 1, s));
-  TRY(e->np_grand.ensure(1, s));
+  const uint32_t chunks = (uint32_t)((npos + kCountPerBlock - 1) / kCountPerBlock);
+  TRY(e->np_partial.ensure(chunks, s));
   TRY(e->np_excl.ensure(npos + 1, s));
   TRY(e->np_pos.ensure(npos + 1, s));
   TRY(e->pos_kmer.ensure(npos, s));
@@ -913,25 +912,20 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       TRY(e->launch("lookup_count", [&] {
         const uint32_t ch = lookup_chunks(npos);
         const uint64_t span = (uint64_t)ch * kCountPerBlock;
-        lookup_count_kernel<<<(unsigned)((npos + span - 1) / span), kCountThreads, 0, s>>>(w, ch, e->pos_hits.p,
-                                                                                          e->tot.p);
+        lookup_count_kernel<<<(unsigned)((npos + span - 1) / span), kCountThreads, 0, s>>>(
+            w, ch, e->pos_hits.p, e->tot.p, e->np_partial.p);
       }));
       TRY(e->launch(
           "np_scan",
           [&] {
-            np_reduce_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(e->pos_hits.p, npos, e->np_partial.p);
-            scan_partials_kernel<HitNz><<<1, kScanThreads, 0, s>>>(e->np_partial.p, tiles, e->np_grand.p);
-            np_emit_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(e->pos_hits.p, npos, e->np_partial.p,
-                                                                    e->np_excl.p, e->np_pos.p, e->pos_kmer.p,
-                                                                    e->np_kmer.p);
-            np_totals_kernel<<<1, 32, 0, s>>>(e->np_grand.p, e->tot.p, e->np_excl.p);
+            np_partials_kernel<<<1, kPartialThreads, 0, s>>>(e->np_partial.p, chunks, e->tot.p, e->np_excl.p,
+                                                             (uint32_t)tile, e->tile_first.p, e->tile_cap);
+            np_emit_kernel<<<chunks, kCountThreads, 0, s>>>(e->pos_hits.p, (uint32_t)npos, e->np_partial.p,
+                                                            e->np_excl.p, e->np_pos.p, e->pos_kmer.p, e->np_kmer.p,
+                                                            e->calls.p, (uint32_t)n, e->tot.p, (uint32_t)tile,
+                                                            e->tile_first.p, e->tile_call.p);
           },
-          4));
-      TRY(e->launch("tile_table", [&] {
-        tile_table_kernel<<<grid_for(npos, 256, e->sm_count * 8), 256, 0, s>>>(
-            e->np_excl.p, e->pos_hits.p, e->np_pos.p, e->calls.p, (uint32_t)n, e->tot.p, (uint32_t)tile,
-            e->tile_first.p, e->tile_call.p, e->tile_cap);
-      }));
+          2));
       TRY(e->launch("scopes", [&] {
         scopes_kernel<<<1, kScopeThreads, 0, s>>>(w, e->np_excl.p, e->np_pos.p, e->tot.p, e->max_hits,
                                                   e->call_hit_lo.p, e->call_nz_lo.p, e->scope_lo.p, e->scope_call.p,
@@ -1358,7 +1352,6 @@ void hz_engine_destroy(hz_engine *e) {
   e->call_hit_lo.release();
   e->scope_lo.release();
   e->np_partial.release();
-  e->np_grand.release();
   e->tot.release();
   e->cand.release();
   e->gate_ring.release();
@@ -1643,7 +1636,7 @@ int hz_generate_seeds(hz_engine *e, uint32_t slot, int rev, uint32_t start, uint
       const uint32_t ch = lookup_chunks(w.npos);
       const uint64_t span = (uint64_t)ch * kCountPerBlock;
       lookup_count_kernel<<<(unsigned)((w.npos + span - 1) / span), kCountThreads, 0, e->st>>>(w, ch, e->pos_hits.p,
-                                                                                              e->tot.p);
+                                                                                              e->tot.p, nullptr);
     }));
     CK(cudaMemcpyAsync(e->h_tot.p, e->tot.p, sizeof(WaveTotals), cudaMemcpyDeviceToHost, e->st));
     TRY(e->sync());
@@ -2395,7 +2388,7 @@ uint64_t wave_footprint(const hz_engine *w) {
        dbytes(w->pos_kmer) + dbytes(w->np_kmer) +
        dbytes(w->scope_call) + dbytes(w->raw_scope) + dbytes(w->tile_first) + dbytes(w->tile_call) +
        dbytes(w->np_excl) + dbytes(w->call_hit_lo) + dbytes(w->scope_lo) + dbytes(w->np_partial) +
-       dbytes(w->np_grand) + dbytes(w->tot) + dbytes(w->cand) + dbytes(w->gate_ring) + dbytes(w->raw) + dbytes(w->d_out);
+       dbytes(w->tot) + dbytes(w->cand) + dbytes(w->gate_ring) + dbytes(w->raw) + dbytes(w->d_out);
   for (const DBuf<uint32_t> *x : {&w->d_set, &w->d_perm_a, &w->d_perm_b, &w->d_kept, &w->d_total})
     b += dbytes(*x);
   return b;
@@ -2418,7 +2411,6 @@ void release_wave_buffers(hz_engine *w) {
   w->call_hit_lo.release();
   w->scope_lo.release();
   w->np_partial.release();
-  w->np_grand.release();
   w->cand.release();
   w->gate_ring.release();
   w->raw.release();

@@ -80,7 +80,7 @@ struct GateArgs {
   uint32_t cap;  // cells per direction before a hit goes to the exact kernel (multiple of 8, < 65536)
   Cand *cand;
   uint32_t cand_cap;
-  const uint32_t *tile_first;  // first position with hits of each tile (tile_table_kernel)
+  const uint32_t *tile_first;  // first position with hits of each tile (np_emit_kernel)
   const uint32_t *tile_call;   // call of that position
   // 7 * (largest substitution score) <= xdrop: no cell within seven cells
   // after a dropping cell can raise the maximum, so an extension that drops

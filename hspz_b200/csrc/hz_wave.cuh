@@ -2,7 +2,8 @@
 // one strand of one query each) processed by one fixed sequence of launches.
 //
 //   lookup_count   per query position: the capped hit counts of its seeds
-//   np_*           scan of the counts; compaction of positions with hits
+//   np_*           scan of the counts; compaction of positions with hits; the
+//                  gate's tile table
 //   scopes         per call: hit range and MAX_HITS dedup scopes
 //   gate           fused hit expansion + thread-per-hit X-drop score gate
 //   long           lane-per-candidate exact extension of the gate's long candidates
@@ -172,6 +173,8 @@ __device__ __forceinline__ uint32_t last_le(const unsigned long long *v, uint32_
 // the packed query, a thread takes four consecutive positions of a chunk:
 // one 32-base window gives their four k-mers, their four counts are
 // gathered together, and counts and k-mers go out as 16-byte stores.
+// A chunk's hits and positions with hits go out as one partial sum, so the
+// scan needs no pass of its own over the counts.
 constexpr int kCountThreads = 256;
 constexpr int kCountPerBlock = 1024;
 constexpr uint32_t kCountMaxChunks = 16;
@@ -185,7 +188,8 @@ inline uint32_t lookup_chunks(uint64_t npos) {
 
 __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, uint32_t chunks,
                                                                      uint32_t *__restrict__ pos_hits,
-                                                                     WaveTotals *__restrict__ tot) {
+                                                                     WaveTotals *__restrict__ tot,
+                                                                     HitNz *__restrict__ partial) {
   __shared__ uint32_t s_c0;
   const uint32_t base = blockIdx.x * chunks * kCountPerBlock;
   if (threadIdx.x == 0) s_c0 = call_of(w.calls, w.ncalls, base);
@@ -195,16 +199,16 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
   constexpr int kPer = kCountPerBlock / kCountThreads;
   static_assert(kPer % 4 == 0, "a thread's counts go out as 16-byte stores");
   const bool by_table = w.nbr_hits && w.per_pos > 1;
-  // kPer consecutive positions per thread from one 32-base packed window
-  const bool by_window = by_table && w.qp2 && !w.seeds && w.shape.size + kPer - 1 <= 32;
+  // kPer consecutive positions per thread from one 32-base packed window (a
+  // position's one seed, without transitions, is looked up in its bucket)
+  const bool by_window = (by_table || w.per_pos == 1) && w.qp2 && !w.seeds && w.shape.size + kPer - 1 <= 32;
   const uint32_t win_mask = w.shape.size >= 32 ? 0xFFFFFFFFu : (1u << w.shape.size) - 1u;
-#pragma unroll 1
-  for (uint32_t chunk = 0; chunk < chunks; chunk++) {
-    const uint32_t p0 = base + chunk * kCountPerBlock;
-    if (p0 >= w.npos) break;
+  // the thread's positions of a chunk; their hits and how many have any
+  auto count_chunk = [&](uint32_t p0) {
+    HitNz acc{0ull, 0u};
     if (by_window) {
       const uint32_t p = p0 + kPer * threadIdx.x;
-      if (p >= w.npos) continue;
+      if (p >= w.npos) return acc;
       while (c + 1 < w.ncalls && w.calls[c + 1].pos_off <= p) c++;
       const CallDev cd = w.calls[c];
       const uint32_t next_off = c + 1 < w.ncalls ? w.calls[c + 1].pos_off : 0xFFFFFFFFu;
@@ -235,8 +239,14 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
         sum[j] = 0;
         if (kmer[j] != kInvalidKmer) {
           valid++;
-          sum[j] = __ldg(w.nbr_hits + kmer[j]);
+          uint32_t beg;
+          sum[j] = by_table ? __ldg(w.nbr_hits + kmer[j]) : bucket(w, kmer[j], &beg);
         }
+      }
+#pragma unroll
+      for (uint32_t j = 0; j < kPer; j++) {
+        acc.h += sum[j];
+        acc.n += sum[j] > 0;
       }
       if (p + kPer - 1 < w.npos) {
 #pragma unroll
@@ -254,7 +264,7 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
             if (w.pos_kmer) w.pos_kmer[p + j] = kmer[j];
           }
       }
-      continue;
+      return acc;
     }
     if (by_table) {
       // all of the thread's k-mers first, then their neighbourhood counts, so
@@ -285,9 +295,11 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
         if (p < w.npos) {
           pos_hits[p] = sum[i];
           if (w.pos_kmer) w.pos_kmer[p] = kmer[i];
+          acc.h += sum[i];
+          acc.n += sum[i] > 0;
         }
       }
-      continue;
+      return acc;
     }
 #pragma unroll 1
     for (int i = 0; i < kPer; i++) {
@@ -319,106 +331,172 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
       }
       pos_hits[p] = sum;
       if (w.pos_kmer) w.pos_kmer[p] = kmer;
+      acc.h += sum;
+      acc.n += sum > 0;
+    }
+    return acc;
+  };
+  __shared__ HitNz s_part[kCountThreads / 32];
+#pragma unroll 1
+  for (uint32_t chunk = 0; chunk < chunks; chunk++) {
+    const uint32_t p0 = base + chunk * kCountPerBlock;
+    if (p0 >= w.npos) break;
+    HitNz acc = count_chunk(p0);
+    if (!partial) continue;
+    for (int d = 16; d > 0; d >>= 1) {
+      acc.h += __shfl_down_sync(0xffffffffu, acc.h, d);
+      acc.n += __shfl_down_sync(0xffffffffu, acc.n, d);
+    }
+    __syncthreads();  // the chunk before has been summed
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 1; i < kCountThreads / 32; i++) acc = Sum<HitNz>::add(acc, s_part[i]);
+      partial[p0 / kCountPerBlock] = acc;
     }
   }
   for (int d = 16; d > 0; d >>= 1) valid += __shfl_down_sync(0xffffffffu, valid, d);
   if ((threadIdx.x & 31) == 0 && valid) atomicAdd(&tot->valid, (unsigned long long)valid);
 }
 
-// Scan of (hits, has-hits) over positions, then compaction of the positions
-// with hits: np_excl = hits of the wave before the position, np_pos = its
-// flat index, np_kmer = its k-mer (when lookup_count kept the k-mers).
-__global__ void __launch_bounds__(kScanThreads) np_reduce_kernel(const uint32_t *__restrict__ pos_hits, uint64_t n,
-                                                                 HitNz *__restrict__ partial) {
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  HitNz acc = HitNz{0ull, 0u};
+// The scan of (hits, has-hits) over positions: the chunks' partial sums become
+// the hits and positions with hits before each, in one block; the totals go to
+// WaveTotals, with the sentinel np_excl[nz], and the gate's tile table is
+// checked against the total: tile_first[n_tiles] = nz, or status bit 2 when the
+// table is too small (the wave is then rerun with a larger one).
+constexpr int kPartialThreads = 1024;
+constexpr int kPartialItems = 4;
+
+__global__ void __launch_bounds__(kPartialThreads) np_partials_kernel(HitNz *partial, uint32_t n,
+                                                                      WaveTotals *__restrict__ t,
+                                                                      unsigned long long *__restrict__ np_excl,
+                                                                      uint32_t tile, uint32_t *__restrict__ tile_first,
+                                                                      uint32_t tile_cap) {
+  __shared__ HitNz s_warp[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  HitNz carry{0ull, 0u};
+  for (uint32_t off = 0; off < n; off += kPartialThreads * kPartialItems) {
+    const uint32_t base = off + threadIdx.x * kPartialItems;
+    HitNz v[kPartialItems], acc{0ull, 0u};
 #pragma unroll
-  for (int i = 0; i < kScanItems; i++)
-    if (base + i < n) {
-      uint32_t h = pos_hits[base + i];
-      acc.h += h;
-      acc.n += h > 0;
+    for (int i = 0; i < kPartialItems; i++) {
+      v[i] = base + i < n ? partial[base + i] : HitNz{0ull, 0u};
+      acc = Sum<HitNz>::add(acc, v[i]);
     }
-  HitNz tot;
-  block_exclusive_scan<HitNz>(acc, &tot);
-  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+    HitNz incl = acc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const HitNz up = Sum<HitNz>::shfl_up(incl, d);
+      if (lane >= (uint32_t)d) incl = Sum<HitNz>::add(incl, up);
+    }
+    __syncthreads();  // the round before has read the warps' sums
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    HitNz w = s_warp[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const HitNz up = Sum<HitNz>::shfl_up(w, d);
+      if (lane >= (uint32_t)d) w = Sum<HitNz>::add(w, up);
+    }
+    HitNz ex = carry;
+    if (warp) {
+      ex.h += __shfl_sync(0xffffffffu, w.h, warp - 1);
+      ex.n += __shfl_sync(0xffffffffu, w.n, warp - 1);
+    }
+    ex.h += incl.h - acc.h;
+    ex.n += incl.n - acc.n;
+#pragma unroll
+    for (int i = 0; i < kPartialItems; i++) {
+      if (base + i < n) partial[base + i] = ex;
+      ex = Sum<HitNz>::add(ex, v[i]);
+    }
+    carry.h += __shfl_sync(0xffffffffu, w.h, 31);
+    carry.n += __shfl_sync(0xffffffffu, w.n, 31);
+  }
+  if (threadIdx.x == 0) {
+    t->hits = carry.h;
+    t->nz = carry.n;
+    np_excl[carry.n] = carry.h;
+    const unsigned long long n_tiles = (carry.h + tile - 1) / tile;
+    if (n_tiles + 1 > tile_cap) t->status |= 4u;
+    else tile_first[n_tiles] = carry.n;
+  }
 }
 
-__global__ void __launch_bounds__(kScanThreads) np_emit_kernel(const uint32_t *__restrict__ pos_hits, uint64_t n,
-                                                               const HitNz *__restrict__ partial,
-                                                               unsigned long long *__restrict__ np_excl,
-                                                               uint32_t *__restrict__ np_pos,
-                                                               const uint32_t *__restrict__ pos_kmer,
-                                                               uint32_t *__restrict__ np_kmer) {
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t v[kScanItems];
-  HitNz acc = HitNz{0ull, 0u};
+// Compaction of the positions with hits: np_excl = hits of the wave before the
+// position, np_pos = its flat index, np_kmer = its k-mer (when lookup_count
+// kept the k-mers).  And the gate's tile table: tile_first[j] = the position
+// with hits that holds wave hit j * tile (positions tile the hit space, so
+// every tile start has exactly one), tile_call[j] = the call of that position;
+// a gate warp then finds its positions and call with three loads instead of
+// searches.  A block per chunk of lookup_count.
+__global__ void __launch_bounds__(kCountThreads) np_emit_kernel(
+    const uint32_t *__restrict__ pos_hits, uint32_t n, const HitNz *__restrict__ partial,
+    unsigned long long *__restrict__ np_excl, uint32_t *__restrict__ np_pos, const uint32_t *__restrict__ pos_kmer,
+    uint32_t *__restrict__ np_kmer, const CallDev *__restrict__ calls, uint32_t ncalls,
+    const WaveTotals *__restrict__ t, uint32_t tile, uint32_t *__restrict__ tile_first,
+    uint32_t *__restrict__ tile_call) {
+  constexpr int kPer = kCountPerBlock / kCountThreads;
+  static_assert(kPer == 4, "a thread's counts are one 16-byte load");
+  __shared__ HitNz s_warp[kCountThreads / 32];
+  __shared__ uint32_t s_c0;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t base = blockIdx.x * kCountPerBlock + threadIdx.x * kPer;
+  uint32_t v[kPer] = {0, 0, 0, 0}, km[kPer] = {0, 0, 0, 0};
+  if (base + kPer <= n) {
+    const uint4 x = *reinterpret_cast<const uint4 *>(pos_hits + base);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    if (np_kmer) {
+      const uint4 y = *reinterpret_cast<const uint4 *>(pos_kmer + base);
+      km[0] = y.x, km[1] = y.y, km[2] = y.z, km[3] = y.w;
+    }
+  } else {
+    for (int i = 0; i < kPer; i++)
+      if (base + i < n) {
+        v[i] = pos_hits[base + i];
+        if (np_kmer) km[i] = pos_kmer[base + i];
+      }
+  }
+  if (threadIdx.x == 0) s_c0 = call_of(calls, ncalls, base);
+  HitNz acc{0ull, 0u};
 #pragma unroll
-  for (int i = 0; i < kScanItems; i++) {
-    v[i] = base + i < n ? pos_hits[base + i] : 0u;
+  for (int i = 0; i < kPer; i++) {
     acc.h += v[i];
     acc.n += v[i] > 0;
   }
-  // the k-mers of the positions with hits, loaded while the block scans
-  uint32_t km[kScanItems];
+  HitNz incl = acc;
 #pragma unroll
-  for (int i = 0; i < kScanItems; i++) km[i] = np_kmer && v[i] ? pos_kmer[base + i] : 0u;
-  HitNz tot;
-  HitNz ex = block_exclusive_scan<HitNz>(acc, &tot);
-  HitNz off = partial[blockIdx.x];
-  ex.h += off.h;
-  ex.n += off.n;
+  for (int d = 1; d < 32; d <<= 1) {
+    const HitNz up = Sum<HitNz>::shfl_up(incl, d);
+    if (lane >= (uint32_t)d) incl = Sum<HitNz>::add(incl, up);
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  const HitNz before = partial[blockIdx.x];
+  const bool tiles = (t->status & 4u) == 0;
+  __syncthreads();
+  HitNz ex = before;
+  for (uint32_t i = 0; i < warp; i++) ex = Sum<HitNz>::add(ex, s_warp[i]);
+  ex.h += incl.h - acc.h;
+  ex.n += incl.n - acc.n;
+  uint32_t c = s_c0;
 #pragma unroll
-  for (int i = 0; i < kScanItems; i++) {
+  for (int i = 0; i < kPer; i++) {
     if (v[i]) {
       np_excl[ex.n] = ex.h;
-      np_pos[ex.n] = (uint32_t)(base + i);
+      np_pos[ex.n] = base + i;
       if (np_kmer) np_kmer[ex.n] = km[i];
-      ex.h += v[i];
+      const unsigned long long hi = ex.h + v[i];
+      unsigned long long j = (ex.h + tile - 1) / tile;
+      if (tiles && j * tile < hi) {
+        while (c + 1 < ncalls && calls[c + 1].pos_off <= base + i) c++;
+        for (; j * tile < hi; j++) {
+          tile_first[j] = ex.n;
+          tile_call[j] = c;
+        }
+      }
+      ex.h = hi;
       ex.n += 1;
     }
-  }
-}
-
-// The gate's tile table: tile_first[j] = the position with hits that holds
-// wave hit j * tile (positions tile the hit space, so every tile start has
-// exactly one), tile_call[j] = the call of that position, and
-// tile_first[n_tiles] = nz.  Lets a gate warp find its positions and call
-// with three loads instead of searches.  Sets status bit 2 when the
-// table is too small (the wave is then rerun with a larger one).
-__global__ void tile_table_kernel(const unsigned long long *__restrict__ np_excl, const uint32_t *__restrict__ pos_hits,
-                                  const uint32_t *__restrict__ np_pos, const CallDev *__restrict__ calls,
-                                  uint32_t ncalls, WaveTotals *__restrict__ t, uint32_t tile,
-                                  uint32_t *__restrict__ tile_first, uint32_t *__restrict__ tile_call, uint32_t cap) {
-  const uint32_t nz = t->nz;
-  const unsigned long long total = t->hits;
-  const unsigned long long n_tiles = (total + tile - 1) / tile;
-  if (n_tiles + 1 > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&t->status, 4u);
-    return;
-  }
-  uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nz; k += stride) {
-    const uint32_t p = np_pos[k];
-    unsigned long long lo = np_excl[k], hi = lo + pos_hits[p];
-    unsigned long long j = (lo + tile - 1) / tile;
-    if (j * tile >= hi) continue;
-    const uint32_t c = call_of(calls, ncalls, p);
-    for (; j * tile < hi; j++) {
-      tile_first[j] = k;
-      tile_call[j] = c;
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) tile_first[n_tiles] = nz;
-}
-
-// Grand totals of the scan into WaveTotals, and the sentinel np_excl[nz].
-__global__ void np_totals_kernel(const HitNz *__restrict__ grand, WaveTotals *__restrict__ t,
-                                 unsigned long long *__restrict__ np_excl) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    t->hits = grand->h;
-    t->nz = grand->n;
-    np_excl[grand->n] = grand->h;
   }
 }
 
