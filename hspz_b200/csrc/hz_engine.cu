@@ -316,18 +316,15 @@ struct hz_engine {
   // working memory of the on-device seed table build, kept between builds
   // of up to kKeepBuildScratch bytes (per-bin loads reuse it)
   struct BuildScratch {
-    DBuf<uint8_t> ascii, junk;
-    DBuf<uint32_t> kmers, flags, keys, vals, keys2, vals2, partial, total, hist, hpartial, excl, ipart;
+    DBuf<uint8_t> ascii;
+    DBuf<uint32_t> kmers, keys, vals, keys2, vals2, total, hist, hpartial, ipart;
     uint64_t bytes() const {
-      return ascii.cap + junk.cap +
-             4 * (kmers.cap + flags.cap + keys.cap + vals.cap + keys2.cap + vals2.cap + partial.cap + total.cap +
-                  hist.cap + hpartial.cap + excl.cap + ipart.cap);
+      return ascii.cap + 4 * (kmers.cap + keys.cap + vals.cap + keys2.cap + vals2.cap + total.cap + hist.cap +
+                              hpartial.cap + ipart.cap);
     }
     void release() {
       ascii.release();
-      junk.release();
-      for (auto *b : {&kmers, &flags, &keys, &vals, &keys2, &vals2, &partial, &total, &hist, &hpartial, &excl, &ipart})
-        b->release();
+      for (auto *b : {&kmers, &keys, &vals, &keys2, &vals2, &total, &hist, &hpartial, &ipart}) b->release();
     }
   } build;
   Packed ref_p;  // the reference packed for the lockstep gate
@@ -1432,91 +1429,88 @@ int hz_engine_load_target(hz_engine *e, const uint8_t *ref_ascii, uint64_t len) 
   uint64_t start_offset = step - offset;
   uint64_t num_steps = (len + offset) > sh.size ? (len + offset - sh.size) / step : 0;
 
-  // ASCII -> device codes
+  // ASCII -> device codes and the packed copy
   auto &bs = e->build;
-  DBuf<uint8_t> &ascii = bs.ascii, &junk = bs.junk;
+  DBuf<uint8_t> &ascii = bs.ascii;
   TRY(ascii.ensure(len + 1, st));
   TRY(e->ref.ensure(len, st));
-  TRY(junk.ensure(len + 1, st));
   if (len) CK(cudaMemcpyAsync(ascii.p, ref_ascii, len, cudaMemcpyHostToDevice, st));
   uint8_t *codes = e->ref.base();
   if (len)
     TRY(e->launch("encode", [&] {
-      encode_kernel<<<grid_for(len / 4 + 1, 256), 256, 0, st>>>(ascii.p, len, codes, junk.p);
+      encode_kernel<<<grid_for(len / 4 + 1, 256), 256, 0, st>>>(ascii.p, len, codes, nullptr);
     }));
+  TRY(pack_seq(e, e->ref.base(), len, &e->ref_p));
   TRY(e->index_table.ensure(index_len, st));
   CK(cudaMemsetAsync(e->index_table.p, 0, index_len * 4, st));
 
-  DBuf<uint32_t> &kmers = bs.kmers, &flags = bs.flags, &keys = bs.keys, &vals = bs.vals, &keys2 = bs.keys2,
-                 &vals2 = bs.vals2, &partial = bs.partial, &total = bs.total, &hist = bs.hist,
-                 &hpartial = bs.hpartial;
+  DBuf<uint32_t> &kmers = bs.kmers, &keys = bs.keys, &vals = bs.vals, &keys2 = bs.keys2, &vals2 = bs.vals2,
+                 &total = bs.total, &hist = bs.hist, &hpartial = bs.hpartial;
   uint64_t n_valid = 0;
   if (num_steps) {
+    // stable radix sort by k-mer, 8 bits per pass: each bucket keeps
+    // ascending position order (src/seed.rs:157-170).  The first pass reads
+    // the k-mers of all positions and leaves the invalid ones out.
+    const uint64_t tiles0 = (num_steps + kRadixTile - 1) / kRadixTile;
     TRY(kmers.ensure(num_steps, st));
-    TRY(flags.ensure(num_steps, st));
-    TRY(partial.ensure(scan_tiles(num_steps) + 1, st));
     TRY(total.ensure(1, st));
+    TRY(hist.ensure(tiles0 * kRadixBins, st));
+    TRY(hpartial.ensure(scan_tiles(tiles0 * kRadixBins) + 1, st));
+    const uint4 *blk = e->ref_p.half_ptr(0);
     TRY(e->launch("ref_kmer", [&] {
-      ref_kmer_kernel<<<grid_for(num_steps, 256), 256, 0, st>>>(codes, num_steps, start_offset, step, sh, kmers.p,
-                                                                flags.p);
+      ref_kmer_kernel<<<(unsigned)tiles0, kRadixThreads, 0, st>>>(codes, blk, num_steps, start_offset, step, sh,
+                                                                  kmers.p, hist.p, tiles0);
     }));
-    TRY(e->launch("ref_scan", [&] { exclusive_scan<uint32_t>(flags.p, flags.p, num_steps, partial.p, total.p, st); }, 3));
+    TRY(e->launch("radix_scan", [&] {
+      exclusive_scan<uint32_t>(hist.p, hist.p, tiles0 * kRadixBins, hpartial.p, total.p, st);
+    }, 3));
     uint32_t tot = 0;
     CK(cudaMemcpyAsync(&tot, total.p, 4, cudaMemcpyDeviceToHost, st));
     TRY(e->sync());
     n_valid = tot;
-    TRY(keys.ensure(n_valid + 1, st));
-    TRY(vals.ensure(n_valid + 1, st));
-    TRY(e->launch("ref_compact", [&] {
-      ref_compact_kernel<<<grid_for(num_steps, 256), 256, 0, st>>>(kmers.p, flags.p, num_steps, start_offset, step,
-                                                                   keys.p, vals.p, e->index_table.p);
-    }));
-    // stable radix sort by k-mer, 8 bits per pass: each bucket keeps
-    // ascending position order (src/seed.rs:157-170)
     if (n_valid) {
-      TRY(keys2.ensure(n_valid + 1, st));
-      TRY(vals2.ensure(n_valid + 1, st));
-      uint64_t rtiles = (n_valid + kRadixTile - 1) / kRadixTile;
-      TRY(hist.ensure(rtiles * kRadixBins, st));
-      TRY(hpartial.ensure(scan_tiles(rtiles * kRadixBins) + 1, st));
-      int bits = 2 * (int)sh.kmer_size;
+      TRY(keys.ensure(n_valid, st));
+      TRY(vals.ensure(n_valid, st));
+      TRY(keys2.ensure(n_valid, st));
+      TRY(vals2.ensure(n_valid, st));
+      TRY(e->pos_table.ensure(n_valid + 1, st));
+      const uint64_t rtiles = (n_valid + kRadixTile - 1) / kRadixTile;
+      const int bits = 2 * (int)sh.kmer_size;
       uint32_t *ka = keys.p, *va = vals.p, *kb = keys2.p, *vb = vals2.p;
       for (int shift = 0; shift < bits; shift += 8) {
-        TRY(e->launch("radix_hist", [&] {
-          radix_hist_kernel<<<(unsigned)rtiles, kRadixThreads, 0, st>>>(ka, n_valid, shift, hist.p, rtiles);
-        }));
-        TRY(e->launch("radix_scan", [&] {
-          exclusive_scan<uint32_t>(hist.p, hist.p, rtiles * kRadixBins, hpartial.p, total.p, st);
-        }, 3));
-        TRY(e->launch("radix_scatter", [&] {
-          radix_scatter_kernel<<<(unsigned)rtiles, kRadixThreads, 0, st>>>(ka, va, n_valid, shift, hist.p, rtiles, kb,
-                                                                          vb);
-        }));
+        uint32_t *vout = shift + 8 >= bits ? e->pos_table.p : vb;  // the last pass writes the table
+        if (shift == 0) {
+          TRY(e->launch("radix_scatter", [&] {
+            radix_scatter_kernel<true><<<(unsigned)tiles0, kRadixThreads, 0, st>>>(
+                kmers.p, nullptr, num_steps, 0, hist.p, tiles0, kb, vout, start_offset, step);
+          }));
+        } else {
+          TRY(e->launch("radix_hist", [&] {
+            radix_hist_kernel<<<(unsigned)rtiles, kRadixThreads, 0, st>>>(ka, n_valid, shift, hist.p, rtiles);
+          }));
+          TRY(e->launch("radix_scan", [&] {
+            exclusive_scan<uint32_t>(hist.p, hist.p, rtiles * kRadixBins, hpartial.p, total.p, st);
+          }, 3));
+          TRY(e->launch("radix_scatter", [&] {
+            radix_scatter_kernel<false><<<(unsigned)rtiles, kRadixThreads, 0, st>>>(
+                ka, va, n_valid, shift, hist.p, rtiles, kb, vout, 0, 0);
+          }));
+        }
         std::swap(ka, kb);
         std::swap(va, vb);
       }
-      TRY(e->pos_table.ensure(n_valid + 1, st));
-      CK(cudaMemcpyAsync(e->pos_table.p, va, n_valid * 4, cudaMemcpyDeviceToDevice, st));
+      // index_table = inclusive cumulative bucket counts (src/seed.rs:162-164)
+      TRY(bs.ipart.ensure(scan_tiles(index_len) + 1, st));
+      TRY(e->launch("index", [&] {
+        bucket_ends_kernel<<<grid_for(n_valid, 256), 256, 0, st>>>(ka, n_valid, e->index_table.p);
+        inclusive_scan<MaxU32>(reinterpret_cast<MaxU32 *>(e->index_table.p), index_len,
+                               reinterpret_cast<MaxU32 *>(bs.ipart.p), st);
+      }, 4));
     }
   }
   TRY(e->pos_table.ensure(1, st));
-  // index_table = inclusive cumulative bucket counts (src/seed.rs:162-164)
-  {
-    DBuf<uint32_t> &excl = bs.excl, &ipart = bs.ipart;
-    TRY(excl.ensure(index_len, st));
-    TRY(ipart.ensure(scan_tiles(index_len) + 1, st));
-    TRY(total.ensure(1, st));
-    TRY(e->launch("index_scan", [&] {
-      exclusive_scan<uint32_t>(e->index_table.p, excl.p, index_len, ipart.p, total.p, st);
-    }, 3));
-    TRY(e->launch("index_add", [&] {
-      add_counts_kernel<<<grid_for(index_len, 256), 256, 0, st>>>(excl.p, e->index_table.p, index_len);
-    }));
-    CK(cudaMemcpyAsync(e->index_table.p, excl.p, index_len * 4, cudaMemcpyDeviceToDevice, st));
-    TRY(e->sync());
-  }
+  TRY(e->sync());
   if (bs.bytes() > kKeepBuildScratch) bs.release();
-  TRY(pack_seq(e, e->ref.base(), len, &e->ref_p));
   TRY(build_nbr_hits(e, index_len));
   e->index_len = index_len;
   e->n_pos = n_valid;

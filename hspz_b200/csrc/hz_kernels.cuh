@@ -5,12 +5,14 @@
 #include <cuda_runtime.h>
 
 #include "hz_device.cuh"
+#include "hz_scan.cuh"
 
 namespace hz {
 
 // ---------------------------------------------------------------------------
 // Encoding.  ASCII -> device alphabet for the forward block and, in the same
-// pass, for its reverse complement (encode(REV_COMP[c]) read backwards).
+// pass, for its reverse complement (encode(REV_COMP[c]) read backwards; a
+// reference has none: rc null).
 // src/sequence.rs:66-86, 212-230.
 
 __constant__ uint8_t c_enc[256];
@@ -27,13 +29,14 @@ __global__ void encode_kernel(const uint8_t *__restrict__ ascii, uint64_t n, uin
 #pragma unroll
       for (int b = 0; b < 4; b++) f |= (uint32_t)c_enc[(w >> (8 * b)) & 0xFF] << (8 * b);
       *reinterpret_cast<uint32_t *>(fwd + i) = f;
+      if (rc)
 #pragma unroll
-      for (int b = 0; b < 4; b++) rc[n - 1 - (i + b)] = c_enc_rc[(w >> (8 * b)) & 0xFF];
+        for (int b = 0; b < 4; b++) rc[n - 1 - (i + b)] = c_enc_rc[(w >> (8 * b)) & 0xFF];
     } else {
       for (uint64_t j = i; j < i + 4 && j < n; j++) {
         uint8_t c = ascii[j];
         fwd[j] = c_enc[c];
-        rc[n - 1 - j] = c_enc_rc[c];
+        if (rc) rc[n - 1 - j] = c_enc_rc[c];
       }
     }
   }
@@ -168,44 +171,60 @@ __device__ __forceinline__ uint32_t kmer_12of19(uint32_t lo, uint32_t hi, uint32
 }
 
 // ---------------------------------------------------------------------------
-// Seed table on device (SeedTable::build, src/seed.rs:135-180): k-mers of
-// the strided reference positions, compaction of the valid ones in position
-// order, a stable radix sort by k-mer (so each bucket stays in ascending
-// position order), and the inclusive bucket counts.
+// Seed table on device (SeedTable::build, src/seed.rs:135-180): the k-mers of
+// the strided reference positions, a stable radix sort of the valid ones by
+// k-mer (so each bucket stays in ascending position order), and the inclusive
+// bucket counts.
 
-__global__ void ref_kmer_kernel(const uint8_t *__restrict__ codes, uint64_t num_steps, uint64_t start_offset,
-                                uint32_t step, ShapeDev sh, uint32_t *__restrict__ kmers,
-                                uint32_t *__restrict__ valid) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < num_steps; i += stride) {
-    uint32_t k = kmer_at(codes, start_offset + i * step, sh);
-    kmers[i] = k;
-    valid[i] = k != kInvalidKmer;
-  }
-}
-
-__global__ void ref_compact_kernel(const uint32_t *__restrict__ kmers, const uint32_t *__restrict__ excl,
-                                   uint64_t num_steps, uint64_t start_offset, uint32_t step,
-                                   uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
-                                   uint32_t *__restrict__ hist) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < num_steps; i += stride) {
-    uint32_t k = kmers[i];
-    if (k != kInvalidKmer) {
-      uint32_t at = excl[i];
-      keys[at] = k;
-      vals[at] = (uint32_t)(start_offset + i * step);
-      atomicAdd(&hist[k], 1u);
+// The k-mers (kInvalidKmer for windows with other bases) and each sort tile's
+// histogram of their lowest digit.  A thread takes four consecutive positions
+// from one packed window where it can.
+__global__ void __launch_bounds__(kRadixThreads) ref_kmer_kernel(const uint8_t *__restrict__ codes,
+                                                                 const uint4 *__restrict__ blk, uint64_t num_steps,
+                                                                 uint64_t start_offset, uint32_t step, ShapeDev sh,
+                                                                 uint32_t *__restrict__ kmers,
+                                                                 uint32_t *__restrict__ hist, uint64_t tiles) {
+  __shared__ uint32_t h[kRadixBins];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  const bool by_window = step == 1 && sh.size + 3 <= 32;
+  const uint32_t win_mask = sh.size >= 32 ? 0xFFFFFFFFu : (1u << sh.size) - 1u;
+  for (int g = 0; g < kRadixItems / 4; g++) {
+    const uint64_t e = (uint64_t)blockIdx.x * kRadixTile + (uint32_t)(g * kRadixThreads + threadIdx.x) * 4u;
+    if (e >= num_steps) break;
+    uint32_t k[4];
+    const uint32_t m = (uint32_t)min((unsigned long long)4, (unsigned long long)(num_steps - e));
+    if (by_window && m == 4) {
+      uint32_t lo, hi, sp;
+      window32(blk, (uint32_t)(start_offset + e), &lo, &hi, &sp);
+      const uint64_t w64 = (uint64_t)hi << 32 | lo;
+#pragma unroll
+      for (uint32_t j = 0; j < 4; j++)
+        k[j] = ((sp >> j) & win_mask) ? kInvalidKmer : sh.is_12of19 ? kmer_12of19(lo, hi, j) : kmer_runs(w64, j, sh);
+      *reinterpret_cast<uint4 *>(kmers + e) = make_uint4(k[0], k[1], k[2], k[3]);
+    } else {
+      for (uint32_t j = 0; j < m; j++) {
+        const uint64_t pos = start_offset + (e + j) * step;
+        k[j] = sh.size <= 32 ? kmer_packed(blk, (uint32_t)pos, sh) : kmer_at(codes, pos, sh);
+        kmers[e + j] = k[j];
+      }
     }
+    for (uint32_t j = 0; j < m; j++)
+      if (k[j] != kInvalidKmer) atomicAdd(&h[k[j] & 0xFFu], 1u);
   }
+  __syncthreads();
+  hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// inclusive = exclusive + count (index_table, src/seed.rs:162-164)
-__global__ void add_counts_kernel(uint32_t *__restrict__ excl_inout, const uint32_t *__restrict__ counts,
-                                  uint64_t n) {
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    excl_inout[i] += counts[i];
+// index_table[k] = keys up to and including bucket k, for the buckets that
+// have any (the others stay 0; a running maximum fills them,
+// src/seed.rs:162-164).
+__global__ void bucket_ends_kernel(const uint32_t *__restrict__ keys, uint64_t n, uint32_t *__restrict__ index_table) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint32_t k = keys[i];
+    if (i + 1 == n || keys[i + 1] != k) index_table[k] = (uint32_t)(i + 1);
+  }
 }
 
 }  // namespace hz

@@ -1,10 +1,11 @@
-// Device-wide exclusive scan (reduce-then-scan, three launches, no
-// inter-block waits) and a stable LSD radix sort of (u32 key, u32 value)
-// pairs built on it.  Used for seed-count prefixes, stream compaction and
+// Device-wide scans (reduce-then-scan, three launches, no inter-block waits)
+// and a stable LSD radix sort of (u32 key, u32 value) pairs built on them, for
 // the on-device seed-table build.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+
+#include "hz_device.cuh"
 
 namespace hz {
 
@@ -37,6 +38,18 @@ template <> struct Sum<HitNz> {
   __device__ __forceinline__ static HitNz add(HitNz a, HitNz b) { return HitNz{a.h + b.h, a.n + b.n}; }
   __device__ __forceinline__ static HitNz shfl_up(HitNz v, int d) {
     return HitNz{__shfl_up_sync(0xffffffffu, v.h, d), __shfl_up_sync(0xffffffffu, v.n, d)};
+  }
+};
+
+// A maximum, for scans that carry the last value seen in ascending data.
+struct MaxU32 {
+  uint32_t v;
+};
+template <> struct Sum<MaxU32> {
+  __device__ __forceinline__ static MaxU32 zero() { return MaxU32{0u}; }
+  __device__ __forceinline__ static MaxU32 add(MaxU32 a, MaxU32 b) { return MaxU32{max(a.v, b.v)}; }
+  __device__ __forceinline__ static MaxU32 shfl_up(MaxU32 v, int d) {
+    return MaxU32{__shfl_up_sync(0xffffffffu, v.v, d)};
   }
 };
 
@@ -114,8 +127,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(T *partial,
   if (threadIdx.x == 0 && grand) *grand = carry;
 }
 
-// Pass 3: per-tile exclusive scan plus the tile offset.
-template <typename T>
+// Pass 3: per-tile exclusive or inclusive scan plus the tile offset.
+template <typename T, bool INCLUSIVE = false>
 __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const T *__restrict__ in, uint64_t n,
                                                                   const T *__restrict__ partial,
                                                                   T *__restrict__ out) {
@@ -131,8 +144,9 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const T *__res
   T ex = Sum<T>::add(partial[blockIdx.x], block_exclusive_scan<T>(acc, &tot));
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) {
-    if (base + i < n) out[base + i] = ex;
-    ex = Sum<T>::add(ex, v[i]);
+    const T next = Sum<T>::add(ex, v[i]);
+    if (base + i < n) out[base + i] = INCLUSIVE ? next : ex;
+    ex = next;
   }
 }
 
@@ -150,6 +164,15 @@ inline void exclusive_scan(const T *in, T *out, uint64_t n, T *partial, T *grand
   scan_reduce_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, partial);
   scan_partials_kernel<T><<<1, kScanThreads, 0, s>>>(partial, tiles, grand);
   scan_apply_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, partial, out);
+}
+
+// Inclusive scan in place.
+template <typename T> inline void inclusive_scan(T *data, uint64_t n, T *partial, cudaStream_t s) {
+  const uint64_t tiles = scan_tiles(n);
+  if (n == 0) return;
+  scan_reduce_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(data, n, partial);
+  scan_partials_kernel<T><<<1, kScanThreads, 0, s>>>(partial, tiles, (T *)nullptr);
+  scan_apply_kernel<T, true><<<(unsigned)tiles, kScanThreads, 0, s>>>(data, n, partial, data);
 }
 
 // ---------------------------------------------------------------------------
@@ -176,49 +199,86 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_kernel(const uint32_
   hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Stable scatter: element order within a tile is round-major, lane-minor,
-// and ranks among equal digits follow that order, so the pass is stable.
+// Stable scatter of a tile, in element order: a warp takes 512 consecutive
+// elements, 32 at a time.  An element's rank among its digit is the warp's
+// count so far plus its earlier peers in the round; the warps' counts and the
+// digits' totals are scanned once per tile, the tile is put in order in shared
+// memory, and its runs (16 elements of a digit on average) go out side by
+// side.  FIRST: the keys are the k-mers of all strided positions, invalid ones
+// (kInvalidKmer) left out, and an element's value is its position.  16 M
+// pairs: 0.31 ms a pass with a block-wide round of ranks per 256 elements and
+// a scattered store each, 0.17 here.
+template <bool FIRST>
 __global__ void __launch_bounds__(kRadixThreads) radix_scatter_kernel(
     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t n, int shift,
     const uint32_t *__restrict__ offsets, uint64_t tiles, uint32_t *__restrict__ keys_out,
-    uint32_t *__restrict__ vals_out) {
+    uint32_t *__restrict__ vals_out, uint64_t start, uint32_t step) {
   constexpr int W = kRadixThreads / 32;
-  __shared__ uint32_t base_off[kRadixBins];        // global offset + running tile count
-  __shared__ uint32_t warp_cnt[W][kRadixBins];      // per-round per-warp digit counts -> prefixes
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  base_off[threadIdx.x] = offsets[(uint64_t)threadIdx.x * tiles + blockIdx.x];
-  uint64_t base = (uint64_t)blockIdx.x * kRadixTile;
-  for (int r = 0; r < kRadixItems; r++) {
-    for (int w = 0; w < W; w++) warp_cnt[w][threadIdx.x] = 0;
-    __syncthreads();
-    uint64_t e = base + (uint64_t)r * kRadixThreads + threadIdx.x;
-    bool ok = e < n;
-    uint32_t k = ok ? keys[e] : 0u;
-    uint32_t v = ok ? vals[e] : 0u;
-    uint32_t d = ok ? ((k >> shift) & 0xFF) : 0x100u;  // out-of-range lanes form their own group
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t rank = __popc(peers & lanemask_lt());
-    if (ok && rank == 0) warp_cnt[warp][d] = __popc(peers);
-    __syncthreads();
-    {
-      // exclusive prefix over warps for digit threadIdx.x
-      uint32_t acc = 0;
-      for (int w = 0; w < W; w++) {
-        uint32_t c = warp_cnt[w][threadIdx.x];
-        warp_cnt[w][threadIdx.x] = acc;
-        acc += c;
-      }
-      // stash the round total in a register; apply after the scatter reads base_off
-      __syncthreads();
-      if (ok) {
-        uint32_t dst = base_off[d] + warp_cnt[warp][d] + rank;
-        keys_out[dst] = k;
-        vals_out[dst] = v;
-      }
-      __syncthreads();
-      base_off[threadIdx.x] += acc;
+  __shared__ uint32_t cnt[W][kRadixBins];  // per warp: the digit's count so far, then what earlier warps hold
+  __shared__ uint32_t first[kRadixBins];   // the digit's first place in the ordered tile
+  __shared__ uint32_t goff[kRadixBins];    // its place in the output less that
+  __shared__ uint32_t warp_tot[W];
+  __shared__ uint32_t sk[kRadixTile], sv[kRadixTile];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int w = 0; w < W; w++) cnt[w][threadIdx.x] = 0;
+  const uint64_t base = (uint64_t)blockIdx.x * kRadixTile + warp * (kRadixTile / W);
+  uint32_t k[kRadixItems], v[kRadixItems], rank[kRadixItems];
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const uint64_t e = base + (uint32_t)i * 32 + lane;
+    k[i] = e < n ? keys[e] : kInvalidKmer;
+    v[i] = FIRST ? (uint32_t)(start + e * step) : e < n ? vals[e] : 0u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++) {
+    const uint64_t e = base + (uint32_t)i * 32 + lane;
+    const bool ok = e < n && (!FIRST || k[i] != kInvalidKmer);
+    const uint32_t d = ok ? (k[i] >> shift) & 0xFFu : 0x100u;  // left-out lanes form their own group
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    rank[i] = ok ? cnt[warp][d] + __popc(peers & lanemask_lt()) : 0xFFFFFFFFu;
+    __syncwarp();
+    if (ok && (peers & lanemask_lt()) == 0) cnt[warp][d] += __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  uint32_t total = 0;
+#pragma unroll
+  for (int w = 0; w < W; w++) {
+    const uint32_t c = cnt[w][threadIdx.x];
+    cnt[w][threadIdx.x] = total;
+    total += c;
+  }
+  uint32_t incl = total;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= (uint32_t)d) incl += up;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  uint32_t before = incl - total, all = 0;
+#pragma unroll
+  for (int w = 0; w < W; w++) {
+    if ((uint32_t)w < warp) before += warp_tot[w];
+    all += warp_tot[w];
+  }
+  first[threadIdx.x] = before;
+  goff[threadIdx.x] = offsets[(uint64_t)threadIdx.x * tiles + blockIdx.x] - before;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kRadixItems; i++)
+    if (rank[i] != 0xFFFFFFFFu) {
+      const uint32_t d = (k[i] >> shift) & 0xFFu, at = first[d] + cnt[warp][d] + rank[i];
+      sk[at] = k[i];
+      sv[at] = v[i];
     }
-    __syncthreads();
+  __syncthreads();
+  for (uint32_t p = threadIdx.x; p < all; p += kRadixThreads) {
+    const uint32_t key = sk[p], dst = goff[(key >> shift) & 0xFFu] + p;
+    keys_out[dst] = key;
+    vals_out[dst] = sv[p];
   }
 }
 
