@@ -312,6 +312,7 @@ struct hz_engine {
   // per k-mer: hits of its exact seed and all its transition seeds, capped
   // per seed (the hit count of a query position with that k-mer)
   DBuf<uint32_t> nbr_hits;
+  DBuf<uint16_t> nbr_live;  // and which of those seeds have hits, a bit each
   bool has_nbr = false;
   // working memory of the on-device seed table build, kept between builds
   // of up to kKeepBuildScratch bytes (per-bin loads reuse it)
@@ -573,16 +574,18 @@ template <bool SPARSE, int MODE> int launch_gate2_as(hz_engine *e, Gate2Args &a2
 }
 
 // The sparse tile setup (a lane per position) when a tile is expected to span
-// more than 7.5 passes of (position, seed) pairs (32 / per_pos positions
+// more than 6.5 passes of (position, seed) pairs (32 / per_pos positions
 // each), from the hits per query position: seeds per position times the
 // average bucket.  256-hit tiles, 13 seeds, ps per hit by hits per position,
-// pairs against lanes: 4.7: 48.1 / 41.8, 9.5: 37.7 / 35.0, 18.9: 32.2 / 32.6,
-// 42: 29.3 / 32.2, 113: 28.4 / 32.4.
+// pairs against lanes: 4.7: 48.1 / 34.8, 9.5: 37.8 / 32.5, 18.9: 32.1 / 32.0,
+// 28: 30.3 / 32.0, 42: 29.2 / 32.1, 113: 28.3 / 32.3; 128-hit tiles: 9.5:
+// 39.2 / 36.5, 18.9: 33.7 / 37.5.
 int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   Gate2Args a2;
   a2.g = ga;
   a2.ref = e->ref_p.half_ptr(0) - kPackPad;
   a2.qry = e->qry_p.half_ptr(0) - kPackPad;
+  a2.nbr_live = e->has_nbr ? e->nbr_live.p : nullptr;
   a2.ring = e->gate_ring.p;
   a2.tile = (uint32_t)tile;
   a2.soft_codes = 0;
@@ -609,7 +612,7 @@ int launch_gate2(hz_engine *e, const GateArgs &ga, int tile) {
   const double hits_per_pos = std::max(expected_hits(e, 1, ga.w.per_pos), 1e-9);
   const double positions_per_pass = (double)(32 / ga.w.per_pos);
   const bool sparse =
-      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 7.5 * positions_per_pass;
+      e->gate_sparse >= 0 ? e->gate_sparse == 1 : (double)a2.tile / hits_per_pos > 6.5 * positions_per_pass;
   int32_t top = 0;
   for (int i = 0; i < 16; i++) top = std::max(top, ga.sub[(i >> 2) * kNuc + (i & 3)]);
   a2.cost_base = (uint32_t)(kLeft * top);
@@ -1095,19 +1098,21 @@ void query_calls(const hz_engine *e, uint32_t qid, std::vector<HostCall> *out) {
   }
 }
 
-// The per-k-mer neighbourhood hit counts, for seed patterns of at most 14
-// care positions (a 4^k table of at most 1 GB); larger patterns look up
+// The per-k-mer neighbourhood hit counts and live seeds, for seed patterns of at most 14
+// care positions (4^k tables of at most 1 and 0.5 GB); larger patterns look up
 // every seed of a position instead.
 int build_nbr_hits(hz_engine *e, uint64_t index_len) {
   e->has_nbr = false;
   if (e->shape.kmer_size > 14) return HZ_OK;
   cudaStream_t s = e->st;
   TRY(e->nbr_hits.ensure(index_len, s));
+  TRY(e->nbr_live.ensure(index_len, s));
   const uint32_t *idx = e->index_table.p;
   uint32_t *out = e->nbr_hits.p;
+  uint16_t *live = e->nbr_live.p;
   const uint32_t ks = e->shape.kmer_size, cap = e->cfg.occ_cap;
   TRY(e->launch("nbr_hits", [&] {
-    nbr_hits_kernel<<<grid_for(index_len, 256), 256, 0, s>>>(idx, index_len, ks, cap, out);
+    nbr_hits_kernel<<<grid_for(index_len, 256), 256, 0, s>>>(idx, index_len, ks, cap, out, live);
   }));
   e->has_nbr = true;
   return HZ_OK;
@@ -1328,6 +1333,7 @@ void hz_engine_destroy(hz_engine *e) {
     e->index_table.release();
     e->pos_table.release();
     e->nbr_hits.release();
+    e->nbr_live.release();
     e->ref_p.release();
   }
   if (!e->aliases_query) {
@@ -2445,6 +2451,8 @@ void share_target(hz_engine *w, const hz_engine *e) {
   w->pos_table.cap = e->pos_table.cap;
   w->nbr_hits.p = e->nbr_hits.p;
   w->nbr_hits.cap = e->nbr_hits.cap;
+  w->nbr_live.p = e->nbr_live.p;
+  w->nbr_live.cap = e->nbr_live.cap;
   w->has_nbr = e->has_nbr;
   w->n_pos = e->n_pos;
   w->ref_p = e->ref_p;

@@ -126,9 +126,11 @@ __device__ __forceinline__ uint32_t bucket(const WaveIn &w, uint32_t k, uint32_t
 
 // Per k-mer: the capped hit counts of its exact seed and of its kmer_size
 // transition seeds, summed -- what lookup_count adds up for a query
-// position with that k-mer (u32, wrapping like that sum).
+// position with that k-mer (u32, wrapping like that sum) -- and which of them
+// have hits, bit v for seed v (kmer_size <= 14: 15 bits), which the gate's
+// sparse setup looks up one by one.
 __global__ void nbr_hits_kernel(const uint32_t *__restrict__ index_table, uint64_t n, uint32_t kmer_size,
-                                uint32_t occ_cap, uint32_t *__restrict__ out) {
+                                uint32_t occ_cap, uint32_t *__restrict__ out, uint16_t *__restrict__ live) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const uint32_t kmer = (uint32_t)i;
@@ -142,14 +144,16 @@ __global__ void nbr_hits_kernel(const uint32_t *__restrict__ index_table, uint64
         lo[v] = k ? __ldg(index_table + k - 1) : 0u;
       }
     }
-    uint32_t sum = 0;
+    uint32_t sum = 0, bits = 0;
 #pragma unroll
     for (uint32_t v = 0; v < kMaxCare + 1; v++) {
       uint32_t c = hi[v] - lo[v];
       if (occ_cap && c > occ_cap) c = 0;
       sum += c;
+      bits |= c ? 1u << v : 0u;
     }
     out[i] = sum;
+    live[i] = (uint16_t)bits;
   }
 }
 

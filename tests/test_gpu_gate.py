@@ -81,6 +81,25 @@ def test_gate_edges_match_the_oracle(kind, xdrop, cap, sparse):
         assert st[k] == st_o[k], k
 
 
+@pytest.mark.parametrize("seed,occ_cap,transitions", [
+    ("12of19", 0, True), ("12of19", 2, True), ("12of19", 0, False), ("14of22", 1, True), ("1111", 200, True),
+    ("1" * 8 + "0" + "1" * 7, 0, True)])  # 15 care positions: no per-k-mer tables
+def test_sparse_setup_skips_seeds_without_hits(seed, occ_cap, transitions):
+    t, q = sequences(31)
+    if seed == "1111":
+        t, q = t[:3000], q[:2000]
+    sm = EngineConfig().sub_mat
+    want, st_o = oracle_run(t, q, sm, seed=seed, occ_cap=occ_cap, transitions=transitions)
+    with engine_for(sm, seed=seed, occ_cap=occ_cap, transitions=transitions) as e:
+        e.set_tuning(gate_sparse=1)
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
+
+
 @pytest.mark.parametrize("n", [19, 20, 40, 57, 95, 96, 97, 130])
 def test_short_sequences_match_the_oracle(n):
     """Targets and queries around a window long: windows reach past both ends."""
