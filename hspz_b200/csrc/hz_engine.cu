@@ -238,7 +238,7 @@ unsigned grid_for(uint64_t n, unsigned threads, unsigned cap = 148u * 64u) {
 
 }  // namespace
 
-// A sequence packed 2 bits per base for the lockstep gate (pack2_kernel):
+// A sequence packed 2 bits per base for the kernels that extend (pack2_kernel):
 // the forward half and the reversed half, each `half` bases, codes and
 // special masks, after kPackPad zero records (a gate window may start before
 // the sequence).  Component w of the first record holds the non-ACGT codes
@@ -841,6 +841,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
              std::vector<WaveRecord> *out, hz_stats *st, bool device_dedup, bool graph = false,
              DeferredDedup *defer = nullptr, uint32_t call_base = 0) {
   if (n == 0) return HZ_OK;
+  // a load or a swap that failed half way leaves its sequence unpacked
+  if (!e->ref_p.valid || !e->qry_p.valid) return fail(HZ_E_STATE, "a sequence was not loaded completely");
   cudaStream_t s = e->st;
   uint64_t npos = 0;
   TRY(e->h_calls.ensure(n));
@@ -967,6 +969,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       xa.ref = w.ref;
       xa.rlen = w.rlen;
       xa.qbuf = w.qbuf;
+      xa.ref2 = e->ref_p.half_ptr(0);
+      xa.qry2 = e->qry_p.half_ptr(0);
       xa.calls = w.calls;
       xa.cand = e->cand.p;
       xa.cand_cap = e->cand_cap;

@@ -653,6 +653,7 @@ struct ExactArgs {
   const uint8_t *ref;
   uint32_t rlen;
   const uint8_t *qbuf;
+  const uint4 *ref2, *qry2;  // packed forward halves of both (pack2_kernel)
   const CallDev *calls;
   const Cand *cand;
   uint32_t cand_cap;
@@ -809,6 +810,47 @@ __device__ __forceinline__ int32_t exact_argmax(const uint8_t *ref, const uint8_
 
 constexpr int kExactThreads = 128;
 
+// How many of the first v of 32 base pairs (codes r, rh and q, qh, sixteen a
+// word) match, by code, in four 16-bit fields -- packed as the reference packs
+// its match counters, so that sums carry from one field into the next as its
+// do.  special: pairs with a base outside ACGT, which never count.
+__device__ __forceinline__ unsigned long long matches32(uint32_t r, uint32_t rh, uint32_t q, uint32_t qh,
+                                                        uint32_t special, uint32_t v) {
+  // planes of 32 bases, base k at bit 2k (its first sixteen) or 2(k - 16) + 1
+  const uint32_t x = r ^ q, xh = rh ^ qh;
+  uint32_t eq = (~(x | x >> 1) & 0x55555555u) | (~(xh | xh >> 1) & 0x55555555u) << 1;
+  if (v < 32) {
+    const uint32_t first = v >= 16 ? 0xFFFFFFFFu : (1u << (2 * v)) - 1u;
+    const uint32_t second = v <= 16 ? 0u : (1u << (2 * (v - 16))) - 1u;
+    eq &= (first & 0x55555555u) | (second & 0x55555555u) << 1;
+  }
+  if (special) {
+    uint32_t lo = special & 0xFFFFu, hi = special >> 16;
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) {
+      const uint32_t m = d == 8 ? 0x00FF00FFu : d == 4 ? 0x0F0F0F0Fu : d == 2 ? 0x33333333u : 0x55555555u;
+      lo = (lo | lo << d) & m;
+      hi = (hi | hi << d) & m;
+    }
+    eq &= ~(lo | hi << 1);
+  }
+  const uint32_t b0 = eq & ((r & 0x55555555u) | (rh & 0x55555555u) << 1);
+  const uint32_t b1 = eq & ((r >> 1 & 0x55555555u) | (rh & 0xAAAAAAAAu));
+  const uint32_t n3 = (uint32_t)__popc(b0 & b1), n1 = (uint32_t)__popc(b0) - n3, n2 = (uint32_t)__popc(b1) - n3;
+  const uint32_t n0 = (uint32_t)__popc(eq) - n1 - n2 - n3;
+  // at most 32 a field
+  return (unsigned long long)(n2 | n3 << 16) << 32 | (n0 | n1 << 16);
+}
+
+// The candidates' entropy and accept, and before it the extension of those
+// that long_kernel has not extended.  A warp takes up to 32 candidates, a lane
+// each: the double-precision logarithms and divisions of an entropy, about 250
+// instructions, are then issued once for 32 candidates; with a warp per
+// candidate they, and its strided byte loads, were the kernel's time.  The
+// bases that match are counted eight lanes a candidate, four candidates at a
+// time, 32 bases a lane from the packed sequences.  2.3 k candidates take 10.5
+// us (a warp each 9), 46 k 11 (39), 105 k 14 (80), 631 k 34 (437), 3.5 M 102
+// (2394): near the 32 bytes of each candidate and its windows' sectors.
 __global__ void __launch_bounds__(kExactThreads) exact_kernel(ExactArgs a) {
   __shared__ int32_t sub[64];
   if (threadIdx.x < 64) sub[threadIdx.x] = a.sub[threadIdx.x];
@@ -816,51 +858,78 @@ __global__ void __launch_bounds__(kExactThreads) exact_kernel(ExactArgs a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t ncand = min(a.tot->cand, a.cand_cap);
   unsigned long long cells_acc = 0;
-  const uint32_t warps = gridDim.x * (blockDim.x / 32);
-  for (uint32_t i = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; i < ncand; i += warps) {
-    Cand cd = a.cand[i];
+  const uint32_t warps = gridDim.x * (kExactThreads / 32), warp = blockIdx.x * (kExactThreads / 32) + threadIdx.x / 32;
+  // few candidates go to all warps
+  const uint32_t each = min(max((ncand + warps - 1) / warps, 1u), 32u);
+  const int32_t T = a.hspthresh;
+  const int32_t T3 = (int32_t)((uint32_t)T * 3u);
+  for (uint32_t base = warp * each; base < ncand; base += warps * each) {
+    const bool have = lane < each && base + lane < ncand;
+    Cand cd{};
+    if (have) cd = a.cand[base + lane];
     const bool done = (cd.call & kDoneFlag) != 0;  // long_kernel extended it: maxima and positions known
-    const bool is_long = !done && (cd.call & kLongFlag) != 0;
-    CallDev call = a.calls[cd.call & ~(kLongFlag | kDoneFlag)];
-    const uint8_t *qry = a.qbuf + call.qoff;
-    uint32_t q0 = cd.q0 - call.qoff, r0 = cd.r0;
-    unsigned long long cells = 0;
-    int32_t rmax, rpos, lmax, lpos;
-    if (done) {
-      rmax = cd.rmax;
-      lmax = cd.lmax;
-      rpos = cd.rpos;
-      lpos = cd.lpos;
-    } else if (is_long) {  // reached the gate's cap: long runs, four cells per lane
-      exact_dir4<false>(a.ref, qry, sub, a.xdrop, r0, q0, min(a.rlen - r0, call.qlen - q0), lane, &rmax, &rpos,
-                        &cells);
-      exact_dir4<true>(a.ref, qry, sub, a.xdrop, r0, q0, min(r0, q0), lane, &lmax, &lpos, &cells);
-    } else {  // both maxima came from the gate; only their positions are left to find
-      rmax = cd.rmax;
-      lmax = cd.lmax;
-      rpos = exact_argmax<false>(a.ref, qry, sub, r0, q0, min(a.rlen - r0, call.qlen - q0), rmax, lane);
-      lpos = exact_argmax<true>(a.ref, qry, sub, r0, q0, min(r0, q0), lmax, lane);
-    }
-    if (is_long) cells_acc += cells;
-    int32_t total = (int32_t)((uint32_t)rmax + (uint32_t)lmax);
-    int32_t extent = (int32_t)((uint32_t)rpos + (uint32_t)lpos);
-    int32_t T = a.hspthresh;
-    int32_t T3 = (int32_t)((uint32_t)T * 3u);
-    double entropy = 1.0;
-    if (total >= T && total <= T3 && a.noentropy == 0) {
-      uint32_t rs = r0 - (uint32_t)lpos, qs = q0 - (uint32_t)lpos;
-      int32_t positions = (int32_t)((uint32_t)extent + 1u);
-      unsigned long long packed = 0;  // four 16-bit match counters, packed as the reference packs them
-      for (int32_t j = (int32_t)lane; j < positions; j += 32) {
-        uint32_t x = a.ref[rs + (uint32_t)j], y = qry[qs + (uint32_t)j];
-        if (x == y && x < 4) packed += 1ull << (16 * x);
+    int32_t rmax = cd.rmax, lmax = cd.lmax, rpos = cd.rpos, lpos = cd.lpos;
+    for (uint32_t left = __ballot_sync(0xffffffffu, have && !done); left; left &= left - 1) {
+      const int src = __ffs((int)left) - 1;
+      const uint32_t word = __shfl_sync(0xffffffffu, cd.call, src);
+      const CallDev call = a.calls[word & ~(kLongFlag | kDoneFlag)];
+      const uint8_t *qry = a.qbuf + call.qoff;
+      const uint32_t q0 = __shfl_sync(0xffffffffu, cd.q0, src) - call.qoff, r0 = __shfl_sync(0xffffffffu, cd.r0, src);
+      int32_t m0 = __shfl_sync(0xffffffffu, cd.rmax, src), m1 = __shfl_sync(0xffffffffu, cd.lmax, src), p0, p1;
+      if (word & kLongFlag) {  // reached the gate's cap: long runs, four cells per lane
+        unsigned long long cells = 0;
+        exact_dir4<false>(a.ref, qry, sub, a.xdrop, r0, q0, min(a.rlen - r0, call.qlen - q0), lane, &m0, &p0, &cells);
+        exact_dir4<true>(a.ref, qry, sub, a.xdrop, r0, q0, min(r0, q0), lane, &m1, &p1, &cells);
+        cells_acc += cells;
+      } else {  // both maxima came from the gate; only their positions are left to find
+        p0 = exact_argmax<false>(a.ref, qry, sub, r0, q0, min(a.rlen - r0, call.qlen - q0), m0, lane);
+        p1 = exact_argmax<true>(a.ref, qry, sub, r0, q0, min(r0, q0), m1, lane);
       }
+      if ((int)lane == src) {
+        rmax = m0;
+        rpos = p0;
+        lmax = m1;
+        lpos = p1;
+      }
+    }
+    const int32_t total = (int32_t)((uint32_t)rmax + (uint32_t)lmax);
+    const int32_t extent = (int32_t)((uint32_t)rpos + (uint32_t)lpos);
+    const uint32_t rs = cd.r0 - (uint32_t)lpos, qs = cd.q0 - (uint32_t)lpos;  // qs: in the query store
+    const int32_t positions = (int32_t)((uint32_t)extent + 1u);
+    double entropy = 1.0;
+    const bool count = have && total >= T && total <= T3 && a.noentropy == 0;
+    const uint32_t counted = __ballot_sync(0xffffffffu, count);
+    unsigned long long packed = 0;  // four 16-bit match counters, packed as the reference packs them
+    const uint32_t g = lane >> 3, mine = (uint32_t)__popc(counted & lanemask_lt());
+    uint32_t at = 0;
+    for (uint32_t left = counted; left; at += 4) {
+      uint32_t src = 32;  // the group's candidate
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) packed += __shfl_xor_sync(0xffffffffu, packed, d);
-      int32_t c[4] = {(int32_t)(packed & 0xFFFF), (int32_t)((packed >> 16) & 0xFFFF),
-                      (int32_t)((packed >> 32) & 0xFFFF), (int32_t)((packed >> 48) & 0xFFFF)};
+      for (uint32_t k = 0; k < 4; k++) {
+        if (k == g && left) src = (uint32_t)__ffs((int)left) - 1u;
+        left &= left - 1;
+      }
+      const uint32_t r = __shfl_sync(0xffffffffu, rs, src & 31u), q = __shfl_sync(0xffffffffu, qs, src & 31u);
+      const int32_t n = __shfl_sync(0xffffffffu, positions, src & 31u);
+      unsigned long long sum = 0;
+      if (src < 32)
+        for (int32_t j = 32 * (int32_t)(lane & 7u); j < n; j += 256) {
+          uint32_t rlo, rhi, rsp, qlo, qhi, qsp;
+          window32(a.ref2, r + (uint32_t)j, &rlo, &rhi, &rsp);
+          window32(a.qry2, q + (uint32_t)j, &qlo, &qhi, &qsp);
+          sum += matches32(rlo, rhi, qlo, qhi, rsp | qsp, (uint32_t)min(n - j, 32));
+        }
+      __syncwarp();
+#pragma unroll
+      for (int d = 4; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      const unsigned long long got = __shfl_sync(0xffffffffu, sum, (mine & 3u) * 8u);
+      if (count && mine - at < 4u) packed = got;
+    }
+    if (count) {
+      const int32_t c[4] = {(int32_t)(packed & 0xFFFF), (int32_t)((packed >> 16) & 0xFFFF),
+                            (int32_t)((packed >> 32) & 0xFFFF), (int32_t)((packed >> 48) & 0xFFFF)};
       if (c[0] + c[1] + c[2] + c[3] >= 20) {
-        double denom = (double)((int32_t)((uint32_t)extent + 1u));
+        double denom = (double)positions;
         double ent = 0.0;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -871,10 +940,10 @@ __global__ void __launch_bounds__(kExactThreads) exact_kernel(ExactArgs a) {
         entropy = __ddiv_rn(-ent, 1.3862943649291992);  // (double)logf(4.0f), src/gpu/mod.rs:2349-2352
       }
     }
-    if (lane == 0 && sat_i32(__dmul_rn((double)__int2float_rn(total), entropy)) >= T) {
+    if (have && sat_i32(__dmul_rn((double)__int2float_rn(total), entropy)) >= T) {
       SegmentPair h;
-      h.ref_start = r0 - (uint32_t)lpos;
-      h.query_start = q0 - (uint32_t)lpos;
+      h.ref_start = rs;
+      h.query_start = qs - a.calls[cd.call & ~(kLongFlag | kDoneFlag)].qoff;
       h.len = (uint32_t)extent;
       h.score = entropy > 0.0 ? sat_i32(__dmul_rn((double)total, entropy)) : 0;
       uint32_t at = atomicAdd(&a.tot->raw, 1u);

@@ -115,3 +115,34 @@ def test_short_sequences_match_the_oracle(n):
     assert got.tobytes() == want.tobytes()
     for k in ("hits", "raw_hsps", "hsps", "cells"):
         assert st[k] == st_o[k], k
+
+
+@pytest.mark.parametrize("period", [1, 5, 33])
+@pytest.mark.parametrize("copies", [1, 40])
+def test_match_counts_of_every_segment_length(period, copies):
+    """Planted segments of 40..700 cells, N and soft-masked bases `period` or
+    more apart among them: the entropy's match counts at the ends of 32-base
+    words and of 256-base steps, with few candidates and with several a warp."""
+    rng = np.random.default_rng(period)
+    t, q = [], []
+    for n in list(range(40, 100)) + list(range(250, 262)) + [287, 288, 289, 511, 512, 513, 545, 700]:
+        seg = synth.random_bases(rng, n)
+        seg = np.where(rng.random(n) < 0.6, np.uint8(ord("A")), seg) if n % 3 else seg  # low entropy
+        other = seg.copy()
+        other[rng.integers(0, n, max(1, n // 30))] = ord("C")
+        for at in rng.integers(0, n, n // (16 * period)).tolist():
+            other[at] = seg[at] = ord("N") if at % 2 else seg[at] | 0x20
+        pad = synth.random_bases(rng, 60)
+        t += [seg, pad]
+        q += [other, pad[::-1]]
+    t, q = np.concatenate(t), np.concatenate(q * copies)
+    sm = EngineConfig().sub_mat
+    want, st_o = oracle_run(t, q, sm, hspthresh=1500)
+    with engine_for(sm, hspthresh=1500) as e:
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+    assert want.size > 50
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
