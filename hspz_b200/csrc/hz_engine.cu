@@ -1744,6 +1744,11 @@ int run_plain_wave(hz_engine *e, const std::vector<HostCall> &calls, std::pair<s
 // order.
 int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls,
                    const std::vector<std::pair<size_t, size_t>> &waves, std::vector<WaveRecord> *recs, hz_stats *st) {
+  // What this engine's stream still writes -- load_target returns with the
+  // neighbourhood counts and live seeds in flight -- is ordered before nothing
+  // on the workspaces' own streams, and counts that do not match the table
+  // would send the gate past its buckets.
+  TRY(e->sync());
   while ((int)e->twins.size() < k - 1) {
     hz_engine *w = nullptr;
     TRY(clone_shared(e, &w));
