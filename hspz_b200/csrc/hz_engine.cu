@@ -48,12 +48,16 @@ int fail(int code, const char *fmt, ...) {
   return code;
 }
 
-#define CK(x)                                                                                  \
-  do {                                                                                         \
-    cudaError_t e_ = (x);                                                                      \
-    if (e_ != cudaSuccess)                                                                     \
-      return fail(e_ == cudaErrorMemoryAllocation ? HZ_E_OOM : HZ_E_CUDA, "%s: %s (%s:%d)", #x, \
-                  cudaGetErrorString(e_), __FILE__, __LINE__);                                 \
+// (the runtime also remembers a failed call, and the next launch's check would
+// report it once more: a refused allocation is over once it is returned)
+#define CK(x)                                                                                     \
+  do {                                                                                            \
+    cudaError_t e_ = (x);                                                                         \
+    if (e_ != cudaSuccess) {                                                                      \
+      cudaGetLastError();                                                                         \
+      return fail(e_ == cudaErrorMemoryAllocation ? HZ_E_OOM : HZ_E_CUDA, "%s: %s (%s:%d)", #x,   \
+                  cudaGetErrorString(e_), __FILE__, __LINE__);                                    \
+    }                                                                                             \
   } while (0)
 
 #define TRY(x)                  \
@@ -841,7 +845,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
              std::vector<WaveRecord> *out, hz_stats *st, bool device_dedup, bool graph = false,
              DeferredDedup *defer = nullptr, uint32_t call_base = 0) {
   if (n == 0) return HZ_OK;
-  // a load or a swap that failed half way leaves its sequence unpacked
+  // the candidates' kernels read the packed sequences (a target or a query is
+  // there with its packed copy, or not at all)
   if (!e->ref_p.valid || !e->qry_p.valid) return fail(HZ_E_STATE, "a sequence was not loaded completely");
   cudaStream_t s = e->st;
   uint64_t npos = 0;
@@ -1102,6 +1107,22 @@ void query_calls(const hz_engine *e, uint32_t qid, std::vector<HostCall> *out) {
   }
 }
 
+// A load or a swap replaces buffers one by one.  Until all of it is in place
+// there is no target, or no query: one that fails half way must not leave the
+// new tables beside the old lengths.
+void drop_target(hz_engine *e) {
+  e->has_target = false;
+  e->has_nbr = false;
+  e->ref_p.valid = false;
+}
+void drop_query(hz_engine *e) {
+  e->has_query = false;
+  e->queries.clear();
+  e->cur_query = 0;
+  e->qry_p.valid = false;
+  e->slot[0].kind = e->slot[1].kind = 0;
+}
+
 // The per-k-mer neighbourhood hit counts and live seeds, for seed patterns of at most 14
 // care positions (4^k tables of at most 1 and 0.5 GB); larger patterns look up
 // every seed of a position instead.
@@ -1138,6 +1159,7 @@ int stage_ascii(hz_engine *e, const uint8_t *const *ascii, const uint64_t *lens,
   }
   if (total >= 0xFFFFFFFFull) return fail(HZ_E_INVALID, "staged queries exceed 4 GB");
   cudaStream_t s = e->st;
+  drop_query(e);
   TRY(e->qstore.ensure(total, s));
   uint64_t maxlen = 0;
   for (uint32_t i = 0; i < nq; i++) maxlen = std::max<uint64_t>(maxlen, lens[i]);
@@ -1155,9 +1177,7 @@ int stage_ascii(hz_engine *e, const uint8_t *const *ascii, const uint64_t *lens,
   TRY(pack_seq(e, e->qstore.base(), total, &e->qry_p));
   TRY(e->sync());
   e->queries = qs;
-  e->cur_query = 0;
   e->has_query = nq > 0;
-  e->slot[0].kind = e->slot[1].kind = 0;
   return HZ_OK;
 }
 
@@ -1410,6 +1430,7 @@ int hz_engine_load_tables(hz_engine *e, const uint32_t *index_table, uint64_t in
     if (ref_seq[i] > 7) return fail(HZ_E_INVALID, "ref_seq[%llu]=%u is not a device-alphabet code", (unsigned long long)i, ref_seq[i]);
   TRY(set_device(e));
   cudaStream_t s = e->st;
+  drop_target(e);
   TRY(e->index_table.ensure(index_len, s));
   TRY(e->pos_table.ensure(pos_len + 1, s));
   TRY(e->ref.ensure(ref_len, s));
@@ -1432,6 +1453,7 @@ int hz_engine_load_target(hz_engine *e, const uint8_t *ref_ascii, uint64_t len) 
   if (len > 0xFFFFFFFFull) return fail(HZ_E_INVALID, "reference block exceeds u32 coordinates");
   TRY(set_device(e));
   cudaStream_t st = e->st;
+  drop_target(e);
   const ShapeDev &sh = e->shape;
   uint64_t index_len = 1ull << (2 * sh.kmer_size);
   uint32_t step = e->cfg.step;
@@ -1552,6 +1574,7 @@ int hz_swap_query(hz_engine *e, const uint8_t *query, const uint8_t *query_rc, u
   q.off_f = 0;
   q.off_r = (uint32_t)((len + kPad + 15) & ~15ull);
   uint64_t total = q.off_r + len + kPad;
+  drop_query(e);
   TRY(e->qstore.ensure(total, e->st));
   CK(cudaMemsetAsync(e->qstore.base(), 0, total, e->st));
   if (len) {
@@ -1561,9 +1584,7 @@ int hz_swap_query(hz_engine *e, const uint8_t *query, const uint8_t *query_rc, u
   TRY(pack_seq(e, e->qstore.base(), total, &e->qry_p));
   TRY(e->sync());
   e->queries.assign(1, q);
-  e->cur_query = 0;
   e->has_query = true;
-  e->slot[0].kind = e->slot[1].kind = 0;
   return HZ_OK;
 }
 
