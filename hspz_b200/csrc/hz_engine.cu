@@ -1044,21 +1044,28 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     }
     if (again) continue;  // a capacity was too small: run the wave again with larger buffers
 
-    // per-scope dedup on the host, in scope order
-    e->cand_seen += t.cand;
-    if (st) {
+    // once nothing more can fail: a wave that does may be run again in parts
+    auto count = [&] {
+      e->cand_seen += t.cand;
+      if (!st) return;
       st->hits += t.hits;
       st->cells += t.cells;
       st->seeds += t.valid * w.per_pos;
       st->raw_hsps += t.raw;
       st->calls += n;
-    }
+    };
     const uint32_t nh = t.distinct;
-    if (nh == 0) return HZ_OK;
+    if (nh == 0) {
+      count();
+      return HZ_OK;
+    }
     // per-call waves (the plain form) dedup on the host like the reference,
     // unless the call holds so many HSPs that the device sort is faster
-    if (device_dedup || (e->device_dedup && nh >= e->device_dedup_min))
-      return dedup_on_device(e, nh, t.n_scopes, call_base, out, st);
+    if (device_dedup || (e->device_dedup && nh >= e->device_dedup_min)) {
+      TRY(dedup_on_device(e, nh, t.n_scopes, call_base, out, st));
+      count();
+      return HZ_OK;
+    }
     if (nh > pre_raw || t.n_scopes > pre_scopes) {  // not all read back with the totals
       TRY(e->d_out.ensure(nh, s));
       TRY(e->h_out.ensure(nh));
@@ -1071,6 +1078,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       CK(cudaMemcpyAsync(e->h_scope_call.p, e->scope_call.p, (size_t)t.n_scopes * 4, cudaMemcpyDeviceToHost, s));
       TRY(e->sync());
     }
+    count();
+    // per-scope dedup on the host, in scope order
     if (defer) {
       defer->pending = true;
       defer->n = nh;
@@ -1702,6 +1711,7 @@ int hz_seed_and_filter(hz_engine *e, uint32_t slot, int rev, hz_segment_pair **o
 namespace {
 void share_target(hz_engine *w, const hz_engine *e);
 int clone_shared(hz_engine *e, hz_engine **out);
+void release_wave(hz_engine *w);
 
 void add_stats(hz_stats *a, const hz_stats &b) {
   a->seeds += b.seeds;
@@ -1744,13 +1754,22 @@ std::vector<std::pair<size_t, size_t>> plain_waves(const hz_engine *e, const std
   return out;
 }
 
-// One wave of a plain pass; one that holds too many hits runs call by call.
+// One wave of a plain pass; one that holds too many hits, or whose buffers do
+// not fit the device, runs call by call.
 int run_plain_wave(hz_engine *e, const std::vector<HostCall> &calls, std::pair<size_t, size_t> wave,
                    std::vector<WaveRecord> *recs, hz_stats *st, DeferredDedup *defer = nullptr) {
   const size_t n = wave.second - wave.first;
+  const uint32_t tile_cap = e->tile_cap, cand_cap = e->cand_cap, raw_cap = e->raw_cap, scope_cap = e->scope_cap;
   int rc = run_wave(e, &calls[wave.first], n, nullptr, e->cfg.transitions, recs, st, false, false, defer,
                     (uint32_t)wave.first);
-  if (rc != kSplitWave) return rc;
+  if (n == 1 || (rc != kSplitWave && rc != HZ_E_OOM)) return rc;
+  if (rc == HZ_E_OOM) {  // a call needs a part of what the wave asked for
+    release_wave(e);
+    e->tile_cap = tile_cap;
+    e->cand_cap = cand_cap;
+    e->raw_cap = raw_cap;
+    e->scope_cap = scope_cap;
+  }
   for (size_t i = wave.first; i < wave.second; i++)
     TRY(run_wave(e, &calls[i], 1, nullptr, e->cfg.transitions, recs, st, false, false, defer, (uint32_t)i));
   return HZ_OK;
@@ -1797,11 +1816,11 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls,
   std::vector<std::vector<WaveRecord>> per(waves.size());
   std::atomic<size_t> next{0};
   std::atomic<bool> stop{false};
-  // waves an extra workspace could not finish for lack of device memory;
-  // this engine runs them once the others are done
+  // waves a workspace could not finish for lack of device memory; this
+  // engine runs them, and what is left, once the others are done
   std::vector<size_t> orphans;
   std::mutex orphans_mu;
-  auto drive = [&](hz_engine *x, hz_stats *sx, bool extra) -> int {
+  auto drive = [&](hz_engine *x, hz_stats *sx) -> int {
     for (;;) {
       if (stop.load()) return HZ_OK;
       size_t i = next.fetch_add(1);
@@ -1809,7 +1828,7 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls,
       hz_stats one;  // counted only once the wave has finished
       memset(&one, 0, sizeof one);
       int rc = run_plain_wave(x, calls, waves[i], &per[i], &one);
-      if (rc == HZ_E_OOM && extra) {  // this workspace stops; its wave moves on
+      if (rc == HZ_E_OOM) {  // this workspace stops; its wave moves on
         per[i].clear();
         std::lock_guard<std::mutex> lock(orphans_mu);
         orphans.push_back(i);
@@ -1836,17 +1855,19 @@ int run_pass_multi(hz_engine *e, int k, const std::vector<HostCall> &calls,
           stop.store(true);
           return;
         }
-        rcs[j] = drive(ws[j], &sts[j], true);
+        rcs[j] = drive(ws[j], &sts[j]);
         if (rcs[j] != HZ_OK) errs[j] = g_err;
       });
     } catch (const std::exception &) {  // no thread: its workspace takes no calls, the others take them all
       break;
     }
   }
-  rcs[0] = drive(e, &sts[0], false);
+  rcs[0] = drive(e, &sts[0]);
   for (auto &t : helpers) t.join();
-  if (rcs[0] == HZ_OK && !stop.load()) {
-    std::sort(orphans.begin(), orphans.end());
+  if (!orphans.empty() && !stop.load()) {
+    for (size_t j = 1; j < ws.size(); j++) release_wave(ws[j]);  // they are idle: their memory goes to this one
+    for (size_t i = next.load(); i < waves.size(); i++) orphans.push_back(i);  // when every workspace stopped
+    rcs[0] = HZ_OK;
     for (size_t i : orphans) {
       hz_stats one;
       memset(&one, 0, sizeof one);
@@ -2424,15 +2445,9 @@ uint64_t wave_footprint(const hz_engine *w) {
   return b;
 }
 
-// Gives an idle serving worker's query store, wave and dedup buffers back
-// (they grow again on its next batch, which restages its queries anyway).
-void release_wave_buffers(hz_engine *w) {
+// Gives an engine's wave and dedup buffers back (its next wave makes them again).
+void release_wave(hz_engine *w) {
   cudaStreamSynchronize(w->st);
-  if (!w->aliases_query) {
-    w->qstore.buf.release();
-    w->qry_p.release();
-  }
-  w->qascii.release();
   for (DBuf<uint32_t> *x : {&w->pos_hits, &w->np_pos, &w->call_nz_lo, &w->scope_call, &w->raw_scope, &w->tile_first,
                             &w->tile_call, &w->pos_kmer, &w->np_kmer, &w->d_set, &w->d_perm_a,
                             &w->d_perm_b, &w->d_kept, &w->d_total})
@@ -2447,6 +2462,17 @@ void release_wave_buffers(hz_engine *w) {
   w->d_out.release();
   w->calls.release();
   w->tot.release();
+}
+
+// The same and the query store, of an idle serving worker (its next batch
+// restages its queries anyway).
+void release_wave_buffers(hz_engine *w) {
+  release_wave(w);
+  if (!w->aliases_query) {
+    w->qstore.buf.release();
+    w->qry_p.release();
+  }
+  w->qascii.release();
 }
 
 // Device working memory a request of `len` bases is expected to need while

@@ -1,9 +1,11 @@
 """How a plain pass's calls share waves changes no record and no count."""
+import numpy as np
 import pytest
 
 from hspz_b200 import EngineConfig, synth
 from hspz_b200.build import build
 from tests.test_gpu_parity import engine_for, oracle_run
+from tests.test_gpu_reload import device_memory_left
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +38,24 @@ def test_calls_per_wave_and_streams(kw):
         assert st == runs[0][1]
     for k in ("hits", "raw_hsps", "hsps", "cells"):
         assert runs[0][1][k] == st_o[k], k
+
+
+@pytest.mark.parametrize("streams,calls,left", [(1, 80, 40 << 20), (4, 20, 12 << 20)])
+def test_waves_that_do_not_fit_run_call_by_call(streams, calls, left):
+    """A wave of several calls needs 24 bytes a position, 96 MB and 24 MB here;
+    where that is not to be had, its calls still fit one by one."""
+    rng = np.random.default_rng(2)
+    t, q = synth.random_bases(rng, 1_000_000), synth.random_bases(rng, 2_000_000)
+    synth.plant(rng, t, q, 100, 200, 3000, 0.05, 0.3)
+    with engine_for(EngineConfig().sub_mat, wga_chunk=50_000) as e:
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        e.set_tuning(plain_streams=streams, plain_calls=1)
+        want, st = e.run_pass()
+        e.set_tuning(plain_calls=calls)
+        with device_memory_left(left):
+            got, st2 = e.run_pass()
+        assert want.size > 100
+        assert got.tobytes() == want.tobytes() and st2 == st
+        got, st2 = e.run_pass()
+        assert got.tobytes() == want.tobytes() and st2 == st
