@@ -516,10 +516,14 @@ int cost_mode(const hz_engine *e) {
   if (X < 0) return -1;
   // drawdowns are kept in 16 bits (gate2_kernel), and long_kernel's group
   // states modulo 2^16 (near16)
-  if (top <= 127 && cost <= 127) return X <= kGate2MaxXdrop && X + kRound * 255 < 32768 ? (alike ? kAlike : kGeneral) : -1;
+  const bool bytes = X <= kGate2MaxXdrop && X + kRound * 255 < 32768;
+  if (top <= 127 && cost <= 127) return bytes ? (alike ? kAlike : kGeneral) : -1;
   // costs of 16 bits: the drop test's word holds kLeft costs above bit 15, the
   // running costs a round's rise above xdrop, the rescoring a score below it
   if (alike && cost * kLeft <= 32768 && top * kLeft + X + cost * kLeft <= 65535 && X + top <= 32767) return kWide;
+  // (a score of -128 also fits kGeneral: 1 Mbp against 100 Mbp, 209 M hits, 9.1
+  // ms, in the lane-refill gate 18.6; alike, kWide takes it in 6.9)
+  if (top <= 127 && cost <= 128 && bytes) return kGeneral;
   return -1;
 }
 

@@ -172,12 +172,14 @@ __device__ __forceinline__ void window_codes(const uint4 r[4], uint32_t a, uint3
 }
 
 // How a matrix's ACGT scores are looked up.  kAlike: complementary pairs score
-// alike and costs fit a signed byte; kGeneral: any byte scores; kWide: alike,
-// costs of 16 bits.
+// alike and costs fit a signed byte; kGeneral: any scores of a signed byte, whose
+// tables hold the scores themselves, since the cost of -128 is no signed byte
+// (sums negate them in the dot product's other factor, and the rescoring runs
+// on complements, so that costs nothing); kWide: alike, costs of 16 bits.
 enum CostMode : int { kAlike, kGeneral, kWide };
 
-// The costs of eight cells: bytes of the even cells, of the odd cells (kAlike,
-// kGeneral); 16-bit pairs of cells 0 2, 4 6, 1 3, 5 7 (kWide).
+// The costs of eight cells: bytes of the even cells, of the odd cells (kAlike;
+// kGeneral: of their scores); 16-bit pairs of cells 0 2, 4 6, 1 3, 5 7 (kWide).
 template <int MODE> struct Cells8 {
   uint32_t w[MODE == kWide ? 4 : 2];
 };
@@ -203,7 +205,8 @@ struct CostTable {
       for (int x = 0; x < 4; x++) {
         const int low = MODE == kGeneral ? i >> 1 : 0, parity = i & 1;
         const int r = (parity ^ low) << 1 | low;
-        const uint32_t cost = (uint32_t)-sub[r * kNuc + (r ^ x)];
+        const int32_t score = sub[r * kNuc + (r ^ x)];
+        const uint32_t cost = (uint32_t)(MODE == kGeneral ? score : -score);
         t[i] |= (cost >> (MODE == kWide && i >= 2 ? 8 : 0) & 0xFFu) << (8 * x);
       }
     }
@@ -254,9 +257,10 @@ template <int MODE> __device__ __forceinline__ uint32_t cost_word(const Cells8<M
 // acc + the cost of base b.
 template <int MODE> __device__ __forceinline__ uint32_t add_cost(const Cells8<MODE> &c, int b, uint32_t acc) {
   if (MODE == kWide) return (uint32_t)__dp2a_lo((int)cost_word(c, b), b & 2 ? 0x100 : 1, (int)acc);
-  return (uint32_t)__dp4a((int)cost_word(c, b), 1 << (8 * (b >> 1)), (int)acc);
+  return (uint32_t)__dp4a((int)cost_word(c, b), (int)((MODE == kGeneral ? 0xFFu : 1u) << (8 * (b >> 1))), (int)acc);
 }
-// The costs of base br of one group and base bl of another, as 16-bit halves.
+// The costs (kGeneral: the scores) of base br of one group and base bl of
+// another, as 16-bit halves.
 template <int MODE>
 __device__ __forceinline__ uint32_t cost_pair(const Cells8<MODE> &r, int br, const Cells8<MODE> &l, int bl) {
   uint32_t s;
@@ -582,12 +586,14 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
       const uint32_t shl = (fl & 1u) << 4, shr = (fr & 1u) << 4;
       const Cells8<MODE> lc = tab.cells(wl.x >> shl, wl.y >> shl), rc = tab.cells(wr.x >> shr, wr.y >> shr);
       uint32_t E = permute(wt.grp[gr][lane], wt.grp[gl][lane], 0x7610u);
+      if (MODE == kGeneral) E = ~E;  // the complement falls by a cost as it rises by the score
       uint32_t F = 0;      // bits 15 and 31: the direction has dropped
       uint32_t after = 0;  // 128 * (cells from the drop on: right + 16 * left)
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        E = __viaddmax_u16x2(E, cost_pair(rc, k, lc, 7 - k), thr2);
-        F = (F | E) & 0x80008000u;
+        const uint32_t pair = cost_pair(rc, k, lc, 7 - k);
+        E = MODE == kGeneral ? __viaddmin_u16x2(E, pair, ~thr2) : __viaddmax_u16x2(E, pair, thr2);
+        F = (F | (MODE == kGeneral ? ~E : E)) & 0x80008000u;
         after = __dp4a(F, 0x10000100u, after);
       }
       const uint32_t n = ((after >> 7) * 0x1001u) & 0x000F000Fu;  // the two counts in halves

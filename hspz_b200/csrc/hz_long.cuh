@@ -70,7 +70,7 @@ __device__ __forceinline__ Cells8<MODE> costs8(const CostTable<MODE> &tab, uint3
 }
 template <int MODE> __device__ __forceinline__ int32_t add_score(int32_t s, const Cells8<MODE> &c, int k) {
   if (MODE == kWide) return __dp2a_lo((int)cost_word(c, k), k & 2 ? 0xFF00 : 0xFF, s);
-  return __dp4a((int)cost_word(c, k), (int)(0xFFu << (8 * (k >> 1))), s);
+  return __dp4a((int)cost_word(c, k), (int)((MODE == kGeneral ? 1u : 0xFFu) << (8 * (k >> 1))), s);
 }
 
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }

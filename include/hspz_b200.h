@@ -229,7 +229,7 @@ int hz_engine_profile_reset(hz_engine *e);
 
 /* Launch-shape knobs (no reference counterpart; results never depend on
  * them): "gate_version" (2, the default: the lockstep gate over 2-bit packed
- * sequences, used whenever ACGT scores lie in -127..127, or complementary pairs score alike and costs
+ * sequences, used whenever ACGT scores lie in -128..127, or complementary pairs score alike and costs
  * fit the 16-bit sums, up to 585; 1: the
  * lane-refill gate over 8-bit codes, which also serves wider scores),
  * "gate_sparse" (the lockstep gate's tile setup: -1, the default, chosen

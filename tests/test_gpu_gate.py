@@ -146,3 +146,35 @@ def test_match_counts_of_every_segment_length(period, copies):
     assert got.tobytes() == want.tobytes()
     for k in ("hits", "raw_hsps", "hsps", "cells"):
         assert st[k] == st_o[k], k
+
+
+@pytest.mark.parametrize("alike", [False, True])
+@pytest.mark.parametrize("xdrop,cap,sparse,seed", [(910, 128, 0, "12of19"), (910, 56, 1, "12of19"), (0, 128, 0, "12of19"),
+                                                   (20000, 256, 1, "12of19"), (910, 8, 0, "1111")])
+def test_scores_of_the_whole_signed_byte(xdrop, cap, sparse, seed, alike):
+    """-128 and 127 beside strands that score differently (and alike): the
+    lockstep gate and the candidates' kernel take them, by half warps and
+    (the short seed's candidates, more than 32768) by lanes."""
+    t, q = sequences(xdrop + cap)
+    if seed == "1111":
+        t, q = t[:3000], q[:3000]
+    m = matrix("default", xdrop)
+    m[0 * 8 + 3], m[3 * 8 + 0], m[2 * 8 + 2] = -128, -128, 127  # A-T, T-A and G-G
+    if alike:
+        m[1 * 8 + 1] = 127  # C-C
+    else:
+        m[0 * 8 + 1], m[2 * 8 + 0] = -127, -128  # A-C and G-A, but not T-G and C-T
+    hspthresh = 3000 if xdrop >= 500 else 1500
+    want, st_o = oracle_run(t, q, m, xdrop=xdrop, hspthresh=hspthresh, seed=seed)
+    with engine_for(m, xdrop=xdrop, hspthresh=hspthresh, seed=seed) as e:
+        e.set_tuning(gate_cap=cap, gate_sparse=sparse)
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+        e.set_profiling(True)
+        e.run_pass()
+        assert "long" in e.profile()  # it follows the lockstep gate only
+    assert want.size > 0
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
