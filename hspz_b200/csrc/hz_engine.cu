@@ -2230,8 +2230,8 @@ int hz_engine_set_tuning(hz_engine *e, const char *key, int64_t value) {
   if (!e || !key) return fail(HZ_E_INVALID, "null argument");
   std::string k(key);
   if (k == "gate_tile") {
-    if (value != 64 && value != 128 && value != 256)
-      return fail(HZ_E_INVALID, "gate_tile must be 64, 128 or 256");
+    if (value != 0 && value != 64 && value != 128 && value != 256)
+      return fail(HZ_E_INVALID, "gate_tile must be 0, 64, 128 or 256");
     e->gate_tile = (int)value;
   } else if (k == "gate_version") {
     if (value != 1 && value != 2) return fail(HZ_E_INVALID, "gate_version must be 1 or 2");

@@ -235,8 +235,9 @@ int hz_engine_profile_reset(hz_engine *e);
  * "gate_sparse" (the lockstep gate's tile setup: -1, the default, chosen
  * from the target's average bucket; 0 a lane per (position, seed) pair;
  * 1 a lane per position, for targets whose tiles span many positions),
- * "gate_tile" (hits per gate warp tile: 64, 128, 256; unless set, what suits
- * the gate that runs: 256 for the lockstep gate, 128 for the lane-refill one),
+ * "gate_tile" (hits per gate warp tile: 64, 128 or 256; 0, the default: for
+ * the lockstep gate one of them by the hits each wave is expected to have, for
+ * the lane-refill gate 128),
  * "gate_cap" (cells per direction before a hit leaves the gate as a long
  * candidate -- for the lane-per-candidate long kernel after the lockstep
  * gate, for the warp kernel after the lane-refill gate -- multiple of 8,
@@ -275,7 +276,9 @@ int hz_engine_set_tuning(hz_engine *e, const char *key, int64_t value);
  * fastest: gate_tile (hits a gate warp stages per tile: 64, 128, 256, i.e.
  * 2..8 per lane), gate_cap (cells a lane scores before a hit moves to the warp
  * kernel: 64..1024) and graph (the wave chain replayed as a CUDA graph or
- * launched kernel by kernel).  Results never depend on the choice. */
+ * launched kernel by kernel).  Results never depend on the choice.  What it
+ * keeps holds for waves of every size.  Where no fixed tile beat the default
+ * of 0, that stays in place, and gate_tile is the one a large wave takes. */
 typedef struct hz_tuning {
   int32_t gate_tile;
   int32_t gate_cap;

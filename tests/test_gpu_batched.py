@@ -4,6 +4,7 @@ exactly the records the plain form gives for that query alone."""
 import pytest
 
 from hspz_b200 import Engine, EngineConfig
+from hspz_b200 import _native as N
 from hspz_b200 import synth
 from hspz_b200.build import build
 from tests.test_gpu_parity import oracle_run
@@ -172,3 +173,19 @@ def test_batched_equals_plain_under_flags(workload, kw):
             r, _ = e.run_pass()
             want.append([tuple(int(x[f]) for f in FIELDS) for x in r])
     assert per_query(got, len(chunks)) == want
+
+
+def test_the_default_tile_can_be_set_back(workload):
+    target, chunks = workload
+    with Engine(EngineConfig()) as e:
+        e.load_target(target)
+        e.stage_queries(chunks[:6])
+        base, st0 = e.run_batched()
+        for tile in (256, 0, 64, 0):
+            e.set_tuning(gate_tile=tile)
+            got, st = e.run_batched()
+            assert got.tobytes() == base.tobytes() and st == st0
+        for tile in (-1, 1, 32, 512):
+            with pytest.raises(N.HzError) as ex:
+                e.set_tuning(gate_tile=tile)
+            assert ex.value.code == N.HZ_E_INVALID
