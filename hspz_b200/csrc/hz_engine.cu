@@ -1136,15 +1136,16 @@ void drop_query(hz_engine *e) {
   e->slot[0].kind = e->slot[1].kind = 0;
 }
 
-// The per-k-mer neighbourhood hit counts and live seeds, for seed patterns of at most 14
-// care positions (4^k tables of at most 1 and 0.5 GB); larger patterns look up
-// every seed of a position instead.
+// The per-k-mer neighbourhood hit counts, for seed patterns of at most 14 care
+// positions (a 4^k table of at most 1 GB; larger patterns look up every seed of
+// a position instead), and, for engines with transitions, the live seeds
+// (0.5 GB): the gate looks at them only where a position has several seeds.
 int build_nbr_hits(hz_engine *e, uint64_t index_len) {
   e->has_nbr = false;
   if (e->shape.kmer_size > 14) return HZ_OK;
   cudaStream_t s = e->st;
   TRY(e->nbr_hits.ensure(index_len, s));
-  TRY(e->nbr_live.ensure(index_len, s));
+  if (e->cfg.transitions) TRY(e->nbr_live.ensure(index_len, s));
   const uint32_t *idx = e->index_table.p;
   uint32_t *out = e->nbr_hits.p;
   uint16_t *live = e->nbr_live.p;

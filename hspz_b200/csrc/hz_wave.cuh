@@ -128,7 +128,7 @@ __device__ __forceinline__ uint32_t bucket(const WaveIn &w, uint32_t k, uint32_t
 // transition seeds, summed -- what lookup_count adds up for a query
 // position with that k-mer (u32, wrapping like that sum) -- and which of them
 // have hits, bit v for seed v (kmer_size <= 14: 15 bits), which the gate's
-// sparse setup looks up one by one.
+// sparse setup looks up one by one (live may be null).
 __global__ void nbr_hits_kernel(const uint32_t *__restrict__ index_table, uint64_t n, uint32_t kmer_size,
                                 uint32_t occ_cap, uint32_t *__restrict__ out, uint16_t *__restrict__ live) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -153,7 +153,7 @@ __global__ void nbr_hits_kernel(const uint32_t *__restrict__ index_table, uint64
       bits |= c ? 1u << v : 0u;
     }
     out[i] = sum;
-    live[i] = (uint16_t)bits;
+    if (live) live[i] = (uint16_t)bits;
   }
 }
 

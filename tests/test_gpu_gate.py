@@ -178,3 +178,30 @@ def test_scores_of_the_whole_signed_byte(xdrop, cap, sparse, seed, alike):
     assert got.tobytes() == want.tobytes()
     for k in ("hits", "raw_hsps", "hsps", "cells"):
         assert st[k] == st_o[k], k
+
+
+def test_exact_seeds_keep_no_live_mask():
+    """An engine for exact seeds holds no 16-bit word per k-mer (0.5 GB for 14
+    care positions), and seeds with transitions still run on it."""
+    import torch
+
+    t, q = sequences(31)
+    sm = EngineConfig().sub_mat
+    want, _ = oracle_run(t, q, sm, seed="14of22")
+    held, got = [], []
+    with engine_for(sm) as e:  # the library's own memory is in place
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        e.run_pass()
+    for transitions in (True, False):
+        free = torch.cuda.mem_get_info()[0]
+        with engine_for(sm, seed="14of22", transitions=transitions) as e:
+            e.set_tuning(gate_sparse=1)
+            e.load_target(t)
+            held.append(free - torch.cuda.mem_get_info()[0])
+            e.swap_query_ascii(q)
+            e.generate_seeds(0, False, (0, q.size - e.seed_size + 1), transitions=True)
+            got.append(e.seed_and_filter(0, False))
+    assert held[0] - held[1] >= 2 * 4 ** 14 - (8 << 20)
+    assert got[0][0].size > 10 and want.size > 10
+    assert got[0][0].tobytes() == got[1][0].tobytes() and got[0][1] == got[1][1]
