@@ -674,7 +674,7 @@ int launch_long(hz_engine *e, const GateArgs &ga) {
   switch (cost_mode(e)) {
     case kAlike: return launch_long_as<kAlike>(e, la);
     case kGeneral: return launch_long_as<kGeneral>(e, la);
-    default: la.wide_max = 0xFFFFFFFFu; return launch_long_as<kWide>(e, la);
+    default: return launch_long_as<kWide>(e, la);
   }
 }
 

@@ -8,7 +8,7 @@
 // candidate and marks it kDoneFlag, so the exact kernel is left with the
 // entropy and the accept.
 //
-// Few candidates (LongArgs::wide_max; all of them where scores are kWide, whose
+// Few candidates (LongArgs::wide_max; all of them where costs are kWide, whose
 // group states would not fit 16 bits) go half a warp per direction, 256 cells
 // per step (long_wide): their time is that of the longest extension.  More go
 // one lane per candidate-direction, in rounds of kRound cells, which takes
@@ -69,7 +69,7 @@ __device__ __forceinline__ Cells8<MODE> costs8(const CostTable<MODE> &tab, uint3
   return tab.cells(sel.x, sel.y);
 }
 template <int MODE> __device__ __forceinline__ int32_t add_score(int32_t s, const Cells8<MODE> &c, int k) {
-  if (MODE == kWide) return __dp2a_lo((int)cost_word(c, k), k & 2 ? 0xFF00 : 0xFF, s);
+  static_assert(MODE != kWide, "the lane rounds' sums");
   return __dp4a((int)cost_word(c, k), (int)((MODE == kGeneral ? 1u : 0xFFu) << (8 * (k >> 1))), s);
 }
 
@@ -80,7 +80,7 @@ __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)
 // its kRound cells, which lies within kRound * 128 of every stored sum; a
 // stored maximum read back exceeds its sum by at most xdrop plus one group's
 // fall, so every value read lies within kRound * 255 + xdrop of the base
-// (gate2_usable checks that this is below 32768).
+// (cost_mode in hz_engine.cu admits only matrices and xdrops that keep this below 32768).
 __device__ __forceinline__ int32_t near16(int32_t base, uint32_t h) {
   return wadd(base, (int32_t)(int16_t)(uint16_t)(h - (uint32_t)base));
 }
@@ -98,7 +98,7 @@ struct LongArgs {
   int32_t sub[64];
   int32_t xdrop;
   uint32_t late_max_safe;  // as GateArgs::late_max_safe
-  uint32_t wide_max;       // candidates up to which half a warp extends each direction
+  uint32_t wide_max;       // candidates up to which half a warp extends each direction (kWide: always)
 };
 
 struct LongWarp {
@@ -264,15 +264,11 @@ template <int MODE> __device__ __forceinline__ void long_wide(const LongArgs &a,
   if (lane == 0 && cells_acc) atomicAdd(&a.tot->cells, cells_acc);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constant__ LongArgs a) {
+// More candidates: a lane per candidate and direction, in rounds of kRound cells.
+template <int MODE> __device__ __forceinline__ void long_lanes(const LongArgs &a, uint32_t ncand) {
+  static_assert(MODE != kWide, "group states are kept modulo 2^16 (near16)");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   LongSmem &sm = *reinterpret_cast<LongSmem *>(smem_raw);
-  const uint32_t ncand = min(a.tot->cand, a.cand_cap);
-  if (ncand <= a.wide_max) {
-    long_wide<MODE>(a, ncand);
-    return;
-  }
   LongWarp &wp = sm.warp[threadIdx.x >> 5];
   const CostTable<MODE> tab(a.sub);
   const uint32_t lane = threadIdx.x & 31;
@@ -523,6 +519,17 @@ __global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constan
   }
   for (int d = 16; d > 0; d >>= 1) cells_acc += __shfl_down_sync(0xffffffffu, cells_acc, d);
   if (lane == 0 && cells_acc) atomicAdd(&a.tot->cells, cells_acc);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kGateThreads) long_kernel(const __grid_constant__ LongArgs a) {
+  const uint32_t ncand = min(a.tot->cand, a.cand_cap);
+  if constexpr (MODE == kWide) {
+    long_wide<MODE>(a, ncand);
+  } else {
+    if (ncand <= a.wide_max) long_wide<MODE>(a, ncand);
+    else long_lanes<MODE>(a, ncand);
+  }
 }
 
 }  // namespace hz
