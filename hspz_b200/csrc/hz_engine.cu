@@ -405,7 +405,7 @@ struct hz_engine {
   std::map<std::string, ProfEntry> prof;
   std::vector<std::string> prof_order;
   uint64_t launches = 0;
-  uint64_t cand_seen = 0;  // gate candidates of every finished wave (serving admission learns from it)
+  uint64_t cand_seen = 0, distinct_seen = 0;  // gate candidates and different HSPs of every finished wave (serving admission learns from them)
 
   cudaEvent_t get_event() {
     if (!event_pool.empty()) {
@@ -547,11 +547,12 @@ double expected_hits(const hz_engine *e, uint64_t positions, uint32_t per_pos) {
 // warp (4144 of them) then runs on a part of the chip: gate time by tile size
 // 64 / 128 / 256, 0.11 M hits: 37 / 51 / 84 us, 0.52 M: 43 / 41 / 59, 0.86 M:
 // 73 / 72 / 79, 2.1 M: 116 / 116 / 113, 21 M: 732 / 658 / 628.
-int wave_tile(const hz_engine *e, double hits) {
-  if (e->gate_tile) return e->gate_tile;
-  if (!gate2_usable(e)) return 128;
+int tile_for(int knob, bool lockstep, double hits) {
+  if (knob) return knob;
+  if (!lockstep) return 128;
   return hits < 3e5 ? 64 : hits < 1.2e6 ? 128 : 256;
 }
+int wave_tile(const hz_engine *e, double hits) { return tile_for(e->gate_tile, gate2_usable(e), hits); }
 
 // Prepares one instance of the lockstep gate for 'smem' bytes of shared
 // memory and returns its blocks per SM.
@@ -1051,6 +1052,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
     // once nothing more can fail: a wave that does may be run again in parts
     auto count = [&] {
       e->cand_seen += t.cand;
+      e->distinct_seen += t.distinct;
       if (!st) return;
       st->hits += t.hits;
       st->cells += t.cells;
@@ -2412,11 +2414,12 @@ struct Server {
   // those and the batch's estimate; in_flight is their sum.
   uint64_t budget = 0, in_flight = 0;
   std::vector<uint64_t> reserved;
-  // rates the estimates use: hits per seed position, candidates and raw HSPs
-  // per hit -- the largest seen so far, starting from the target's average
-  // and 1e-3
-  double hits_per_pos = 0, cand_per_hit = 1e-3, raw_per_hit = 1e-3;
-  int gate_tile = 128;
+  // rates the estimates use: hits per seed position, candidates, raw HSPs and
+  // different HSPs per hit -- the largest seen so far, starting from the
+  // target's average and 1e-3
+  double hits_per_pos = 0, cand_per_hit = 1e-3, raw_per_hit = 1e-3, distinct_per_hit = 1e-3;
+  int gate_tile = 0;  // the knob, and whether the lockstep gate runs (tile_for)
+  bool lockstep = false;
   // bumped by a worker whose head request cannot fit while nothing runs:
   // idle workers then give their buffers back
   uint64_t trim_epoch = 0;
@@ -2484,12 +2487,17 @@ void release_wave_buffers(hz_engine *w) {
 // it runs: both strands of the query store (1 B per base, and 1 B for its
 // packed copy) and of the per-position counts, k-mers and compaction (24 B
 // per position), plus the hit-dependent buffers -- the gate's tile table (8 B
-// per tile of hits), candidates (32 B each), raw HSPs (20 B each) and their
-// dedup scratch (24 B each) -- at the server's current rates.
+// per tile of hits; a wave's tiles are at least as large as those of one of its
+// requests alone), candidates (32 B each), raw HSPs (20 B each, and 12 B of the
+// set that finds the different ones) and the different ones (12 B of sorted
+// indices and 32 B of output each) -- at the server's current rates.  What a
+// workspace holds from its first wave on whatever the request (the starting
+// capacities and the gate's ring) counts once it is there (wave_footprint).
 uint64_t serve_estimate(const Server *s, uint64_t len) {
   const double pos = 2.0 * (double)len;
   const double hits = pos * s->hits_per_pos;
-  const double per_hit = 8.0 / s->gate_tile + 32.0 * s->cand_per_hit + 44.0 * s->raw_per_hit;
+  const double per_hit = 8.0 / tile_for(s->gate_tile, s->lockstep, hits) + 32.0 * s->cand_per_hit +
+                         32.0 * s->raw_per_hit + 44.0 * s->distinct_per_hit;
   return (uint64_t)(pos * (2 + 24) + hits * per_hit) + (1ull << 20);
 }
 
@@ -2665,11 +2673,12 @@ void serve_worker(Server *s, uint32_t index, hz_engine *w) {
     std::vector<int> rcs(batch.size(), HZ_OK);
     std::vector<std::string> msgs(batch.size());
     hz_stats st{};
-    uint64_t l0 = w->launches, c0 = w->cand_seen;
+    uint64_t l0 = w->launches, c0 = w->cand_seen, d0 = w->distinct_seen;
     int rc = serve_pass(w, batch, &recs, &st);
     if (rc != HZ_OK && batch.size() > 1) {
       st = hz_stats{};
       c0 = w->cand_seen;
+      d0 = w->distinct_seen;
       recs.assign(batch.size(), {});
       for (size_t k = 0; k < batch.size(); k++) {
         std::vector<std::vector<hz_pass_record>> one;
@@ -2714,6 +2723,7 @@ void serve_worker(Server *s, uint32_t index, hz_engine *w) {
         s->hits_per_pos = std::max(s->hits_per_pos, (double)st.hits / (double)positions);
         s->cand_per_hit = std::max(s->cand_per_hit, (double)(w->cand_seen - c0) / (double)st.hits);
         s->raw_per_hit = std::max(s->raw_per_hit, (double)st.raw_hsps / (double)st.hits);
+        s->distinct_per_hit = std::max(s->distinct_per_hit, (double)(w->distinct_seen - d0) / (double)st.hits);
       }
       s->launches += w->launches - l0;
       s->totals.seeds += st.seeds;
@@ -2769,7 +2779,8 @@ int hz_serve_start(hz_engine *e, const hz_serve_config *cfg) {
   // starting rate: a query k-mer drawn uniformly meets per_pos buckets of the
   // average size
   s->hits_per_pos = e->index_len ? (double)e->per_pos(e->cfg.transitions) * (double)e->n_pos / (double)e->index_len : 0;
-  s->gate_tile = e->gate_tile ? e->gate_tile : 128;  // the smallest tile a wave takes by itself
+  s->gate_tile = e->gate_tile;
+  s->lockstep = e->gate_version == 2 && cost_mode(e) >= 0 && (uint64_t)e->rlen + 128 < (1ull << 32);
   e->server = s;
   for (uint32_t i = 0; i < (uint32_t)s->workers.size(); i++) s->threads.emplace_back(serve_worker, s, i, s->workers[i]);
   return HZ_OK;

@@ -228,3 +228,28 @@ def test_many_workers_random_poll_order_and_totals():
         assert (queued, running) == (0, 0)
         assert totals["hits"] == hits
         e.serve_stop()
+
+
+def test_the_estimate_covers_what_a_batch_holds():
+    """Every fourth hit an HSP, most of them different: what a worker holds after a
+    batch is the estimate at the rates it has shown, a quarter more where a
+    capacity grew (by as much beyond the need), and the starting capacities:
+    the tile table, the candidate, raw-HSP and set entries, the gate's ring."""
+    import torch
+
+    rng = np.random.default_rng(8)
+    target, query = synth.random_bases(rng, 10_000_000), synth.random_bases(rng, 4_000_000)
+    starting = (8 << 23) + (32 + 20 + 12 << 20) + 148 * 7 * 4 * 8 * 64 * 4
+    with Engine(EngineConfig(hspthresh=1000, noentropy=True)) as e:
+        e.load_target(target)
+        e.swap_query_ascii(query[:60_000])
+        e.run_pass()  # the library's own memory is in place
+        e.serve_start(budget_bytes=64 << 30, workers=1)
+        free = torch.cuda.mem_get_info()[0]
+        got, _ = e.serve_poll(e.serve_submit(query))
+        held = free - torch.cuda.mem_get_info()[0]
+        totals, _, _ = e.serve_stats()
+        est = e.serve_estimate(query.size)
+        e.serve_stop()
+    assert totals["raw_hsps"] > 8 << 20 and got.size > totals["raw_hsps"] // 2  # far beyond the starting capacities
+    assert held <= 1.25 * est + starting + (32 << 20)
