@@ -4,9 +4,9 @@
 // and two seed slots, mirroring the reference's Engine (src/gpu/mod.rs:817-2307).
 //
 // Every seed_and_filter call goes through the same wave pipeline
-// (hz_wave.cuh).  The plain per-chunk form runs one call per wave and reads
-// its HSPs back after each call, as the reference does; the batched form runs
-// many calls per wave with one read-back per wave.
+// (hz_wave.cuh).  The plain form runs one call per wave, or a few small ones,
+// and dedups their HSPs on the host, as the reference does; the batched form
+// runs many calls per wave with one read-back per wave.
 #include <algorithm>
 #include <atomic>
 #include <cstdarg>
@@ -365,7 +365,7 @@ struct hz_engine {
   HBuf<uint32_t> h_scope_call;
   // device dedup of the batched form
   bool device_dedup = true;
-  uint32_t device_dedup_min = 1u << 16;  // raw HSPs from which a per-call wave dedups on the device
+  uint32_t device_dedup_min = 1u << 16;  // different HSPs from which a plain wave dedups on the device
   // the wave's different HSPs: the hash set that finds them (2 raw_cap words),
   // their indices (raw_cap words) and the first kRawPrefix of them; and the
   // sorts' buffers

@@ -275,7 +275,7 @@ __device__ __forceinline__ uint32_t cost_pair(const Cells8<MODE> &r, int br, con
 }
 
 // SPARSE: the setup for targets whose buckets hold few positions, where a
-// 128-hit tile spans many query positions (10-20 Mbp bins): a lane per
+// tile spans many query positions (10-20 Mbp bins): a lane per
 // position instead of per (position, seed) pair.  The engine picks it from
 // the target's average bucket size.  MODE: see CostMode.
 template <bool SPARSE, int MODE>

@@ -103,7 +103,7 @@ struct LongArgs {
 
 struct LongWarp {
   uint32_t queue[64];          // long candidates claimed by the warp, not yet on a lane
-  uint32_t grp[kGroups][32];   // group states of a round, as in gate2_kernel
+  uint32_t grp[kGroups][32];   // the sum (low half) and maximum (high half) before each group of a round
 };
 
 struct LongSmem {
@@ -372,7 +372,7 @@ template <int MODE> __device__ __forceinline__ void long_lanes(const LongArgs &a
         gi = M > Mg ? g : gi;
       }
     }
-    // exact end of the round, as in gate2_kernel
+    // the exact end of the round: the flagged groups in turn, cell by cell
     const uint32_t gv = vv >> 3;
     uint32_t todo = have ? (flags | (gv < (uint32_t)kGroups ? 1u << gv : 0u)) & ((2u << gv) - 1u) : 0u;
     bool ended = false, dropped = false;

@@ -5,9 +5,12 @@
 //   np_*           scan of the counts; compaction of positions with hits; the
 //                  gate's tile table
 //   scopes         per call: hit range and MAX_HITS dedup scopes
-//   gate           fused hit expansion + thread-per-hit X-drop score gate
-//   long           lane-per-candidate exact extension of the gate's long candidates
-//   exact          warp-per-candidate X-drop positions, entropy, accept
+//   gate           fused hit expansion + X-drop score gate, a lane per hit
+//   long           exact extension of the lockstep gate's candidates, half a
+//                  warp or a lane per direction
+//   exact          entropy and accept, a lane per candidate (after the
+//                  lane-refill gate also the extensions, a warp each)
+//   distinct       exact copies out of the accepted HSPs
 //
 // Semantics follow hspZ src/gpu/kernels.rs and src/gpu/mod.rs (cited per
 // kernel).  Hit indices are 64-bit across a wave (a call's own hit count is
@@ -643,11 +646,12 @@ __global__ void __launch_bounds__(kScopeThreads) scopes_kernel(WaveIn w, const u
 namespace hz {
 
 // ---------------------------------------------------------------------------
-// Exact extension, one warp per candidate (find_hsps, src/gpu/kernels.rs:
-// 1279-1543): the positions of both maxima -- from the gate's maxima with one
-// sum scan per 32 cells, or, for a long candidate, the whole extension with
-// sum and maximum scans -- then the entropy correction and the final
-// threshold (:1555-1701).
+// The entropy correction and the final threshold of every candidate
+// (src/gpu/kernels.rs:1555-1701), a lane each, and before them, for the
+// candidates of the lane-refill gate, the positions of both maxima, a warp each
+// (find_hsps, :1279-1543): from the gate's maxima with one sum scan per 32
+// cells, or, past the gate's cap, the whole extension with sum and maximum
+// scans.
 
 struct ExactArgs {
   const uint8_t *ref;

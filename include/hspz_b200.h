@@ -92,7 +92,10 @@ int hz_engine_load_tables(hz_engine *e, const uint32_t *index_table, uint64_t in
 
 /* The same target built on the device from the ASCII reference block:
  * encode (src/sequence.rs:66-79) + SeedTable::build (src/seed.rs:135-180),
- * byte-identical tables, resident until the next load. */
+ * byte-identical tables, resident until the next load.  This load, the one
+ * above and the swaps and staging of queries below replace what was there: one
+ * that fails half way leaves no target, or no query (HZ_E_STATE from the calls
+ * that need it); refused arguments leave it as it was. */
 int hz_engine_load_target(hz_engine *e, const uint8_t *ref_ascii, uint64_t len);
 
 /* Copies the resident seed table back (tests / interop): index_len entries
@@ -229,8 +232,8 @@ int hz_engine_profile_reset(hz_engine *e);
 
 /* Launch-shape knobs (no reference counterpart; results never depend on
  * them): "gate_version" (2, the default: the lockstep gate over 2-bit packed
- * sequences, used whenever ACGT scores lie in -128..127, or complementary pairs score alike and costs
- * fit the 16-bit sums, up to 585; 1: the
+ * sequences, used whenever ACGT scores lie in -128..127, or complementary
+ * pairs score alike and costs fit the 16-bit sums, up to 585; 1: the
  * lane-refill gate over 8-bit codes, which also serves wider scores),
  * "gate_sparse" (the lockstep gate's tile setup: -1, the default, chosen
  * from the target's average bucket; 0 a lane per (position, seed) pair;
@@ -239,31 +242,31 @@ int hz_engine_profile_reset(hz_engine *e);
  * the lockstep gate one of them by the hits each wave is expected to have, for
  * the lane-refill gate 128),
  * "gate_cap" (cells per direction before a hit leaves the gate as a long
- * candidate -- for the lane-per-candidate long kernel after the lockstep
- * gate, for the warp kernel after the lane-refill gate -- multiple of 8,
- * 8..65528), "gate_blocks_per_sm" (0 = occupancy maximum),
+ * candidate, which a kernel of its own extends -- multiple of 8, 8..65528), "gate_blocks_per_sm" (0 = occupancy maximum),
  * "wave_positions" (seed positions per batched wave), "wave_hits_cap" (a
  * batched wave of several calls holding more seed hits than this, default
  * 2^33, is run again as smaller waves, which bounds the hit-dependent wave
  * buffers on repeat-dense input), "device_dedup" (1: the
- * batched form dedups on the device, and so does a plain-form call holding at
- * least "device_dedup_min" raw HSPs (default 65536); 0: every dedup on the
- * host, as the reference does),
+ * batched form dedups on the device, and so does a plain-form wave holding at
+ * least "device_dedup_min" different HSPs (default 65536); 0: every dedup on
+ * the host, as the reference does),
  * "graph" (1: the batched form captures each wave's kernel chain as a CUDA
  * graph and replays it, updating the instantiated graph in place),
  * "plain_calls" (calls that share a launch chain of hz_run_pass, 0..1000000;
  * 0, the default: as many as fill the device; 1: one chain per call),
  * "plain_streams" (1..4, default 4: hz_run_pass runs its chains on this
  * engine and plain_streams - 1 more workspaces over the same target, each
- * with its own host thread and stream, so one call's read-back and host dedup
- * overlap other calls' kernels; 1: one call at a time on this engine; an
- * engine given a caller's stream by hz_engine_set_stream runs every call on
- * that stream.  Each extra workspace is made on first use and holds its own
- * grow-only wave buffers -- about as much device memory as the largest call
- * it has run needs, i.e. up to plain_streams times one engine's wave memory
- * in all -- until the engine is destroyed or plain_streams is lowered, which
- * frees the workspaces beyond the new count.  A workspace that runs out of
- * device memory hands its call to this engine and is freed; the pass goes on),
+ * with its own host thread and stream, so one chain's read-back and host
+ * dedup overlap other chains' kernels; 1: one chain at a time on this engine;
+ * an engine given a caller's stream by hz_engine_set_stream runs every chain
+ * on that stream.  Each extra workspace is made on first use and holds its own
+ * grow-only wave buffers -- about as much device memory as the largest wave
+ * it has run needs, up to 2^22 seed positions of calls unless plain_calls says
+ * otherwise, i.e. up to plain_streams times one engine's wave memory in all --
+ * until the engine is destroyed or plain_streams is lowered, which frees the
+ * workspaces beyond the new count.  A wave that does not fit the device's
+ * memory runs call by call; a workspace without room for a call hands it to
+ * this engine and is freed, and the pass goes on),
  * "tile_cap" / "cand_cap" / "raw_cap" (starting capacities of the gate's
  * tile table, the candidate list and the raw-HSP list; a wave that needs more
  * grows them and runs again; the extra workspaces start from at least this
@@ -317,8 +320,8 @@ int hz_engine_set_stream(hz_engine *e, void *stream);
  * A batch is formed only while the sum over all workers stays within the
  * budget.  A worker whose buffers outgrow the budget after a batch frees
  * them; idle workers free theirs when a queued request could not fit
- * otherwise.  The estimates grow with the hits per position, candidates and
- * raw HSPs per hit the loop has seen, so a request accepted by
+ * otherwise.  The estimates grow with the hits per position, candidates, raw
+ * and different HSPs per hit the loop has seen, so a request accepted by
  * hz_serve_submit may later estimate above the whole budget; it then runs
  * alone once no other worker holds memory.
  * Failures: if a batch fails, each of its requests runs again alone, so only
