@@ -899,6 +899,13 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
   w.qp2 = packed_q ? e->qry_p.half_ptr(0) : nullptr;
   w.pos_kmer = e->pos_kmer.p;
   const int tile = wave_tile(e, expected_hits(e, npos, w.per_pos));
+  // A wave of several calls holding more hits than this is cut smaller
+  // (run_calls halves its position budget), so the grow-only wave buffers stay
+  // bounded on repeat-dense input.  Its gate must not run: where the tile table
+  // happened to have room for it, the rejected waves' gates took 16 to 36 % of
+  // a step (364 M positions against a 200 Mbp target: 1840 ms with the default table,
+  // 2207 and 2890 with one grown by 128- and 64-hit tiles).
+  const unsigned long long hits_cap = n > 1 ? e->wave_hits_cap : ~0ull;
 
   for (int attempt = 0; attempt < 8; attempt++) {  // each rerun fixes every capacity it found short
     uint32_t scope_cap = std::max<uint32_t>(e->scope_cap, (uint32_t)n * 2 + 16);
@@ -931,7 +938,8 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
           "np_scan",
           [&] {
             np_partials_kernel<<<1, kPartialThreads, 0, s>>>(e->np_partial.p, chunks, e->tot.p, e->np_excl.p,
-                                                             (uint32_t)tile, e->tile_first.p, e->tile_cap);
+                                                             (uint32_t)tile, e->tile_first.p, e->tile_cap,
+                                                             hits_cap);
             np_emit_kernel<<<chunks, kCountThreads, 0, s>>>(e->pos_hits.p, (uint32_t)npos, e->np_partial.p,
                                                             e->np_excl.p, e->np_pos.p, e->pos_kmer.p, e->np_kmer.p,
                                                             e->calls.p, (uint32_t)n, e->tot.p, (uint32_t)tile,
@@ -1027,10 +1035,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
       return fail(HZ_E_INVALID, "the first seed of a call holds more than max_hits=%u hits; the reference's MAX_HITS "
                                 "walk has no valid cut there", e->max_hits);
     bool again = false;
-    // a wave of several calls holding more hits than wave_hits_cap is cut
-    // smaller (run_calls halves its position budget), so the grow-only wave
-    // buffers stay bounded on repeat-dense input
-    if (n > 1 && t.hits > e->wave_hits_cap) return kSplitWave;
+    if (t.hits > hits_cap) return kSplitWave;
     if (t.status & 4u) {  // the gate skipped the wave: its tile table was too small
       e->tile_cap = (uint32_t)std::min<uint64_t>(t.hits / (uint64_t)tile + 1024, 0xFFFFFFF0ull);
       again = true;

@@ -370,7 +370,9 @@ __global__ void __launch_bounds__(kCountThreads) lookup_count_kernel(WaveIn w, u
 // the hits and positions with hits before each, in one block; the totals go to
 // WaveTotals, with the sentinel np_excl[nz], and the gate's tile table is
 // checked against the total: tile_first[n_tiles] = nz, or status bit 2 when the
-// table is too small (the wave is then rerun with a larger one).
+// table is too small (the wave is then rerun with a larger one) or the wave
+// holds more than hits_cap hits (its calls are then rerun in smaller waves); the
+// gate skips a wave with that bit.
 constexpr int kPartialThreads = 1024;
 constexpr int kPartialItems = 4;
 
@@ -378,7 +380,8 @@ __global__ void __launch_bounds__(kPartialThreads) np_partials_kernel(HitNz *par
                                                                       WaveTotals *__restrict__ t,
                                                                       unsigned long long *__restrict__ np_excl,
                                                                       uint32_t tile, uint32_t *__restrict__ tile_first,
-                                                                      uint32_t tile_cap) {
+                                                                      uint32_t tile_cap,
+                                                                      unsigned long long hits_cap) {
   __shared__ HitNz s_warp[32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   HitNz carry{0ull, 0u};
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kPartialThreads) np_partials_kernel(HitNz *par
     t->nz = carry.n;
     np_excl[carry.n] = carry.h;
     const unsigned long long n_tiles = (carry.h + tile - 1) / tile;
-    if (n_tiles + 1 > tile_cap) t->status |= 4u;
+    if (n_tiles + 1 > tile_cap || carry.h > hits_cap) t->status |= 4u;
     else tile_first[n_tiles] = carry.n;
   }
 }

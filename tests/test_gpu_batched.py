@@ -1,6 +1,7 @@
 """The batched form against the plain per-chunk form and the oracle: many
 query chunks of uneven length through shared waves must give, per query,
 exactly the records the plain form gives for that query alone."""
+import numpy as np
 import pytest
 
 from hspz_b200 import Engine, EngineConfig
@@ -189,3 +190,33 @@ def test_the_default_tile_can_be_set_back(workload):
             with pytest.raises(N.HzError) as ex:
                 e.set_tuning(gate_tile=tile)
             assert ex.value.code == N.HZ_E_INVALID
+
+
+def test_waves_cut_for_their_hits_run_no_gate():
+    """A wave with more hits than wave_hits_cap is looked up, then cut in
+    smaller ones.  Its gate does not run, whatever room the tile table has: with
+    the gates of the rejected waves the 134 M hits here would be scored about
+    three times over."""
+    rng = np.random.default_rng(4)
+    target = synth.random_bases(rng, 10_000_000)
+    chunks = [synth.random_bases(rng, 1_000_000) for _ in range(8)]
+    cap = 5 << 20  # two calls of ~2.1 M hits
+    gate, got = [], []
+    # the table fits the waves that are kept, or any
+    for tile_cap in (cap // 256 + 1024, 1 << 23):
+        with Engine(EngineConfig()) as e:
+            e.set_tuning(tile_cap=tile_cap, gate_tile=256, wave_hits_cap=cap)
+            e.load_target(target)
+            e.stage_queries(chunks)
+            got.append(e.run_batched())
+            ms = []
+            for _ in range(5):
+                e.set_profiling(True)
+                e.profile_reset()
+                e.run_batched()
+                ms.append(e.profile()["gate"][0])
+                e.set_profiling(False)
+            gate.append(min(ms))
+    assert got[0][1]["hits"] > 16 * cap  # cut several times
+    assert got[0][0].tobytes() == got[1][0].tobytes() and got[0][1] == got[1][1]
+    assert gate[1] < 1.5 * gate[0]
