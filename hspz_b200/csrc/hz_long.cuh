@@ -463,7 +463,9 @@ template <int MODE> __device__ __forceinline__ void long_lanes(const LongArgs &a
         mpos = (int32_t)(cells + vv);
         pbase = -1;
       } else if (Mr > M0) {
-        if (!dropped && used == (uint32_t)kRound) {  // every group valid: the main pass's last rise
+        // every cell valid: the main pass's last rise (a special base at the
+        // last cell scores as an A there, which may look like one)
+        if (!dropped && vv == (uint32_t)kRound) {
           pbase = (int32_t)(cells + 8u * (uint32_t)gi);
           pS = near16(S, wp.grp[gi][lane] & 0xFFFFu);
         } else {  // the last valid group that starts below Mr holds the first cell reaching it

@@ -205,3 +205,32 @@ def test_exact_seeds_keep_no_live_mask():
     assert held[0] - held[1] >= 2 * 4 ** 14 - (8 << 20)
     assert got[0][0].size > 10 and want.size > 10
     assert got[0][0].tobytes() == got[1][0].tobytes() and got[0][1] == got[1][1]
+
+
+@pytest.mark.parametrize("seed", ["1111", "12of19"])
+def test_special_base_at_a_rounds_last_cell(seed):
+    """An extension that goes on past a soft-masked base: at the last cell of a
+    48-cell round, where it packs as an A and would match, while the maximum
+    lies in an earlier group of the round (the eight cells before it fall by 26
+    from their best).  Anchors lie at every distance from it, both ways; the
+    short seed's candidates are more than 32768."""
+    rng = np.random.default_rng(6)
+    t, q = synth.random_bases(rng, 3000), synth.random_bases(rng, 3000)
+    for i in range(10):
+        at = 100 + 280 * i
+        body = synth.random_bases(rng, 110)
+        # outward from the body: A-T, A-A, A-G, A-C, A-A, A-G, A-A, a-A, three matches
+        tail_t, tail_q = np.frombuffer(b"AAAAAAAaCCC", np.uint8), np.frombuffer(b"TAGCAGAACCC", np.uint8)
+        t[at:at + 132] = np.concatenate([tail_t[::-1], body, tail_t])
+        q[at + 3:at + 135] = np.concatenate([tail_q[::-1], body, tail_q])
+    sm = EngineConfig().sub_mat
+    want, st_o = oracle_run(t, q, sm, xdrop=3000, seed=seed)
+    with engine_for(sm, xdrop=3000, seed=seed) as e:
+        e.set_tuning(gate_cap=8)
+        e.load_target(t)
+        e.swap_query_ascii(q)
+        got, st = e.run_pass()
+    assert want.size >= 10
+    assert got.tobytes() == want.tobytes()
+    for k in ("hits", "raw_hsps", "hsps", "cells"):
+        assert st[k] == st_o[k], k
