@@ -499,9 +499,10 @@ int pack_seq(hz_engine *e, const uint8_t *codes, uint64_t n, Packed *p) {
   return HZ_OK;
 }
 
-// How the lockstep gate looks this matrix's scores up (CostMode), or -1 when
-// they don't fit it and the lane-refill gate runs.
-int cost_mode(const hz_engine *e) {
+// How the lockstep gate (or, with `candidates`, the kernel that extends its
+// candidates) looks this matrix's scores up (CostMode), or -1 when they don't
+// fit it and the lane-refill gate runs.
+int cost_mode(const hz_engine *e, bool candidates = false) {
   const int32_t *sub = e->cfg.sub_mat;
   const int64_t X = e->cfg.xdrop;
   int64_t top = 0, cost = 0;  // the largest score and cost
@@ -520,11 +521,15 @@ int cost_mode(const hz_engine *e) {
   if (top <= 127 && cost <= 127) return bytes ? (alike ? kAlike : kGeneral) : -1;
   // costs of 16 bits: the drop test's word holds kLeft costs above bit 15, the
   // running costs a round's rise above xdrop, the rescoring a score below it
-  if (alike && cost * kLeft <= 32768 && top * kLeft + X + cost * kLeft <= 65535 && X + top <= 32767) return kWide;
-  // (a score of -128 also fits kGeneral: 1 Mbp against 100 Mbp, 209 M hits, 9.1
-  // ms, in the lane-refill gate 18.6; alike, kWide takes it in 6.9)
-  if (top <= 127 && cost <= 128 && bytes) return kGeneral;
-  return -1;
+  const bool wide = alike && cost * kLeft <= 32768 && top * kLeft + X + cost * kLeft <= 65535 && X + top <= 32767;
+  // A score of -128 also fits kGeneral.  The gate takes it so where strands
+  // differ (1 Mbp against 100 Mbp, 209 M hits: 9.1 ms, in the lane-refill gate 18.6);
+  // alike, kWide is faster (6.9).  Its candidates always go kGeneral, which has
+  // the lane rounds that many candidates need (repeat-dense, 16 Mbp by 4 Mbp:
+  // 4.1 ms of extensions, 13.4 as kWide).
+  const bool general = top <= 127 && cost <= 128 && bytes;
+  if (wide && !(candidates && general)) return kWide;
+  return general ? kGeneral : -1;
 }
 
 // The lockstep gate needs packed sequences and 32-bit positions.
@@ -672,7 +677,7 @@ int launch_long(hz_engine *e, const GateArgs &ga) {
   // each, a lane per direction 96 us (its longest extension) and 1 ns:
   // 60 000 candidates 222 / 167 us, 105 000 379 / 170
   la.wide_max = 32768;
-  switch (cost_mode(e)) {
+  switch (cost_mode(e, true)) {
     case kAlike: return launch_long_as<kAlike>(e, la);
     case kGeneral: return launch_long_as<kGeneral>(e, la);
     default: return launch_long_as<kWide>(e, la);

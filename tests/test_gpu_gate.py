@@ -234,3 +234,33 @@ def test_special_base_at_a_rounds_last_cell(seed):
     assert got.tobytes() == want.tobytes()
     for k in ("hits", "raw_hsps", "hsps", "cells"):
         assert st[k] == st_o[k], k
+
+
+def test_many_candidates_of_a_score_of_128_below_zero():
+    """-128 is no signed byte's cost, and the gate takes strands that score alike
+    with 16-bit ones; the candidates still go by lanes, not half a warp each
+    (six times as long here), and match those of half warps."""
+    rng = np.random.default_rng(12)
+    t, q = synth.random_bases(rng, 1_000_000), synth.random_bases(rng, 1_000_000)
+    synth.plant(rng, t, q, 40, 200, 2000, 0.1, 0.3)
+    ms = []
+    for score in (-127, -128):
+        m = list(EngineConfig().sub_mat)
+        m[0 * 8 + 3] = m[3 * 8 + 0] = score
+        got = []
+        with engine_for(m) as e:
+            e.load_target(t)
+            e.swap_query_ascii(q)
+            for cap in (8, 128):  # every hit a candidate, few of them
+                e.set_tuning(gate_cap=cap)
+                got.append(e.run_pass())
+            e.set_tuning(gate_cap=8, plain_streams=1)
+            e.run_pass()
+            for _ in range(5):
+                e.set_profiling(True)
+                e.profile_reset()
+                e.run_pass()
+                ms.append(e.profile()["long"][0])
+                e.set_profiling(False)
+        assert got[0][0].size >= 40 and got[0][0].tobytes() == got[1][0].tobytes() and got[0][1] == got[1][1]
+    assert min(ms[5:]) < 2 * min(ms[:5])
