@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(kGateThreads) gate_kernel(GateArgs a) {
   static_assert(TW % 32 == 0, "a warp tile is a multiple of 32 hits");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GateSmem<TW> &sm = *reinterpret_cast<GateSmem<TW> *>(smem_raw);
-  if (a.tot->status & 4u) return;  // no tile table: the host reruns the wave with a larger one
+  if (a.tot->status & 4u) return;  // no tile table, or too many hits: the host reruns the wave, or its parts
   if (threadIdx.x < 64) sm.sub[threadIdx.x] = a.sub[threadIdx.x];
   __syncthreads();  // the block's only barrier
   const char *subb = reinterpret_cast<const char *>(sm.sub);

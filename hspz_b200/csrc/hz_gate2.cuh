@@ -282,7 +282,7 @@ template <bool SPARSE, int MODE>
 __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel(const __grid_constant__ Gate2Args a2) {
   const GateArgs &a = a2.g;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (a.tot->status & 4u) return;  // no tile table: the host reruns the wave with a larger one
+  if (a.tot->status & 4u) return;  // no tile table, or too many hits: the host reruns the wave, or its parts
   const uint32_t tile = a2.tile;
   unsigned char *mine = smem_raw + (threadIdx.x >> 5) * (sizeof(GateWarp) + tile * 12);
   GateWarp &wt = *reinterpret_cast<GateWarp *>(mine);

@@ -63,7 +63,9 @@ struct WaveTotals {
   unsigned long long tiles;  // gate work-queue cursor
   uint32_t nz;               // positions with at least one hit
   uint32_t n_scopes;
-  uint32_t status;  // bit 0: a call's first seed alone exceeds max_hits; bit 1: a call exceeds 2^32 hits
+  // bit 0: a call's first seed alone exceeds max_hits; bit 1: a call exceeds
+  // 2^32 hits; bit 2: the gate skips the wave (np_partials_kernel)
+  uint32_t status;
   uint32_t cand;    // gate candidates written (may exceed capacity)
   uint32_t raw;     // accepted HSPs written (may exceed capacity)
   uint32_t long_next;  // long_kernel's cursor over the candidates
