@@ -910,7 +910,7 @@ int run_wave(hz_engine *e, const HostCall *hc, size_t n, const uint64_t *seeds, 
   // happened to have room for it, the rejected waves' gates took 16 to 36 % of
   // a step (364 M positions against a 200 Mbp target: 1840 ms with the default table,
   // 2207 and 2890 with one grown by 128- and 64-hit tiles).
-  const unsigned long long hits_cap = n > 1 ? e->wave_hits_cap : ~0ull;
+  const unsigned long long hits_cap = n > 1 ? std::min<uint64_t>(e->wave_hits_cap, kMaxWaveHits) : ~0ull;
 
   for (int attempt = 0; attempt < 8; attempt++) {  // each rerun fixes every capacity it found short
     uint32_t scope_cap = std::max<uint32_t>(e->scope_cap, (uint32_t)n * 2 + 16);

@@ -83,6 +83,10 @@ static_assert(kLeft % 8 == 0 && kRight % 8 == 0 && kLeft > kRight, "groups of ei
 // up to 128 per cell.
 constexpr int32_t kGate2MaxXdrop = 32767 - 128;
 
+// Hits of a wave of several calls, whatever its limit: the lockstep gate keeps
+// a hit's index / 32 in 32 bits.  (A call alone has fewer than 2^32.)
+constexpr uint64_t kMaxWaveHits = 1ull << 37;
+
 // Shared memory of one warp; the slot arrays follow, 12 bytes per hit of a
 // tile: 5.6 KB with 256-hit tiles, 164 KB per SM, which leaves 88 KB of L1.
 // 128-hit tiles take 29.7 ps per hit (a setup every four rounds, mostly
@@ -300,8 +304,8 @@ __global__ void __launch_bounds__(kGate2Threads, kGate2BlocksPerSm) gate2_kernel
   const WaveIn &w = a.w;
   uint32_t cells_acc = 0;  // cells of the lane's hits, added to the wave's count before it can wrap
 
-  // the tile the cursor hands hits out of (warp-uniform); a wave's hits are
-  // below 2^37, so hit indices / 32 fit 32 bits
+  // the tile the cursor hands hits out of (warp-uniform); a wave has at most
+  // kMaxWaveHits hits, so hit indices / 32 fit 32 bits
   uint32_t tile_at = 0, nt = 0, cursor = 0;
   // the next tile's index, claimed from the work queue once half of the
   // current tile is handed out so that its latency is hidden (lane 0 holds it)

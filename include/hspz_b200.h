@@ -246,7 +246,7 @@ int hz_engine_profile_reset(hz_engine *e);
  * "wave_positions" (seed positions per batched wave), "wave_hits_cap" (a
  * batched wave of several calls holding more seed hits than this, default
  * 2^33, is run again as smaller waves, which bounds the hit-dependent wave
- * buffers on repeat-dense input), "device_dedup" (1: the
+ * buffers on repeat-dense input; no wave of several calls holds more than 2^37), "device_dedup" (1: the
  * batched form dedups on the device, and so does a plain-form wave holding at
  * least "device_dedup_min" different HSPs (default 65536); 0: every dedup on
  * the host, as the reference does),

@@ -220,3 +220,31 @@ def test_waves_cut_for_their_hits_run_no_gate():
     assert got[0][1]["hits"] > 16 * cap  # cut several times
     assert got[0][0].tobytes() == got[1][0].tobytes() and got[0][1] == got[1][1]
     assert gate[1] < 1.5 * gate[0]
+
+
+def test_waves_hold_no_more_hits_than_their_indices():
+    """36 calls of 3.9e9 hits each, 1.4e11 in all, more than 2^37: with the
+    largest wave_hits_cap they still do not share one wave, whose last hits'
+    indices would wrap into the first call."""
+    rng = np.random.default_rng(21)
+    unit = synth.random_bases(rng, 19)
+
+    def copies(n):  # of the unit, 31 random bases between them
+        gaps = synth.random_bases(rng, 31 * n).reshape(n, 31)
+        return np.concatenate([np.tile(unit, (n, 1)), gaps], axis=1).ravel()
+
+    target = copies(290_000)
+    chunks = [copies(5000) for _ in range(36)]
+    for q in chunks:
+        a, b = int(rng.integers(0, target.size - 400)), int(rng.integers(0, q.size - 400))
+        q[b:b + 400] = target[a:a + 400]
+    got = []
+    with Engine(EngineConfig(strand="plus", hspthresh=12000)) as e:
+        e.load_target(target)
+        e.stage_queries(chunks)
+        for cap in (1 << 33, 1 << 40):
+            e.set_tuning(wave_hits_cap=cap)
+            got.append(e.run_batched())
+    assert got[0][1]["hits"] > 1 << 37
+    assert sorted(set(got[0][0]["query"].tolist())) == list(range(36))
+    assert got[1][0].tobytes() == got[0][0].tobytes() and got[1][1] == got[0][1]
